@@ -576,10 +576,7 @@ fp_status fpb_workspace_build(const fp_op *op, const Arr &x, const fp_options &o
         A((void **)&ws->an_parent, (size_t)B * (size_t)N * sizeof(int));
         A((void **)&ws->an_cnt, (size_t)B * (size_t)N * sizeof(int));
         A((void **)&ws->an_sum, (size_t)B * (size_t)N * sizeof(unsigned long long));
-        A(&ws->an_ys, img);
         A(&ws->an_segv, img);
-        A((void **)&ws->an_segk, (size_t)B * (size_t)N * sizeof(int));
-        if (!op->spatial.empty()) A(&ws->an_wt, op->spatial.size() * T);
     }
     if (ws->keep) {
         const size_t bn = (size_t)B * (size_t)N, kk = (size_t)g.k;
@@ -640,17 +637,6 @@ fp_status fpb_workspace_build(const fp_op *op, const Arr &x, const fp_options &o
             if (r == cudaSuccess) r = cudaMemsetAsync(ws->err, 0, 16, ps);
             if (r == cudaSuccess && !spatial_h.empty())
                 r = cudaMemcpyAsync(ws->spatial, spatial_h.data(), spatial_h.size(), cudaMemcpyHostToDevice, ps);
-            if (r == cudaSuccess && ws->an_wt && N > 0) {  // the edge weights of strided axes, fibre-major
-                AnGeom ag{};
-                ag.k = g.k;
-                for (int a = 0; a < 3; ++a) ag.L[a] = a < g.k ? g.L[a] : 1;
-                ag.S[g.k - 1] = 1;
-                for (int a = g.k - 2; a >= 0; --a) ag.S[a] = ag.S[a + 1] * ag.L[a + 1];
-                for (int a = g.k; a < 3; ++a) ag.S[a] = 1;
-                ag.N = N;
-                ag.B = B;
-                r = aniso_weights_fm(x.dtype, ag, ws->spatial, ws->an_wt, ps);
-            }
             return r;
         });
         ws->dev_block = base;
@@ -1175,10 +1161,7 @@ fp_status run_aniso(fp_workspace *ws, const fp_op *op, const void *xsrc, void *z
     bf.parent = ws->an_parent;
     bf.sum = ws->an_sum;
     bf.cnt = ws->an_cnt;
-    bf.ys = ws->an_ys;
     bf.segv = ws->an_segv;
-    bf.segk = ws->an_segk;
-    bf.wt = ws->an_wt;
     bf.img = ws->an_img;
     bf.st = ws->an_st;
     bf.gammas = ws->gammas;

@@ -45,12 +45,24 @@ struct Num;
 template <>
 struct Num<double> {
     static __device__ __forceinline__ double inf() { return CUDART_INF; }
-    static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+    static __host__ __device__ __forceinline__ double mul(double a, double b) {
+#ifdef __CUDA_ARCH__
+        return __dmul_rn(a, b);
+#else
+        return a * b;
+#endif
+    }
 };
 template <>
 struct Num<float> {
     static __device__ __forceinline__ float inf() { return CUDART_INF_F; }
-    static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+    static __host__ __device__ __forceinline__ float mul(float a, float b) {
+#ifdef __CUDA_ARCH__
+        return __fmul_rn(a, b);
+#else
+        return a * b;
+#endif
+    }
 };
 
 // 1/m by division.
@@ -357,6 +369,271 @@ __device__ __forceinline__ void tv1d_warp(const In &in, const Sink &out, int n, 
     if (COPY && act && !fill && !serial) {
         for (int i = 0; i < n; ++i) out.segment(i, i, (double)in(i));
         out.finish(n);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// A fibre's scan by several lanes
+// ---------------------------------------------------------------------------
+//
+// Right after a jump at edge e the scan's whole state is (e, up or down): what
+// it does from there on depends on nothing before. So lanes start at P places
+// of a fibre, each in a guessed state, and where a scan from further left
+// jumps at the same edge in the same direction as the lane did, the lane's
+// segments from there on are the left scan's own, bit for bit. (Two taut
+// strings through the same tube, once they touch, stay together: the guess
+// costs a segment or two at the start of a piece.) Lane p
+//  1. scans from entry c_p, as if a fibre began there, until a segment ends
+//     past its piece; the segments that end within the piece are marked (down
+//     1, up 2, the fibre's end 3) with their values;
+//  2. if any did (or p = 0), scans on until it jumps where another lane has
+//     marked the same jump (that lane's segments take over after it), or to
+//     the fibre's end, keeping the segments in a list of its own;
+//  3. the lanes that lane 0 reaches from lane to lane are the valid ones: they
+//     write their lists over the marks, and in each valid lane's piece the
+//     marks past the jump it was reached at stay.
+// The segments are those of CondatScan over the whole fibre, for any input: a
+// lane whose guess never meets the true scan is passed over. The work is the
+// scan's, plus about a segment per piece.
+// The step itself is CondatScan's arithmetic without its opening case: a
+// segment opens at the jump (or start) with its first sample taken, and jumps
+// found within a trip of kPieceUnroll steps are handled together at its end
+// (at 7 jumps per 100 steps nearly every step would take the branch for some
+// lane of the warp).
+
+constexpr unsigned char kMarkFinal = 4;
+// Samples per trip: on 64 x 512^2 with edge weights 171 ms a solve at 4, 165 at
+// 6, 161 at 8, 155 at 12; smaller batches lose at 12 what they gain at 8.
+constexpr int kPieceUnroll = 8;
+
+// An entry and the radius of its edge, read in one load.
+template <class C>
+struct alignas(2 * sizeof(C)) Pair {
+    C y, r;
+};
+
+// W: yr holds (y, radius) pairs; else y, and every radius is l.
+template <class C, bool W>
+struct PieceScan {
+    const C *yr;
+    const C *rc;
+    C l;
+    int n;
+    int k, k0, km, kp;
+    int dir;  // a jump that waits: 1 down, 2 up
+    C vmin, vmax, ref, s;
+
+    __host__ __device__ __forceinline__ C y(int i) const { return yr[W ? 2 * i : i]; }
+    __host__ __device__ __forceinline__ C r(int i) const { return W ? yr[2 * i + 1] : l; }
+    // A segment from entry `at`, its first sample taken: s0 = sigma r_e.
+    __host__ __device__ __forceinline__ void open(int at, C s0) {
+        k = k0 = km = kp = at;
+        ref = y(at);
+        const C ra = r(at);
+        s = s0;
+        vmin = ref + (s0 - ra);
+        vmax = ref + (s0 + ra);
+        dir = 0;
+    }
+    // Takes the next kPieceUnroll samples, up to a jump or the last one. The
+    // samples' loads depend on nothing that the trip computes, and the steps
+    // take no branch: past a jump or the end they compute on and change
+    // nothing (k runs on past n - 1; it is not read then). Entries up to
+    // n + kPieceUnroll - 1 of yr, and 1/m up to that m, are read and unused.
+    __host__ __device__ __forceinline__ void trip() {
+        C yv[kPieceUnroll], rv[kPieceUnroll], q[kPieceUnroll];
+        const int left = n - 1 - k;
+#pragma unroll
+        for (int u = 0; u < kPieceUnroll; ++u) {
+            if (W) {
+                const Pair<C> yp = reinterpret_cast<const Pair<C> *>(yr)[k + 1 + u];
+                yv[u] = yp.y;
+                rv[u] = yp.r;
+            } else {
+                yv[u] = yr[k + 1 + u];
+                rv[u] = l;
+            }
+            q[u] = rc[k - k0 + 2 + u];
+        }
+        bool jump = false;
+#pragma unroll
+        for (int u = 0; u < kPieceUnroll; ++u) {
+            const bool in = u < left;
+            const C s1 = s + (yv[u] - ref);
+            const C a = ref + Num<C>::mul(s1 - rv[u], q[u]), b = ref + Num<C>::mul(s1 + rv[u], q[u]);
+            const bool go = in && !jump;
+            const bool dn = go && b < vmin, up = go && a > vmax;
+            dir = dn ? 1 : (up ? 2 : dir);
+            jump = jump || dn || up;
+            const bool ok = in && !jump;
+            const bool cm = ok && a >= vmin, cp = ok && b <= vmax;
+            s = in ? s1 : s;
+            vmin = cm ? a : vmin;
+            km = cm ? k + 1 + u : km;
+            vmax = cp ? b : vmax;
+            kp = cp ? k + 1 + u : kp;
+        }
+        k += kPieceUnroll;
+    }
+    // The segment that a waiting jump (or the fibre's end) closes: its last
+    // entry and value, and which it was (1 down, 2 up, 3 the end). 0: none.
+    __host__ __device__ __forceinline__ int event(int &e, C &v) const {
+        if (dir == 0 && k < n - 1) return 0;
+        int d = dir;
+        C ve = C(0);
+        if (d == 0) {
+            ve = ref + Num<C>::mul(s, rc[n - k0]);
+            d = ve < vmin ? 1 : (ve > vmax ? 2 : 3);
+        }
+        e = d == 1 ? km : (d == 2 ? kp : n - 1);
+        v = d == 1 ? vmin : (d == 2 ? vmax : ve);
+        return d;
+    }
+    // The next segment after a jump of direction d at edge e.
+    __host__ __device__ __forceinline__ void jump(int e, int d) { open(e + 1, d == 1 ? r(e) : -r(e)); }
+};
+
+// Trips of the scan until `ev` (given each segment as it closes: end, value
+// and direction; it says whether to go on) has stopped every lane. A scan
+// takes at most 2 (n + 1)^2 steps, and every trip takes at least one step or
+// one segment per live lane.
+template <class S, class C, class Ev>
+__device__ __forceinline__ void piece_trips(S &p, bool live, const Ev &ev, C, int *err) {
+    const unsigned most = 2u * (unsigned)(p.n + 1) * (unsigned)(p.n + 1);  // n < 46340
+    for (unsigned it = 0; __any_sync(0xffffffffu, live); ++it) {
+        if (it > most) {
+            if (live) atomicExch(err, 4);
+            break;
+        }
+        if (live) {
+            p.trip();
+            int e;
+            C v;
+            const int dir = p.event(e, v);
+            if (dir) {
+                live = ev(e, v, dir);
+                if (live) p.jump(e, dir);
+            }
+        }
+    }
+}
+
+// The scan of a fibre of n entries by the P lanes of its group (a power of two
+// up to 32, aligned in the warp), lane `sub` on the piece of len entries from
+// sub len; every lane of the warp calls it, with live false for groups that
+// have nothing to scan (their marks stay). mark: n bytes, zero before; val: n
+// values (the segments' at their ends); le, lv: this lane's list of `cap`
+// segments. Afterwards every mark is a segment's end.
+template <class C, bool W>
+__device__ __forceinline__ void tv1d_pieces(const C *yr, const C *rc, C l, int n, int P, int len, int sub, bool live,
+                                            unsigned char *mark, C *val, int *le, C *lv, int cap, int *err) {
+    PieceScan<C, W> p;
+    p.yr = yr;
+    p.rc = rc;
+    p.l = l;
+    p.n = n;
+    const int c0 = sub * len, c1 = c0 + len < n ? c0 + len : n;
+    const bool mine = live && c0 < n;
+    bool own = sub == 0;
+    int xe = 0, xs = 0;  // the segment that ended this lane's piece
+    C xv = C(0);
+    if (mine) p.open(c0, C(0));
+    piece_trips(
+        p, mine,
+        [&](int e, C v, int dir) {
+            if (e < c1) {
+                val[e] = v;
+                mark[e] = (unsigned char)dir;
+                own = true;
+            }
+            if (dir != 3 && e + 1 < c1) return true;
+            xe = e;
+            xs = dir;
+            xv = v;
+            return false;
+        },
+        C(0), err);
+    __syncwarp();
+    // on to a jump that another lane has marked
+    int nxt = -1, at = n, cnt = 0;  // the lane that takes over, after the segment that ends at `at`
+    auto put = [&](int e, C v) {
+        if (cnt < cap) {
+            le[cnt] = e;
+            lv[cnt] = v;
+        }
+        ++cnt;
+    };
+    bool go = mine && own && xs != 3;
+    if (mine && own && xe >= c1) {
+        put(xe, xv);
+        if (xs != 3 && mark[xe] == xs) {
+            nxt = xe / len;
+            at = xe;
+            go = false;
+        }
+    }
+    if (go) p.jump(xe, xs);
+    piece_trips(
+        p, go,
+        [&](int e, C v, int dir) {
+            put(e, v);
+            if (dir == 3) return false;
+            if (mark[e] == dir) {
+                nxt = e / len;
+                at = e;
+                return false;
+            }
+            return true;
+        },
+        C(0), err);
+    __syncwarp();
+    // the lanes reached from lane 0
+    bool valid = mine && sub == 0;
+    int ent = 0;
+    const int base = (threadIdx.x & 31) - sub;
+    for (int h = 0, cur = live ? 0 : -1; h < P; ++h) {
+        const int src = base + (cur >= 0 ? cur : 0);
+        const int nx = __shfl_sync(0xffffffffu, nxt, src), ax = __shfl_sync(0xffffffffu, at, src);
+        if (cur >= 0) {
+            if (nx == sub) {
+                valid = true;
+                ent = ax + 1;
+            }
+            cur = nx > cur ? nx : -1;
+        }
+        if (!__any_sync(0xffffffffu, cur >= 0)) break;
+    }
+    // the marks that do not count: before the jump a valid lane was reached at,
+    // and all of another's
+    if (mine && own) {
+        const int c2 = valid ? (ent < c1 ? ent : c1) : c1;
+        for (int i = c0; i < c2; ++i) mark[i] = 0;
+    }
+    __syncwarp();
+    // the valid lanes' lists over the marks; a list that was too long is scanned again
+    if (valid && cnt <= cap) {
+        for (int j = 0; j < cnt; ++j) {
+            val[le[j]] = lv[j];
+            mark[le[j]] = kMarkFinal;
+        }
+    }
+    const bool again = valid && cnt > cap;
+    if (__any_sync(0xffffffffu, again)) {
+        if (again) {
+            if (xe >= c1) {
+                val[xe] = xv;
+                mark[xe] = kMarkFinal;
+            }
+            p.jump(xe, xs);
+        }
+        piece_trips(
+            p, again,
+            [&](int e, C v, int dir) {
+                val[e] = v;
+                mark[e] = kMarkFinal;
+                return dir != 3 && e != at;
+            },
+            C(0), err);
     }
 }
 

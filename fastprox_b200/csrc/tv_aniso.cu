@@ -15,7 +15,7 @@
 // kernel acts only on the images in its stage, and the last block of an
 // image (a ticket per image) advances the stage with the scalar logic of the
 // reference in FP64. The host issues the same round of launches until no
-// image is live. The 1D steps are Condat's algorithm, one thread per fibre
+// image is live. The 1D steps are Condat's algorithm, several lanes per fibre
 // (tv1d.cuh). Components of the polish are found by union-find with atomic
 // hooking of the larger root to the smaller (so every root is the smallest
 // index of its component, whatever the order), and region sums use 64-bit
@@ -667,240 +667,57 @@ __global__ void __launch_bounds__(kTileThreads) an_fdpg3_tile(AnGeom g, AnCall c
 }
 
 // ---------------------------------------------------------------------------
-// Fibre-major passes
+// Fibre passes by pieces
 // ---------------------------------------------------------------------------
 //
-// The fibre scans are long serial chains (each step of Condat's scan depends on
-// the last), so a pass is bound by how many fibres an SM keeps in flight. The
-// tiles above hold a block's fibres in shared memory, which caps an SM at a few
-// dozen fibres. These passes keep every fibre of the launch in flight at once
-// (a lane per fibre, 32 fibres a warp, in lockstep) and read the fibres through
-// the L1 cache from a fibre-major copy, where each fibre's entries are
-// contiguous: a lane's reads walk its own few cache lines. A pass is:
-//  * stage: y of every fibre of the axis into ys, fibre-major (entry i of fibre
-//    f at f L + i), through 32 x 32 tiles of shared memory (coalesced both
-//    ways); a contiguous axis (stride 1) is fibre-major already, and its scan
-//    reads the image arrays directly;
-//  * scan: Condat's scan of every fibre (tv1d_warp); each segment's last entry
-//    and value go to a list in the order the scan emits them (segk, segv);
-//    after the scan each lane fills its fibre's entries from the list, into ys
-//    in place (or, for the first pass over a contiguous axis, straight into u);
-//  * unstage: the results back into the image's layout with the pass's
-//    epilogue (the dual update and the restart test's sums for the second
-//    pass), through the same tiles.
-// The arithmetic of every step is the tiled passes'. The restart test's FP64
-// sums are formed per tile block in a fixed order (its tiles, then the blocks),
-// a partition that depends on the image's shape only.
-// Edge weights along a strided axis are read from a fibre-major copy made once
-// per workspace (an_weights_fm).
+// One kernel per pass of ADBPG: a block stages the inputs of its fibres (and
+// their radii) in shared memory, coalesced along the fibre when fibres are
+// contiguous and across fibres otherwise, scans every fibre by P pieces at
+// once (tv1d.cuh, PieceScan: a lane per piece), fills the fibres' entries from
+// the segments found, and ends with the pass's epilogue (u, or z with the dual
+// update and the restart test's sums). Each array of the pass is read from HBM
+// once and written once.
+//
+// What bounds a pass is the scan: a chain of dependent steps, two to three
+// per entry. A lane per fibre leaves 1400 chains of 3000 steps for one 1400^2
+// image and lets a block of 512^2 images fill a quarter of each warp; pieces
+// make the chains P times shorter and fill the warps. Measured, ms a solve, a
+// lane per fibre over fibre-major copies in global memory (three kernels a
+// pass), then this: 64 x 512^2 with edge weights 284, 173; 1400^2 67.8, 14.4;
+// 90^2 3.24, 2.16. With pieces of 64 entries (P = 8) a warp takes 37 trips of 8
+// steps for 4 fibres of 512 entries and 1200 steps each; an SM holds 10 warps
+// by shared memory (40 weighted fibres) and issues 0.37 instructions per
+// scheduler and cycle, so latency and occupancy bound it, not HBM (36 B per
+// pixel and iteration, 92 of about 870 us).
+// The segments' values go to global scratch (segv, at their last entry) and
+// their ends to a byte per entry in shared memory, so that a fibre takes 5
+// bytes per entry there (9 with weights) and an SM holds many.
 
-// The segments of a fibre's scan as a list in the order the scan emits them,
-// which is their order along the fibre (a segment, once emitted, is final:
-// the scan goes on from the entry after its end): entry q of the list holds
-// the q-th segment's last entry and value. finish walks the list forwards and
-// fills the fibre's entries; each segment's list entry is read one segment
-// ahead, so the reads do not wait on one another.
+constexpr int kFibList = 6;      // segments a lane may hold beyond its piece before it scans them twice
+constexpr int kFibThreads = 256; // most threads of a block
 template <class T>
-struct SegSink {
-    T *val;
-    int *end;
-    T *out;
-    int *err;
-    mutable int cnt = 0;  // segments emitted
-    __device__ __forceinline__ void segment(int, int k1, double v) const {
-        val[cnt] = (T)v;
-        end[cnt] = k1;
-        ++cnt;
-    }
-    __device__ __forceinline__ void finish(int n) const {
-        int prev = -1;
-        int e = cnt > 0 ? end[0] : -1;
-        T v = cnt > 0 ? val[0] : T(0);
-        for (int q = 0; q < cnt; ++q) {
-            const int en = q + 1 < cnt ? end[q + 1] : -1;
-            const T vn = q + 1 < cnt ? val[q + 1] : T(0);
-            if (e <= prev || e >= n) break;  // not in order: a broken scan, flagged below
-            for (int i = prev + 1; i <= e; ++i) out[i] = v;
-            prev = e;
-            e = en;
-            v = vn;
-        }
-        if (prev != n - 1) atomicExch(err, 4);
-        cnt = 0;
-    }
+constexpr int kFibVec = 16 / (int)sizeof(T);
+
+struct FibCfg {
+    int nf;     // fibres per block
+    int P;      // pieces (lanes) per fibre, a power of two up to 32
+    int len;    // entries per piece (odd, so that a fibre's pieces start in different banks)
+    int pitch;  // entries between fibres in shared memory (odd)
 };
 
-// Entry i of a fibre-major fibre.
+// Shared memory of a block: 1/m, the fibres (y, or (y, r) pairs), a lane's
+// list (values, ends), the end marks. (The scan's trips read a few entries past
+// a fibre's last and 1/m past m = L: the next array's, unused.)
 template <class T>
-struct FmIn {
-    const T *p;
-    __device__ __forceinline__ T operator()(int i) const { return p[i]; }
-};
-// d + w (the first pass) or u - w (the second) of a contiguous fibre.
-template <class T, int PASS>
-struct SumIn {
-    const T *a, *w;
-    __device__ __forceinline__ T operator()(int i) const { return PASS == 1 ? (T)(a[i] + w[i]) : (T)(a[i] - w[i]); }
-};
-
-// Whether pass PASS of a round acts on image b (the stages of an_pass1 / an_pass2).
-template <int PASS>
-__device__ __forceinline__ bool fm_active(const AnState &st, const AnImage &im) {
-    if (st.status != kLive || im.mode != kAnAdbpg) return false;
-    return PASS == 1 ? (st.stage == kStIter || st.stage == kStWarm) : st.stage == kStIter;
+__host__ __device__ __forceinline__ size_t fib_smem(const FibCfg &c, int L, bool w) {
+    const size_t nt = (size_t)c.nf * c.P;
+    size_t b = sizeof(T) * ((size_t)(w ? 2 : 1) * c.nf * c.pitch + nt * kFibList + (size_t)(L + 1));
+    b += sizeof(int) * nt * kFibList;
+    return b + (size_t)c.nf * ((c.pitch + 3) / 4 * 4);
 }
 
-constexpr int kFmTile = 32;     // tile of 32 fibres x 32 entries
-constexpr int kFmThreads = 256; // 32 x 8 threads per tile block
-constexpr int kFmScan = 128;    // threads per scan block
-constexpr int kFmLanes = 8;     // fibres per warp of a scan block (its other lanes idle)
-
-__host__ __device__ __forceinline__ int64_t fm_tiles(int64_t nfib, int64_t L) {
-    return ((nfib + kFmTile - 1) / kFmTile) * ((L + kFmTile - 1) / kFmTile);
-}
-
-// ys = y of axis a's fibres, fibre-major (PASS 1: d + w along a1; 2: u - w along a2).
-template <class T, int PASS>
-__global__ void __launch_bounds__(kFmThreads) an_fm_stage(AnGeom g, AnCall c, AnBuffers bf) {
-    __shared__ T tile[kFmTile][kFmTile + 1];
-    const int b = round_image(bf, blockIdx.y);
-    if (b < 0) return;
-    const AnImage &im = bf.img[b];
-    if (!fm_active<PASS>(bf.st[b], im)) return;
-    const int a = PASS == 1 ? im.a1 : im.a2;
-    const Fib fb = fibers(g, a);
-    const int64_t N = g.N, L = fb.L;
-    const T *P0 = static_cast<const T *>(PASS == 1 ? bf.d : bf.u) + (int64_t)b * N;
-    const T *Wv = static_cast<const T *>(bf.wv) + (int64_t)b * g.k * N;
-    T *Y = static_cast<T *>(bf.ys) + (int64_t)b * N;
-    auto src = [&](int64_t o) -> T { return PASS == 1 ? (T)(P0[o] + Wv[o]) : (T)(P0[o] - Wv[o]); };
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int64_t neg = (L + kFmTile - 1) / kFmTile, nt = fm_tiles(fb.nfib, L);
-    for (int64_t t = blockIdx.x; t < nt; t += gridDim.x) {
-        const int64_t f0 = (t / neg) * kFmTile, i0 = (t % neg) * kFmTile;
-#pragma unroll
-        for (int r = 0; r < kFmTile; r += 8) {  // along the fibres (adjacent fibres are adjacent in memory)
-            const int64_t f = f0 + tx, i = i0 + ty + r;
-            tile[ty + r][tx] = (f < fb.nfib && i < L) ? src(fb.base(f) + i * fb.s) : T(0);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < kFmTile; r += 8) {  // along each fibre
-            const int64_t f = f0 + ty + r, i = i0 + tx;
-            if (f < fb.nfib && i < L) Y[f * L + i] = tile[tx][ty + r];
-        }
-        __syncthreads();
-    }
-}
-
-// Condat's scan of every fibre of the pass's axis, a lane per fibre.
-// DIRECT: the axis is contiguous and the scan reads the image arrays (d + w,
-// or u - w); the first pass then fills u, the second ys.
-template <class T, int PASS, bool DIRECT>
-__global__ void __launch_bounds__(kFmScan) an_fm_scan(AnGeom g, AnCall c, AnBuffers bf) {
-    extern __shared__ __align__(16) unsigned char an_fm_smem[];
-    const int b = round_image(bf, blockIdx.y);
-    if (b < 0) return;
-    const AnImage &im = bf.img[b];
-    if (!fm_active<PASS>(bf.st[b], im)) return;
-    const int a = PASS == 1 ? im.a1 : im.a2;
-    const Fib fb = fibers(g, a);
-    const int L = (int)fb.L;
-    T *rc = reinterpret_cast<T *>(an_fm_smem);  // 1/m, m <= L
-    {
-        const DivRecip<T> div;
-        for (int m = threadIdx.x; m <= L; m += blockDim.x) rc[m] = m ? div(m) : T(0);
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int64_t f = ((int64_t)blockIdx.x * (kFmScan / 32) + (threadIdx.x >> 5)) * kFmLanes + lane;
-    const bool act = lane < kFmLanes && f < fb.nfib;
-    const int64_t N = g.N, fo = act ? f * L : 0;  // fibre-major offset (the image offset when DIRECT)
-    T *Y = static_cast<T *>(bf.ys) + (int64_t)b * N + fo;
-    T *out = (DIRECT && PASS == 1) ? static_cast<T *>(bf.u) + (int64_t)b * N + fo : Y;
-    const SegSink<T> sink{static_cast<T *>(bf.segv) + (int64_t)b * N + fo, bf.segk + (int64_t)b * N + fo, out, bf.err};
-    const double lam = im.lam[a];
-    const TableRecip<T> rcp{rc};
-    auto run = [&](const auto &in) {
-        if (c.has_beta) {
-            const T *bw = static_cast<const T *>(fb.s == 1 ? bf.beta : bf.wt) + (int64_t)a * c.N + fo;
-            tv1d_warp<T, true>(in, sink, L, lam, true, FmIn<T>{bw}, rcp, act);
-        } else {
-            tv1d_warp<T, true>(in, sink, L, lam, false, NoWeight{}, rcp, act);
-        }
-    };
-    if (DIRECT) {
-        const T *P0 = static_cast<const T *>(PASS == 1 ? bf.d : bf.u) + (int64_t)b * N + fo;
-        const T *Wv = static_cast<const T *>(bf.wv) + (int64_t)b * g.k * N + fo;
-        run(SumIn<T, PASS>{P0, Wv});
-    } else {
-        run(FmIn<T>{Y});
-    }
-}
-
-// The scan's results back into the image's layout. PASS 1: u = z. PASS 2:
-// z, and the dual update with the extrapolation (an_pass2's); the last block
-// of the image runs the restart test and advances the iteration.
-template <class T, int PASS>
-__global__ void __launch_bounds__(kFmThreads) an_fm_unstage(AnGeom g, AnCall c, AnBuffers bf) {
-    __shared__ T tile[kFmTile][kFmTile + 1];
-    __shared__ double sh[32];
-    __shared__ int flag;
-    const int b = round_image(bf, blockIdx.y);
-    if (b < 0) return;
-    const AnState st = bf.st[b];
-    const AnImage &im = bf.img[b];
-    if (!fm_active<PASS>(st, im)) return;
-    const int a = PASS == 1 ? im.a1 : im.a2;
-    const Fib fb = fibers(g, a);
-    const int64_t N = g.N, L = fb.L;
-    const T *Y = static_cast<const T *>(bf.ys) + (int64_t)b * N;
-    T *U = static_cast<T *>(bf.u) + (int64_t)b * N;
-    T *Wv = static_cast<T *>(bf.wv) + (int64_t)b * g.k * N;
-    T *Yd = static_cast<T *>(bf.y) + (int64_t)b * g.k * N;
-    T *Z = static_cast<T *>(bf.z) + (int64_t)b * N;
-    const bool test = st.it % kCheck == 0;
-    const T beta = (T)st.beta;
-    double up = 0.0;
-    auto put = [&](int64_t o, T z) {
-        if (PASS == 1) {
-            U[o] = z;
-        } else {
-            const T v = U[o] - Wv[o];
-            const T yn = z - v;
-            const T y = Yd[o], w = Wv[o];
-            if (test) up += (double)((w - yn) * (yn - y));
-            Wv[o] = yn + beta * (yn - y);
-            Yd[o] = yn;
-            Z[o] = z;
-        }
-    };
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    if (fb.s == 1) {  // fibre-major is the image's layout
-        for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += (int64_t)gridDim.x * blockDim.x)
-            put(p, Y[p]);
-    } else {
-        const int64_t neg = (L + kFmTile - 1) / kFmTile, nt = fm_tiles(fb.nfib, L);
-        for (int64_t t = blockIdx.x; t < nt; t += gridDim.x) {
-            const int64_t f0 = (t / neg) * kFmTile, i0 = (t % neg) * kFmTile;
-#pragma unroll
-            for (int r = 0; r < kFmTile; r += 8) {  // along each fibre
-                const int64_t f = f0 + ty + r, i = i0 + tx;
-                tile[ty + r][tx] = (f < fb.nfib && i < L) ? Y[f * L + i] : T(0);
-            }
-            __syncthreads();
-#pragma unroll
-            for (int r = 0; r < kFmTile; r += 8) {  // along the fibres
-                const int64_t f = f0 + tx, i = i0 + ty + r;
-                if (f < fb.nfib && i < L) put(fb.base(f) + i * fb.s, tile[tx][ty + r]);
-            }
-            __syncthreads();
-        }
-    }
-    if (PASS == 1) return;
-    double dot, unused;
-    if (!reduce2(bf, b, blockIdx.x, gridDim.x, test ? up : 0.0, 0.0, sh, &flag, dot, unused)) return;
-    AnState s2 = st;
+// The scalars of an ADBPG iteration after its second pass (tv_aniso.cpp:357-367, 461-480).
+__device__ __forceinline__ void adbpg_advance(AnState s2, const AnCall &c, bool test, double dot, AnState *out) {
     s2.since += 1;
     double t = s2.tn;
     if (test && dot > 0.0 && s2.since >= s2.last) {
@@ -916,36 +733,264 @@ __global__ void __launch_bounds__(kFmThreads) an_fm_unstage(AnGeom g, AnCall c, 
     s2.beta = (t - 1.0) / tn;
     s2.tn = tn;
     if (s2.it == s2.chk_next || s2.it == c.max_iter) s2.stage = kStCheck;
-    bf.st[b] = s2;
+    *out = s2;
 }
 
-// The edge weights of every strided axis, fibre-major (once per workspace).
+// Whether pass PASS of a round acts on image b (the stages of an_pass1 / an_pass2).
+template <int PASS>
+__device__ __forceinline__ bool fib_active(const AnState &st, const AnImage &im) {
+    if (st.status != kLive || im.mode != kAnAdbpg) return false;
+    return PASS == 1 ? (st.stage == kStIter || st.stage == kStWarm) : st.stage == kStIter;
+}
+
+// A segment's end and value at its last entry.
 template <class T>
-__global__ void __launch_bounds__(kFmThreads) an_weights_fm(AnGeom g, const T *__restrict__ beta, T *__restrict__ wt) {
-    __shared__ T tile[kFmTile][kFmTile + 1];
-    const int a = blockIdx.y;
-    const Fib fb = fibers(g, a);
-    if (fb.s == 1) return;
-    const int64_t N = g.N, L = fb.L;
-    const T *Bw = beta + (int64_t)a * N;
-    T *Wt = wt + (int64_t)a * N;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int64_t neg = (L + kFmTile - 1) / kFmTile, nt = fm_tiles(fb.nfib, L);
-    for (int64_t t = blockIdx.x; t < nt; t += gridDim.x) {
-        const int64_t f0 = (t / neg) * kFmTile, i0 = (t % neg) * kFmTile;
-#pragma unroll
-        for (int r = 0; r < kFmTile; r += 8) {
-            const int64_t f = f0 + tx, i = i0 + ty + r;
-            tile[ty + r][tx] = (f < fb.nfib && i < L) ? Bw[fb.base(f) + i * fb.s] : T(0);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < kFmTile; r += 8) {
-            const int64_t f = f0 + ty + r, i = i0 + tx;
-            if (f < fb.nfib && i < L) Wt[f * L + i] = tile[tx][ty + r];
-        }
-        __syncthreads();
+struct MarkSink {
+    T *val;
+    unsigned char *mark;
+    __device__ __forceinline__ void segment(int, int k1, double v) const {
+        val[k1] = (T)v;
+        mark[k1] = kMarkFinal;
     }
+    __device__ __forceinline__ void finish(int) const {}
+};
+
+// V: fibres of a strided axis per load (16 bytes where the rows allow, else 1).
+template <class T, int PASS, bool WT, int V>
+__global__ void __launch_bounds__(kFibThreads, sizeof(T) == 4 ? 4 : 2)
+an_fib_pass(AnGeom g, AnCall c, AnBuffers bf, FibCfg fc) {
+    extern __shared__ __align__(16) unsigned char an_fib_smem[];
+    __shared__ double sh[32];
+    __shared__ int flag;
+    constexpr int E = WT ? 2 : 1;
+    const int b = round_image(bf, blockIdx.y);
+    if (b < 0) return;
+    const AnState &st = bf.st[b];
+    const AnImage &im = bf.img[b];
+    if (!fib_active<PASS>(st, im)) return;
+    const int a = PASS == 1 ? im.a1 : im.a2;
+    const Fib fb = fibers(g, a);
+    const int n = (int)fb.L, nt = blockDim.x, tid = threadIdx.x, lane = tid & 31;
+    const int64_t N = g.N, f0 = (int64_t)blockIdx.x * fc.nf;
+    const int s = (int)fb.s;  // N < 2^31
+    const int nfb = (int)(fb.nfib - f0 < fc.nf ? fb.nfib - f0 : fc.nf);
+    T *yr = reinterpret_cast<T *>(an_fib_smem);
+    T *lv = yr + (size_t)E * fc.nf * fc.pitch;
+    T *rc = lv + (size_t)nt * kFibList;
+    int *le = reinterpret_cast<int *>(rc + n + 1);
+    unsigned char *marks = reinterpret_cast<unsigned char *>(le + nt * kFibList);
+    const int mpitch = (fc.pitch + 3) / 4 * 4;
+    {
+        const DivRecip<T> div;
+        for (int m = tid; m <= n; m += nt) rc[m] = m ? div(m) : T(0);
+        int *mw = reinterpret_cast<int *>(marks);
+        for (int i = tid; i < fc.nf * mpitch / 4; i += nt) mw[i] = 0;
+    }
+    const T *Bw = WT ? static_cast<const T *>(bf.beta) + (int64_t)a * N : nullptr;
+    const T lam = (T)im.lam[a];
+    // staging: y of the block's fibres and their radii (entry n - 1: 0)
+    const int ng = fc.nf / V, tx = tid % ng, ty = tid / ng, rows = nt / ng;
+    const int64_t ob = tx * V < nfb ? fb.base(f0 + tx * V) : 0;
+    {
+        const T *P0 = static_cast<const T *>(PASS == 1 ? bf.d : bf.u) + (int64_t)b * N;
+        const T *Wv = static_cast<const T *>(bf.wv) + (int64_t)b * g.k * N;
+        auto put = [&](T *q, int i, T p0, T w, T bw) {
+            q[i * E] = PASS == 1 ? p0 + w : p0 - w;
+            if (WT) q[i * E + 1] = i < n - 1 ? lam * bw : T(0);
+        };
+        if (s == 1) {
+            for (int f = tid >> 5; f < nfb; f += nt >> 5) {
+                const int64_t o = (f0 + f) * n;
+                const T *p0 = P0 + o, *wv = Wv + o, *bw = WT ? Bw + o : nullptr;
+                T *q = yr + (size_t)f * fc.pitch * E;
+#pragma unroll 8
+                for (int i = lane; i < n; i += 32) put(q, i, p0[i], wv[i], WT ? bw[i] : T(0));
+            }
+        } else if (tx * V < nfb) {
+            const T *p0 = P0 + ob, *wv = Wv + ob, *bw = WT ? Bw + ob : nullptr;
+            T *q = yr + (size_t)tx * V * fc.pitch * E;
+#pragma unroll 4
+            for (int i = ty; i < n; i += rows) {
+                T p[V], w[V], r[V];
+                load_pack<T, V>(p0 + i * s, p);
+                load_pack<T, V>(wv + i * s, w);
+                if (WT) load_pack<T, V>(bw + i * s, r);
+#pragma unroll
+                for (int j = 0; j < V; ++j) put(q + j * fc.pitch * E, i, p[j], w[j], WT ? r[j] : T(0));
+            }
+        }
+    }
+    __syncthreads();
+    // the scan: lane `sub` of a fibre's P lanes takes piece sub
+    const int fib = tid / fc.P, sub = tid & (fc.P - 1);
+    const bool act = fib < nfb;
+    T *q = yr + (size_t)fib * fc.pitch * E;
+    unsigned char *mark = marks + fib * mpitch;
+    T *val = static_cast<T *>(bf.segv) + (int64_t)b * N + (act ? (f0 + fib) * n : 0);
+    const int c0 = sub * fc.len < n ? sub * fc.len : n, c1 = c0 + fc.len < n ? c0 + fc.len : n;
+    bool live = false;
+    T l = lam;
+    {
+        // the fibre's range, its largest radius and whether one is zero (fiber_range)
+        T lo = Num<T>::inf(), hi = -Num<T>::inf(), rmax = T(0);
+        bool zero = false;
+        if (act) {
+#pragma unroll 4
+            for (int i = c0; i < c1; ++i) {
+                T v, r = T(0);
+                if (WT) {
+                    const Pair<T> yp = reinterpret_cast<const Pair<T> *>(q)[i];
+                    v = yp.y;
+                    r = yp.r;
+                } else {
+                    v = q[i];
+                }
+                lo = v < lo ? v : lo;
+                hi = v > hi ? v : hi;
+                if (WT) {
+                    zero = zero || (r == T(0) && i < n - 1);
+                    rmax = r > rmax ? r : rmax;
+                }
+            }
+        }
+        for (int o = fc.P >> 1; o > 0; o >>= 1) {
+            const T lo2 = __shfl_xor_sync(0xffffffffu, lo, o), hi2 = __shfl_xor_sync(0xffffffffu, hi, o);
+            lo = lo2 < lo ? lo2 : lo;
+            hi = hi2 > hi ? hi2 : hi;
+            if (WT) {
+                const T r2 = __shfl_xor_sync(0xffffffffu, rmax, o);
+                rmax = r2 > rmax ? r2 : rmax;
+                zero = __shfl_xor_sync(0xffffffffu, (int)zero, o) || zero;
+            }
+        }
+        const T range = hi - lo;
+        const T *bw = WT && act ? Bw + fb.base(f0 + fib) : nullptr;
+        if (WT && act && zero) {  // a zero weight, or a radius that underflowed
+            zero = false;
+            for (int i = 0; i < n - 1; ++i) zero = zero || bw[i * s] == T(0);
+        }
+        if (act) {
+            if (n == 1 || lam == T(0) || range == T(0)) {  // the fibre is its own prox
+                for (int i = c0; i < c1; ++i) {
+                    val[i] = q[i * E];
+                    mark[i] = kMarkFinal;
+                }
+            } else if (!WT && lam >= (T)(n / 2) * range) {  // no edge can be active: the mean
+                if (sub == 0) fiber_mean([&](int i) { return q[i * E]; }, MarkSink<T>{val, mark}, n);
+            } else if (WT && zero) {  // zero-weight edges: independent pieces, one lane
+                if (sub == 0)
+                    tv1d_fiber_sink<T>([&](int i) { return q[i * E]; }, MarkSink<T>{val, mark}, n, im.lam[a], true,
+                                       [&](int i) { return bw[i * s]; }, TableRecip<T>{rc});
+            } else {
+                live = true;
+                if (!WT) {
+                    const T cap = T(2) * (T)((n / 2) > 0 ? (n / 2) : 1) * range;
+                    l = lam < cap ? lam : cap;
+                } else if (rmax > T(2) * range) {  // radii clamped as in tv1d_fiber_sink (below 2 range none is)
+                    for (int i = c0; i < c1; ++i) {
+                        const T r = q[i * E + 1];
+                        const int jj = i + 1 < n - 1 - i ? i + 1 : n - 1 - i;
+                        const T cap = T(2) * (T)(jj > 0 ? jj : 1) * range;
+                        q[i * E + 1] = r < cap ? r : cap;
+                    }
+                }
+            }
+        }
+    }
+    __syncwarp();
+    tv1d_pieces<T, WT>(q, rc, l, n, fc.P, fc.len, sub, live, mark, val, le + tid * kFibList, lv + tid * kFibList,
+                       kFibList, bf.err);
+    __syncwarp();
+    // fill: a warp takes its fibres in turn, from their ends; entry i's value
+    // is that of the first valid segment end at or after it
+    {
+        const int per = 32 / fc.P, wf = (tid >> 5) * per;
+        T *U = static_cast<T *>(bf.u) + (int64_t)b * N;
+        for (int f = wf; f < wf + per && f < nfb; ++f) {
+            const unsigned char *mk = marks + f * mpitch;
+                    const T *vl = static_cast<const T *>(bf.segv) + (int64_t)b * N + (f0 + f) * n;
+            T *z = yr + (size_t)f * fc.pitch * E;
+            int carry = -1;
+            constexpr int kC = 4;  // chunks of 32 entries whose values are read together
+            for (int cb = (n - 1) >> 5; cb >= 0; cb -= kC) {
+                int idx[kC];
+#pragma unroll
+                for (int u = 0; u < kC; ++u) {
+                    const int i = (cb - u) * 32 + lane;
+                    const bool in = cb - u >= 0 && i < n;
+                    const unsigned w = __ballot_sync(0xffffffffu, in && mk[i] != 0);
+                    const unsigned up = w >> lane;
+                    idx[u] = in ? (up ? i + __ffs(up) - 1 : carry) : -1;
+                    carry = w ? (cb - u) * 32 + __ffs(w) - 1 : carry;
+                }
+                T v[kC];
+#pragma unroll
+                for (int u = 0; u < kC; ++u) v[u] = idx[u] >= 0 ? vl[idx[u]] : T(0);
+#pragma unroll
+                for (int u = 0; u < kC; ++u) {
+                    const int i = (cb - u) * 32 + lane;
+                    if (cb - u < 0 || i >= n) continue;
+                    if (idx[u] < 0) atomicExch(bf.err, 4);  // no end after i: a broken scan
+                    if (PASS == 1 && s == 1) U[(f0 + f) * n + i] = v[u];
+                    else z[i * E] = v[u];
+                }
+            }
+        }
+        if (PASS == 1 && s == 1) return;
+    }
+    __syncthreads();
+    // epilogue
+    const bool test = st.it % kCheck == 0;
+    double up = 0.0;
+    if (tx * V < nfb) {
+        const T beta = (T)st.beta;
+        T *U = static_cast<T *>(bf.u) + (int64_t)b * N + ob;
+        T *Wv = static_cast<T *>(bf.wv) + (int64_t)b * g.k * N + ob;
+        T *Yd = static_cast<T *>(bf.y) + (int64_t)b * g.k * N + ob;
+        T *Z = static_cast<T *>(bf.z) + (int64_t)b * N + ob;
+        const T *zs = yr + (size_t)tx * V * fc.pitch * E;
+        constexpr int kU = V > 1 ? 2 : 4;  // rows whose loads are in flight together
+        for (int i = ty; i < n; i += kU * rows) {
+            T u4[kU][V], w4[kU][V], y4[kU][V];
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                const int o = (i + u * rows < n ? i + u * rows : i) * s;
+                if (PASS == 2) {
+                    load_pack<T, V>(U + o, u4[u]);
+                    load_pack<T, V>(Wv + o, w4[u]);
+                    load_pack<T, V>(Yd + o, y4[u]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                const int ii = i + u * rows;
+                if (ii >= n) break;
+                T z[V];
+#pragma unroll
+                for (int j = 0; j < V; ++j) z[j] = zs[(j * fc.pitch + ii) * E];
+                if (PASS == 1) {
+                    store_pack<T, V>(U + ii * s, z);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < V; ++j) {
+                        const T w = w4[u][j], y = y4[u][j];
+                        const T v = u4[u][j] - w;
+                        const T yn = z[j] - v;
+                        if (test) up += (double)((w - yn) * (yn - y));
+                        w4[u][j] = yn + beta * (yn - y);
+                        y4[u][j] = yn;
+                    }
+                    store_pack<T, V>(Wv + ii * s, w4[u]);
+                    store_pack<T, V>(Yd + ii * s, y4[u]);
+                    store_pack<T, V>(Z + ii * s, z);
+                }
+            }
+        }
+    }
+    if (PASS == 1) return;
+    double dot, unused;
+    if (!reduce2(bf, b, blockIdx.x, gridDim.x, test ? up : 0.0, 0.0, sh, &flag, dot, unused)) return;
+    adbpg_advance(bf.st[b], c, test, dot, bf.st + b);
 }
 
 // ---------------------------------------------------------------------------
@@ -1644,6 +1689,8 @@ constexpr int kTileSmemMax = 200 * 1024;
 constexpr size_t kSmemPerSM = 228 * 1024;  // shared memory of an SM (sm_100)
 constexpr size_t kSmemReserve = 1024 + 512;  // per block: the system's and the kernels' static arrays
 constexpr int kSMs = 148;
+constexpr int kFibMany = 64;         // fibres per SM from which a piece pass has enough of them
+constexpr int kFibSmem = 72 * 1024;  // most shared memory of a block while it can hold fewer fibres
 
 // The tiled kernels may take up to kTileSmemMax of dynamic shared memory. Set
 // once per kernel, before any launch: the attribute is per function, and
@@ -1658,6 +1705,14 @@ void tile_attributes() {
     cudaFuncSetAttribute(an_pass1_tile<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax);
     cudaFuncSetAttribute(an_pass2_tile<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax);
     cudaFuncSetAttribute(an_fdpg3_tile<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax);
+    cudaFuncSetAttribute(an_fib_pass<T, 1, false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax);
+    cudaFuncSetAttribute(an_fib_pass<T, 1, false, kFibVec<T>>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax);
+    cudaFuncSetAttribute(an_fib_pass<T, 1, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax);
+    cudaFuncSetAttribute(an_fib_pass<T, 1, true, kFibVec<T>>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax);
+    cudaFuncSetAttribute(an_fib_pass<T, 2, false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax);
+    cudaFuncSetAttribute(an_fib_pass<T, 2, false, kFibVec<T>>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax);
+    cudaFuncSetAttribute(an_fib_pass<T, 2, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax);
+    cudaFuncSetAttribute(an_fib_pass<T, 2, true, kFibVec<T>>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax);
     done.fetch_or(bit);
 }
 
@@ -1724,13 +1779,50 @@ TileCfg tile_cfg(const AnGeom &g, const AnCall &c, int64_t nimg, size_t &smem) {
     return tc;
 }
 
-// The fibre-major scan keeps its table of 1/m (m <= L) in the default 48 KB
-// of shared memory.
+// The pieces of a pass along axis a: P lanes per fibre and nf fibres per block.
+// Shorter pieces mean shorter chains but more work (each piece scans about a
+// segment twice): launches with many fibres per SM fill it with pieces of 48
+// entries or more, others take pieces down to 10. Measured, ms a solve at
+// P = 4, 8, 16, 32: 64 x 512^2 (221 fibres per SM) 85, 75, 77, 96; 16 x 256^2
+// weighted (28) 13.0, 11.7, 11.9, 13.5; 4 x 1024^2 weighted (28) 59, 40, 32, 30;
+// 2048^2 (14) 63, 45, 38, 38; 200 x 301 (2) 7.9, 6.6, 6.0, 6.2; 90^2 (0.6) 2.6,
+// 2.2, 2.2, 2.3. Blocks of 64, 128 and 256 threads run alike; a block keeps to
+// kFibSmem so that an SM holds several. 0 fibres when one does not fit.
 template <class T>
-bool fm_fits(const AnGeom &g) {
-    for (int a = 0; a < g.k; ++a)
-        if ((size_t)(g.L[a] + 1) * sizeof(T) > 48 * 1024) return false;
-    return true;
+FibCfg fib_cfg(const AnGeom &g, int a, bool w, int64_t nimg, size_t &smem) {
+    const int L = (int)g.L[a];
+    const int64_t fibres = nimg * (g.N / g.L[a]);
+    FibCfg c{};
+    const int piece = fibres >= (int64_t)kSMs * kFibMany ? 48 : 10;
+    c.P = 1;
+    while (c.P < 32 && L / (2 * c.P) >= piece) c.P *= 2;
+    c.len = ((L + c.P - 1) / c.P) | 1;
+    c.pitch = L | 1;
+    // at least a warp, and 8 fibres (a 32-byte sector of floats) across a strided axis
+    const int lo = std::max(32 / c.P, g.S[a] == 1 ? 1 : std::min(8, kFibThreads / c.P));
+    c.nf = std::max(128 / c.P, lo);
+    while ((smem = fib_smem<T>(c, L, w)) > (size_t)kFibSmem && c.nf > lo) c.nf /= 2;
+    while ((smem = fib_smem<T>(c, L, w)) > (size_t)kTileSmemMax && c.nf > 32 / c.P) c.nf /= 2;
+    while (smem > (size_t)kTileSmemMax && c.P < 32) {
+        c.P *= 2;
+        c.nf = 32 / c.P;
+        c.len = ((L + c.P - 1) / c.P) | 1;
+        smem = fib_smem<T>(c, L, w);
+    }
+    if (smem > (size_t)kTileSmemMax) c.nf = 0;
+    return c;
+}
+
+template <class T, int PASS>
+cudaError_t fib_pass(const AnGeom &g, const AnCall &c, const AnBuffers &bf, const FibCfg &fc, size_t smem, int a,
+                     unsigned B, cudaStream_t s) {
+    const dim3 grid((unsigned)((g.N / g.L[a] + fc.nf - 1) / fc.nf), B);
+    // 16-byte loads across the fibres where every row starts on 16 bytes
+    const bool vec = g.S[a] > 1 && g.S[a] % kFibVec<T> == 0 && fc.nf % kFibVec<T> == 0;
+    auto run = [&](auto kernel) { kernel<<<grid, fc.nf * fc.P, smem, s>>>(g, c, bf, fc); };
+    if (c.has_beta) run(vec ? an_fib_pass<T, PASS, true, kFibVec<T>> : an_fib_pass<T, PASS, true, 1>);
+    else run(vec ? an_fib_pass<T, PASS, false, kFibVec<T>> : an_fib_pass<T, PASS, false, 1>);
+    return cudaGetLastError();
 }
 
 template <class T>
@@ -1747,39 +1839,28 @@ cudaError_t round_t(const AnGeom &g, const AnCall &c, const AnBuffers &bf, int64
     int64_t nfmax = 0;
     for (int a = 0; a < g.k; ++a) nfmax = std::max(nfmax, nf[a]);
     const unsigned fbk = (unsigned)((nfmax + 127) / 128);
-    if (c.has_adbpg && aniso_fm_enabled() && fm_fits<T>(g)) {
-        // the fibre-major passes: the active axes (the same for every image of
-        // the call), a1 the one of smaller stride
+    // the active axes of ADBPG (the same for every image of the call), a1 the
+    // one of smaller stride
+    bool pieces = false;
+    int a1 = 0, a2 = 0;
+    FibCfg fc1{}, fc2{};
+    size_t sm1 = 0, sm2 = 0;
+    if (c.has_adbpg && aniso_pieces_enabled()) {
         int act[3], n = 0;
         for (int a = 0; a < g.k; ++a)
             if (c.w[a] > 0.0 && g.L[a] > 1) act[n++] = a;
-        const int a1 = g.S[act[0]] < g.S[act[1]] ? act[0] : act[1], a2 = a1 == act[0] ? act[1] : act[0];
-        auto tiles_grid = [&](int a) {
-            if (g.S[a] == 1) return (unsigned)std::min<int64_t>((g.N + kFmThreads - 1) / kFmThreads, 1024);
-            return (unsigned)std::min<int64_t>(fm_tiles(nf[a], g.L[a]), 1024);
-        };
-        constexpr int per = kFmScan / 32 * kFmLanes;  // fibres per scan block
-        auto scan_grid = [&](int a) { return dim3((unsigned)((nf[a] + per - 1) / per), B); };
-        auto scan_smem = [&](int a) { return (size_t)(g.L[a] + 1) * sizeof(T); };
-        if (g.S[a1] == 1) {
-            an_fm_scan<T, 1, true><<<scan_grid(a1), kFmScan, scan_smem(a1), s>>>(g, c, bf);
-            nl += 1;
-        } else {
-            an_fm_stage<T, 1><<<dim3(tiles_grid(a1), B), kFmThreads, 0, s>>>(g, c, bf);
-            an_fm_scan<T, 1, false><<<scan_grid(a1), kFmScan, scan_smem(a1), s>>>(g, c, bf);
-            an_fm_unstage<T, 1><<<dim3(tiles_grid(a1), B), kFmThreads, 0, s>>>(g, c, bf);
-            nl += 3;
-        }
-        if (g.S[a2] == 1) {
-            an_fm_scan<T, 2, true><<<scan_grid(a2), kFmScan, scan_smem(a2), s>>>(g, c, bf);
-            nl += 1;
-        } else {
-            an_fm_stage<T, 2><<<dim3(tiles_grid(a2), B), kFmThreads, 0, s>>>(g, c, bf);
-            an_fm_scan<T, 2, false><<<scan_grid(a2), kFmScan, scan_smem(a2), s>>>(g, c, bf);
-            nl += 2;
-        }
-        an_fm_unstage<T, 2><<<dim3(tiles_grid(a2), B), kFmThreads, 0, s>>>(g, c, bf);
-        nl += 1;
+        a1 = g.S[act[0]] < g.S[act[1]] ? act[0] : act[1];
+        a2 = a1 == act[0] ? act[1] : act[0];
+        fc1 = fib_cfg<T>(g, a1, c.has_beta, nimg, sm1);
+        fc2 = fib_cfg<T>(g, a2, c.has_beta, nimg, sm2);
+        pieces = fc1.nf > 0 && fc2.nf > 0 && (nf[a2] + fc2.nf - 1) / fc2.nf <= bf.max_part;
+    }
+    if (pieces) {
+        tile_attributes<T>();
+        cudaError_t e = fib_pass<T, 1>(g, c, bf, fc1, sm1, a1, B, s);
+        if (e == cudaSuccess) e = fib_pass<T, 2>(g, c, bf, fc2, sm2, a2, B, s);
+        if (e != cudaSuccess) return e;
+        nl += 2;
     } else if (c.has_adbpg) {
         size_t smem = 0;
         const TileCfg tc = tile_cfg<T>(g, c, nimg, smem);
@@ -1870,24 +1951,12 @@ cudaError_t output_t(const AnGeom &g, const AnBuffers &bf, void *out, cudaStream
 
 }  // namespace
 
-bool aniso_fm_enabled() {
+bool aniso_pieces_enabled() {
     static const bool on = [] {  // tuning hint FASTPROX_B200_AN_FIB=0: the tiled passes
         const char *v = std::getenv("FASTPROX_B200_AN_FIB");
         return !(v && v[0] == '0' && v[1] == 0);
     }();
     return on;
-}
-
-cudaError_t aniso_weights_fm(int dtype, const AnGeom &g, const void *beta, void *wt, cudaStream_t s) {
-    int64_t nt = 1;
-    for (int a = 0; a < g.k; ++a) nt = std::max<int64_t>(nt, fm_tiles(g.N / g.L[a], g.L[a]));
-    const dim3 grid((unsigned)std::min<int64_t>(nt, 4096), (unsigned)g.k);
-    if (dtype == 1)
-        an_weights_fm<float><<<grid, kFmThreads, 0, s>>>(g, static_cast<const float *>(beta), static_cast<float *>(wt));
-    else
-        an_weights_fm<double>
-            <<<grid, kFmThreads, 0, s>>>(g, static_cast<const double *>(beta), static_cast<double *>(wt));
-    return cudaGetLastError();
 }
 
 int an_pixel_blocks(const AnGeom &g) {

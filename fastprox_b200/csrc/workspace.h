@@ -53,8 +53,7 @@ struct fp_workspace {
     uint8_t *an_flag = nullptr;
     int *an_parent = nullptr, *an_cnt = nullptr;
     unsigned long long *an_sum = nullptr;
-    void *an_ys = nullptr, *an_segv = nullptr, *an_wt = nullptr;  // the fibre-major passes
-    int *an_segk = nullptr;
+    void *an_segv = nullptr;  // the piece passes' segment values
     double *gammas = nullptr;
     double *part = nullptr;
     unsigned *ticket = nullptr;
