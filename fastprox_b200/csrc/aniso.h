@@ -103,8 +103,10 @@ cudaError_t aniso_setup(int dtype, const AnGeom &g, const AnCall &c, const AnBuf
 cudaError_t aniso_warm(int dtype, const AnGeom &g, const AnCall &c, const AnBuffers &bf, cudaStream_t s);
 // Kernel attributes the rounds need, set before the first capture or launch.
 void aniso_prepare(int dtype);
-// One round over nimg launch slots (g.B, or at least the count of bf's live list).
-cudaError_t aniso_round(int dtype, const AnGeom &g, const AnCall &c, const AnBuffers &bf, int64_t nimg,
+// One round over nimg launch slots (g.B, or at least the count of bf's live
+// list): an iteration and its check; with tail, the polish, the final rebuild
+// and retirement too (images that need them wait in their stage until then).
+cudaError_t aniso_round(int dtype, const AnGeom &g, const AnCall &c, const AnBuffers &bf, int64_t nimg, bool tail,
                         cudaStream_t s, int64_t *launches);
 // The list of live images (by their states), for bf.lmap / bf.lcnt.
 cudaError_t aniso_live_list(const AnState *st, int64_t B, int *lmap, int *lcnt, cudaStream_t s);

@@ -1058,10 +1058,14 @@ fp_status run_iso(fp_workspace *ws, const fp_op *op, const void *xsrc, void *zds
     return cuda_status(e);
 }
 
-// Anisotropic rounds per captured graph, and the solves that use graphs: a
-// round is about 15 launches, most of which exit at once, so a small solve is
-// bound by launch latency (a 64 x 64 image took 150 us a round in plain
-// launches). FASTPROX_B200_AN_GRAPHS=0 keeps plain launches.
+// Anisotropic rounds per captured graph, and the solves that use graphs: small
+// ones are bound by launch latency. The polish, the final rebuild and retirement
+// (10 launches that mostly exit at once) run in the last round of kAnChunk, with
+// graphs and without; an image that needs them waits, which costs it up to three
+// idle rounds of 3 launches per polish. Measured, ms a solve with them in every,
+// every second and every fourth round: 90^2 2.08, 1.89, 1.74; 16 x 256^2 10.1,
+// 9.3, 8.7; 64 x 512^2 weighted 138, 134, 132. FASTPROX_B200_AN_GRAPHS=0 keeps
+// plain launches.
 constexpr int kAnChunk = 4;
 constexpr int64_t kAnGraphPixels = int64_t(1) << 22;
 
@@ -1096,7 +1100,8 @@ bool an_graph_rounds(fp_workspace *ws, const AnGeom &g, const AnCall &c, const A
         int64_t nl = 0;
         cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            for (int r = 0; r < kAnChunk && e == cudaSuccess; ++r) e = aniso_round(ws->dtype, g, c, bf, nimg, cap, &nl);
+            for (int r = 0; r < kAnChunk && e == cudaSuccess; ++r)
+                e = aniso_round(ws->dtype, g, c, bf, nimg, r == kAnChunk - 1, cap, &nl);
             const cudaError_t e2 = cudaStreamEndCapture(cap, &graph);
             if (e == cudaSuccess) e = e2;
         }
@@ -1185,7 +1190,7 @@ fp_status run_aniso(fp_workspace *ws, const fp_op *op, const void *xsrc, void *z
     // after the first, small solves replay rounds in captured chunks
     int slot = 0, inflight = 0;
     int64_t rounds = 0, nimg = g.B;
-    const int64_t cap = (int64_t)max_iter + 4;
+    const int64_t cap = ((int64_t)max_iter + 4) * (kAnChunk + 1);
     bool done = false;
     bool graphs = an_graphs_enabled() && g.N * g.B <= kAnGraphPixels;
     while (!done) {
@@ -1193,8 +1198,8 @@ fp_status run_aniso(fp_workspace *ws, const fp_op *op, const void *xsrc, void *z
             rounds += kAnChunk;
         } else {
             if (rounds > 0) graphs = false;
-            e = aniso_round(ws->dtype, g, c, bf, nimg, s, &launches);
             ++rounds;
+            e = aniso_round(ws->dtype, g, c, bf, nimg, rounds % kAnChunk == 0, s, &launches);
         }
         if (e != cudaSuccess) return cuda_status(e);
         e = cudaMemcpyAsync(ws->h_live + slot, ws->live, sizeof(int), cudaMemcpyDeviceToHost, s);

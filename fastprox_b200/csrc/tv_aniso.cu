@@ -130,6 +130,52 @@ __device__ __forceinline__ bool reduce2(const AnBuffers &bf, int b, unsigned blk
     return true;
 }
 
+// The same over a partition of an image's pixels into nch chunks (chunk q: the
+// pixels q T + t + j nch T of thread t of T) that does not depend on the grid:
+// each block takes chunks in turn, acc(p) summed over a thread's pixels of the
+// chunk. Batches launch few blocks per image, so that a launch whose images are
+// all in other stages costs little (64 x 512^2: 16384 blocks that return at
+// once took 35 us, 2368 take 5).
+template <class F>
+__device__ __forceinline__ bool reduce_chunks(const AnBuffers &bf, int b, int64_t N, int nch, const F &term, double *sh,
+                                              int *flag, double &total) {
+    double *part = img_part(bf, b);
+    for (int q = blockIdx.x; q < nch; q += gridDim.x) {
+        double acc = 0.0;
+        for (int64_t p = (int64_t)q * blockDim.x + threadIdx.x; p < N; p += (int64_t)nch * blockDim.x) acc += term((int)p);
+        const double s0 = block_sum(acc, sh);
+        if (threadIdx.x == 0) part[q * 2] = s0;
+    }
+    if (!arrive_last(bf.ticket + b, gridDim.x, flag)) return false;
+    total = sum_partials(part, nch, 2, 0, sh);
+    if (threadIdx.x != 0) return false;
+    bf.ticket[b] = 0;
+    return true;
+}
+
+// Chunks of an image (blocks of a launch over one image), at most 256.
+__host__ __device__ __forceinline__ int pixel_chunks(int64_t N) {
+    const int64_t nb = (N + kThreads * 4 - 1) / (kThreads * 4);
+    return (int)(nb < 1 ? 1 : (nb > 256 ? 256 : nb));
+}
+
+// The coordinates of pixel p (axis 0 slowest).
+__device__ __forceinline__ void coords(const AnGeom &g, int p, int co[3]) {
+    unsigned q = (unsigned)p;
+#pragma unroll
+    for (int a = 2; a >= 0; --a) {
+        co[a] = 0;
+        if (a >= g.k) continue;
+        if (a == 0) {
+            co[0] = (int)q;
+        } else {
+            const unsigned L = (unsigned)g.L[a], t = q / L;
+            co[a] = (int)(q - t * L);
+            q = t;
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Set-up (tv_aniso.cpp:260-340)
 // ---------------------------------------------------------------------------
@@ -793,7 +839,8 @@ an_fib_pass(AnGeom g, AnCall c, AnBuffers bf, FibCfg fc) {
     const int64_t ob = tx * V < nfb ? fb.base(f0 + tx * V) : 0;
     {
         const T *P0 = static_cast<const T *>(PASS == 1 ? bf.d : bf.u) + (int64_t)b * N;
-        const T *Wv = static_cast<const T *>(bf.wv) + (int64_t)b * g.k * N;
+        // after a restart the extrapolated dual is y itself (tv_aniso.cpp:474-477)
+        const T *Wv = static_cast<const T *>(st.restart ? bf.y : bf.wv) + (int64_t)b * g.k * N;
         auto put = [&](T *q, int i, T p0, T w, T bw) {
             q[i * E] = PASS == 1 ? p0 + w : p0 - w;
             if (WT) q[i * E + 1] = i < n - 1 ? lam * bw : T(0);
@@ -948,6 +995,7 @@ an_fib_pass(AnGeom g, AnCall c, AnBuffers bf, FibCfg fc) {
         T *Wv = static_cast<T *>(bf.wv) + (int64_t)b * g.k * N + ob;
         T *Yd = static_cast<T *>(bf.y) + (int64_t)b * g.k * N + ob;
         T *Z = static_cast<T *>(bf.z) + (int64_t)b * N + ob;
+        const T *Ws = st.restart ? Yd : Wv;
         const T *zs = yr + (size_t)tx * V * fc.pitch * E;
         constexpr int kU = V > 1 ? 2 : 4;  // rows whose loads are in flight together
         for (int i = ty; i < n; i += kU * rows) {
@@ -957,7 +1005,7 @@ an_fib_pass(AnGeom g, AnCall c, AnBuffers bf, FibCfg fc) {
                 const int o = (i + u * rows < n ? i + u * rows : i) * s;
                 if (PASS == 2) {
                     load_pack<T, V>(U + o, u4[u]);
-                    load_pack<T, V>(Wv + o, w4[u]);
+                    load_pack<T, V>(Ws + o, w4[u]);
                     load_pack<T, V>(Yd + o, y4[u]);
                 }
             }
@@ -1230,16 +1278,17 @@ __global__ void __launch_bounds__(128) an_fdpg3_primal(AnGeom g, AnCall c, AnBuf
 
 template <class T>
 __device__ __forceinline__ double tv_at(const AnGeom &g, const AnCall &c, const AnBuffers &bf, const AnImage &im,
-                                        const T *Z, int64_t p, int64_t Nimg) {
+                                        const T *Z, int p, double z) {
     double s = 0.0;
+    int co[3];
+    coords(g, p, co);
     for (int a = 0; a < g.k; ++a) {
         const double l = im.lam[a];
         if (l == 0.0) continue;
-        const int64_t co = (p / g.S[a]) % g.L[a];
-        if (co + 1 >= g.L[a]) continue;
+        if (co[a] + 1 >= g.L[a]) continue;
         double le = l;
-        if (c.has_beta) le = l * (double)static_cast<const T *>(bf.beta)[(int64_t)a * Nimg + p];
-        s += le * fabs((double)Z[p + g.S[a]] - (double)Z[p]);
+        if (c.has_beta) le = l * (double)static_cast<const T *>(bf.beta)[(int64_t)a * g.N + p];
+        s += le * fabs((double)Z[p + g.S[a]] - z);
     }
     return s;
 }
@@ -1277,13 +1326,12 @@ __global__ void __launch_bounds__(kThreads) an_gap(AnGeom g, AnCall c, AnBuffers
     const int64_t N = g.N;
     const T *D = static_cast<const T *>(bf.d) + (int64_t)b * N;
     const T *Z = static_cast<const T *>(stage == kStCheck ? bf.z : bf.zp) + (int64_t)b * N;
-    double acc = 0.0;
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += (int64_t)gridDim.x * blockDim.x) {
+    auto term = [&](int p) {
         const double z = (double)Z[p];
-        acc += tv_at<T>(g, c, bf, im, Z, p, N) - z * ((double)D[p] - z);
-    }
-    double gz, unused;
-    if (!reduce2(bf, b, blockIdx.x, gridDim.x, acc, 0.0, sh, &flag, gz, unused)) return;
+        return tv_at<T>(g, c, bf, im, Z, p, z) - z * ((double)D[p] - z);
+    };
+    double gz;
+    if (!reduce_chunks(bf, b, N, pixel_chunks(N), term, sh, &flag, gz)) return;
     AnState s2 = st;
     if (stage == kStFinal) {
         // d - q1 - q2 in place of the iterate, unless rounding alone takes its
@@ -1367,46 +1415,141 @@ __global__ void an_dual(AnGeom g, AnBuffers bf, int stage) {
 // mark_edges (tv_aniso.cpp:256-297) along axis a: the 1D dual of each edge
 // from the running sum of q_a along its fibre; an edge strictly inside its
 // bound is flat (bit a), the others move lam_e sign(p_e) from j to i in zp.
+// The running sums are formed by parts (a thread walking a whole fibre took
+// 500 us on 64 x 512^2 and 600 on one 1400^2 image, all of it the wait for one
+// load after another).
 template <class T>
-__global__ void __launch_bounds__(128) an_mark(AnGeom g, AnCall c, AnBuffers bf, int a) {
+struct EdgeMark {
+    const T *q, *bw;
+    double lam;
+    // Whether edge i (pe its dual) is flat, else ls = lam_e sign(p_e).
+    __device__ __forceinline__ bool flat(int64_t o, double pe, double &ls) const {
+        const double lb = bw ? lam * (double)bw[o] : lam;
+        ls = copysign(lb, pe);
+        return fabs(pe) < lb * (1.0 - polish_eta<T>());
+    }
+};
+// zp of entry i from the edges before and after it, in that order.
+template <class T>
+__device__ __forceinline__ T moved(T z, bool before, double lsb, bool after, double lsa) {
+    if (before) z = (T)((double)z - lsb);
+    if (after) z = (T)((double)z + lsa);
+    return z;
+}
+
+// A strided axis: kMarkCols fibres side by side (adjacent in memory), each cut
+// into kMarkParts parts whose sums come first.
+constexpr int kMarkCols = 32, kMarkParts = 16;
+
+template <class T>
+__global__ void __launch_bounds__(kMarkCols *kMarkParts) an_mark_cols(AnGeom g, AnCall c, AnBuffers bf, int a) {
+    __shared__ double part[kMarkParts][kMarkCols];
     const int b = round_image(bf, blockIdx.y);
     if (b < 0) return;
     const AnState &st = bf.st[b];
     if (st.status != kLive || st.stage != kStPolish) return;
-    const AnImage &im = bf.img[b];
-    const double lam = im.lam[a];
+    const double lam = bf.img[b].lam[a];
     if (lam == 0.0) return;
     const Fib fb = fibers(g, a);
-    const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= fb.nfib) return;
-    const int64_t N = g.N, base = fb.base(f), s = fb.s;
-    const T *Q = static_cast<const T *>(bf.dual) + ((int64_t)a * g.B + b) * N + base;
-    const T *Bw = c.has_beta ? static_cast<const T *>(bf.beta) + (int64_t)a * N + base : nullptr;
-    T *ZP = static_cast<T *>(bf.zp) + (int64_t)b * N + base;
-    uint8_t *F = bf.flag + (int64_t)b * N + base;
+    const int tx = threadIdx.x % kMarkCols, ty = threadIdx.x / kMarkCols;
+    const int64_t N = g.N, s = fb.s;
+    const int n = (int)fb.L, len = (n + kMarkParts - 1) / kMarkParts;
     const uint8_t bit = (uint8_t)(1u << a);
-    double acc = 0.0;
-    // zp of the edge's first entry is carried in a register from the last
-    // edge (which may have changed it), so no step waits on its own store
-    T zc = ZP[0];
-    for (int64_t l = 0; l + 1 < fb.L; ++l) {
-        const int64_t o = l * s;
-        T zn = ZP[o + s];
-        acc += (double)Q[o];
-        const double pe = -acc;
-        const double lb = Bw ? lam * (double)Bw[o] : lam;
-        const bool inside = fabs(pe) < lb * (1.0 - polish_eta<T>());
-        if (inside) {
-            F[o] |= bit;
-        } else {
-            const double ls = copysign(lb, pe);
-            zc = (T)((double)zc + ls);
-            zn = (T)((double)zn - ls);
+    for (int64_t f0 = (int64_t)blockIdx.x * kMarkCols; f0 < fb.nfib; f0 += (int64_t)gridDim.x * kMarkCols) {
+        const int64_t f = f0 + tx;
+        const bool act = f < fb.nfib;
+        const int64_t base = act ? fb.base(f) : 0;
+        const T *Q = static_cast<const T *>(bf.dual) + ((int64_t)a * g.B + b) * N + base;
+        const EdgeMark<T> em{Q, c.has_beta ? static_cast<const T *>(bf.beta) + (int64_t)a * N + base : nullptr, lam};
+        T *ZP = static_cast<T *>(bf.zp) + (int64_t)b * N + base;
+        uint8_t *F = bf.flag + (int64_t)b * N + base;
+        const int i0 = ty * len < n ? ty * len : n, i1 = i0 + len < n ? i0 + len : n;
+        double acc = 0.0;
+        if (act) {
+#pragma unroll 8
+            for (int i = i0; i < i1; ++i) acc += (double)Q[i * s];
         }
-        ZP[o] = zc;
-        zc = zn;
+        part[ty][tx] = acc;
+        __syncthreads();
+        acc = 0.0;
+        for (int j = 0; j < ty; ++j) acc += part[j][tx];
+        __syncthreads();
+        if (act && i0 < i1) {
+            double lsb = 0.0;
+            bool before = i0 > 0 && !em.flat((i0 - 1) * s, -acc, lsb);
+#pragma unroll 4
+            for (int i = i0; i < i1; ++i) {
+                const int64_t o = i * s;
+                const bool edge = i + 1 < n;
+                acc += (double)Q[o];
+                double ls;
+                const bool flat = em.flat(o, -acc, ls);
+                if (edge && flat) F[o] |= bit;
+                const bool after = edge && !flat;
+                ZP[o] = moved(ZP[o], before, lsb, after, ls);
+                before = after;
+                lsb = ls;
+            }
+        }
     }
-    ZP[(fb.L - 1) * s] = zc;
+}
+
+// The contiguous axis: a warp per fibre, 32 entries at a time by a warp scan.
+// It also starts the components (parent): within 32 entries, those joined by
+// flat edges point to the first of them.
+template <class T>
+__global__ void __launch_bounds__(kThreads) an_mark_rows(AnGeom g, AnCall c, AnBuffers bf, int a) {
+    const int b = round_image(bf, blockIdx.y);
+    if (b < 0) return;
+    const AnState &st = bf.st[b];
+    if (st.status != kLive || st.stage != kStPolish) return;
+    const double lam = bf.img[b].lam[a];
+    if (lam == 0.0) return;
+    const int64_t N = g.N, nfib = N / g.L[a];
+    const int n = (int)g.L[a], lane = threadIdx.x & 31;
+    const uint8_t bit = (uint8_t)(1u << a);
+    for (int64_t f = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); f < nfib;
+         f += (int64_t)gridDim.x * (kThreads / 32)) {
+        const int64_t base = f * n;
+        const T *Q = static_cast<const T *>(bf.dual) + ((int64_t)a * g.B + b) * N + base;
+        const EdgeMark<T> em{Q, c.has_beta ? static_cast<const T *>(bf.beta) + (int64_t)a * N + base : nullptr, lam};
+        T *ZP = static_cast<T *>(bf.zp) + (int64_t)b * N + base;
+        uint8_t *F = bf.flag + (int64_t)b * N + base;
+        int *P = bf.parent + (int64_t)b * N + base;
+        double carry = 0.0, lsc = 0.0;  // the sum and the last edge of the entries before
+        bool beforec = false;
+        for (int c0 = 0; c0 < n; c0 += 32) {
+            const int i = c0 + lane;
+            const bool in = i < n, edge = i + 1 < n;
+            double x = in ? (double)Q[i] : 0.0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const double y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            x += carry;
+            carry = __shfl_sync(0xffffffffu, x, 31);
+            double ls = 0.0;
+            const bool flat = edge && em.flat(i, -x, ls);
+            const bool after = edge && !flat;
+            double lsb = __shfl_up_sync(0xffffffffu, ls, 1);
+            const unsigned am = __ballot_sync(0xffffffffu, after), fm = __ballot_sync(0xffffffffu, flat);
+            bool before = lane > 0 && (am >> (lane - 1) & 1u);
+            if (lane == 0) {
+                before = beforec;
+                lsb = lsc;
+            }
+            if (in) {
+                if (flat) F[i] |= bit;
+                ZP[i] = moved(ZP[i], before, lsb, after, ls);
+                // the last entry at or before this one that no flat edge joins to the one before
+                const unsigned heads = ~(fm << 1) & (0xffffffffu >> (31 - lane));
+                P[i] = (int)(base + c0 + 31 - __clz(heads));
+            }
+            beforec = am >> 31 & 1u;
+            lsc = __shfl_sync(0xffffffffu, ls, 31);
+        }
+    }
 }
 
 __device__ __forceinline__ int uf_find(int *P, int i) {
@@ -1423,7 +1566,10 @@ __device__ __forceinline__ int uf_find(int *P, int i) {
 
 // components (tv_aniso.cpp:324-439) by union-find: the flat edges join
 // their ends, the larger root hooked under the smaller by compare-and-swap,
-// so each root is the smallest index of its component.
+// so each root is the smallest index of its component. Along the contiguous
+// axis an_mark_rows has joined every 32 entries already; a flat edge of another
+// axis whose neighbour on the left is flat too, and joined to it at both ends,
+// adds nothing. (The unions of every edge took 621 us on 64 x 512^2.)
 __global__ void an_union(AnGeom g, AnBuffers bf) {
     const int b = round_image(bf, blockIdx.y);
     if (b < 0) return;
@@ -1432,11 +1578,21 @@ __global__ void an_union(AnGeom g, AnBuffers bf) {
     const int64_t N = g.N;
     const uint8_t *F = bf.flag + (int64_t)b * N;
     int *P = bf.parent + (int64_t)b * N;
+    const int last = g.k - 1;
+    const unsigned row = 1u << last;  // the contiguous axis' bit
+    const unsigned L = (unsigned)g.L[last];
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += (int64_t)gridDim.x * blockDim.x) {
         const uint8_t fl = F[p];
         if (!fl) continue;
+        const unsigned co = (unsigned)p % L;
         for (int a = 0; a < g.k; ++a) {
             if (!(fl & (1u << a))) continue;
+            if (a == last) {
+                if ((co & 31) != 31) continue;
+            } else if (co > 0) {
+                const unsigned fq = F[p - 1], fr = F[p - 1 + g.S[a]];
+                if ((fq & row) && (fr & row) && (fq & (1u << a))) continue;
+            }
             int x = (int)p, y = (int)(p + g.S[a]);
             int tries = 0;
             for (;;) {
@@ -1470,25 +1626,77 @@ __device__ __forceinline__ int uf_root(const int *P, int i) {
     return i;
 }
 
-// every entry to its root; the region sums of zp (64-bit fixed point) and sizes
+// every entry to its root; the region sums of zp (64-bit fixed point) and
+// sizes. A warp takes kRunSegs x 32 consecutive entries; while all 32 lie in
+// the region of the last ones each lane adds its own, else the entries are
+// added run by run (equal roots side by side), one atomic per run and sum: an
+// atomic per entry took 2.5 ms on 64 x 512^2 and 1.3 ms on one 1400^2 image,
+// nearly all of them on the few largest regions. The sums are integers, so
+// their order does not matter.
+constexpr int kRunSegs = 16;
+
 template <class T>
-__global__ void an_region_sum(AnGeom g, AnBuffers bf) {
+__global__ void __launch_bounds__(kThreads) an_region_sum(AnGeom g, AnBuffers bf) {
     const int b = round_image(bf, blockIdx.y);
     if (b < 0) return;
     const AnState &st = bf.st[b];
     if (st.status != kLive || st.stage != kStPolish) return;
     const int64_t N = g.N;
-    const int sh = bf.img[b].fx_shift;
+    const int sh = bf.img[b].fx_shift, lane = threadIdx.x & 31;
     int *P = bf.parent + (int64_t)b * N;
     const T *ZP = static_cast<const T *>(bf.zp) + (int64_t)b * N;
     unsigned long long *S = bf.sum + (int64_t)b * N;
     int *C = bf.cnt + (int64_t)b * N;
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += (int64_t)gridDim.x * blockDim.x) {
-        const int r = uf_root(P, (int)p);
-        P[p] = r;
-        const long long fx = llrint(ldexp((double)ZP[p], sh));
-        atomicAdd(S + r, (unsigned long long)fx);
-        atomicAdd(C + r, 1);
+    const int64_t warps = (int64_t)gridDim.x * (kThreads / 32), w0 = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    for (int64_t w = w0; w * (kRunSegs * 32) < N; w += warps) {
+        unsigned long long acc = 0;
+        int root = -1, cnt = 0;  // the region the lanes are adding up (warp-uniform), 32 entries cnt times
+        auto flush = [&]() {
+            if (cnt == 0) return;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+            if (lane == 0) {
+                atomicAdd(S + root, acc);
+                atomicAdd(C + root, 32 * cnt);
+            }
+            acc = 0;
+            cnt = 0;
+        };
+        for (int j = 0; j < kRunSegs; ++j) {
+            const int64_t p = (w * kRunSegs + j) * 32 + lane;
+            if (p - lane >= N) break;
+            const bool in = p < N;
+            int r = -1;
+            unsigned long long fx = 0;
+            if (in) {
+                r = uf_root(P, (int)p);
+                P[p] = r;
+                fx = (unsigned long long)llrint(ldexp((double)ZP[p], sh));
+            }
+            const int r31 = __shfl_sync(0xffffffffu, r, 31);
+            if (__all_sync(0xffffffffu, in && r == r31)) {
+                if (r31 != root) flush();
+                root = r31;
+                acc += fx;
+                ++cnt;
+                continue;
+            }
+            // run sums from the inclusive scan, at each run's last lane
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long y = __shfl_up_sync(0xffffffffu, fx, o);
+                if (lane >= o) fx += y;
+            }
+            const int rl = __shfl_up_sync(0xffffffffu, r, 1), rn = __shfl_down_sync(0xffffffffu, r, 1);
+            const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || r != rl);
+            const int first = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+            const unsigned long long before = __shfl_sync(0xffffffffu, fx, first > 0 ? first - 1 : 0);
+            if (in && (lane == 31 || r != rn)) {
+                atomicAdd(S + r, fx - (first > 0 ? before : 0ull));
+                atomicAdd(C + r, lane - first + 1);
+            }
+        }
+        flush();
     }
 }
 
@@ -1510,35 +1718,33 @@ __global__ void __launch_bounds__(kThreads) an_polish_gap(AnGeom g, AnCall c, An
     const int *C = bf.cnt + (int64_t)b * N;
     const T *D = static_cast<const T *>(bf.d) + (int64_t)b * N;
     const T *Q = static_cast<const T *>(bf.dual);
-    T *ZP = static_cast<T *>(bf.zp) + (int64_t)b * N;
-    auto mean = [&](int64_t p) -> double {
+    auto mean = [&](int r) -> double { return ldexp((double)(long long)S[r], -shf) / (double)C[r]; };
+    auto term = [&](int p) {
         const int r = P[p];
-        return ldexp((double)(long long)S[r], -shf) / (double)C[r];
-    };
-    double acc = 0.0;
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += (int64_t)gridDim.x * blockDim.x) {
-        const double zp = mean(p);
+        const double zp = mean(r);
         const double d = (double)D[p];
         const double e = zp - d;
         double sj = 0.0;
         for (int a = 0; a < g.k; ++a) sj += (double)Q[((int64_t)a * B + b) * N + p];
         double tv = 0.0;
+        int co[3];
+        coords(g, p, co);
         for (int a = 0; a < g.k; ++a) {
             const double l = im.lam[a];
             if (l == 0.0) continue;
-            const int64_t co = (p / g.S[a]) % g.L[a];
-            if (co + 1 >= g.L[a]) continue;
+            if (co[a] + 1 >= g.L[a]) continue;
+            const int rn = P[p + g.S[a]];
+            if (rn == r) continue;  // the same region: no jump
             double le = l;
             if (c.has_beta) le = l * (double)static_cast<const T *>(bf.beta)[(int64_t)a * N + p];
-            tv += le * fabs(mean(p + g.S[a]) - zp);
+            tv += le * fabs(mean(rn) - zp);
         }
-        acc += 0.5 * e * e - (d * sj - 0.5 * sj * sj) + tv;
-    }
-    // write the means after every block of this image has read them: the
-    // last block does it (below); here only the gap
-    double pz, unused;
-    if (!reduce2(bf, b, blockIdx.x, gridDim.x, acc, 0.0, sh, &flag, pz, unused)) return;
-    (void)ZP;
+        return 0.5 * e * e - (d * sj - 0.5 * sj * sj) + tv;
+    };
+    // the means are written after every block of this image has read the sums
+    // (an_polish_write); here only the gap
+    double pz;
+    if (!reduce_chunks(bf, b, N, pixel_chunks(N), term, sh, &flag, pz)) return;
     AnState s2 = st;
     const double gz = s2.gz;
     const bool last = s2.it == c.max_iter;
@@ -1580,24 +1786,19 @@ __global__ void an_polish_write(AnGeom g, AnBuffers bf) {
     }
 }
 
-// images whose stage is done leave the live set
+// images whose stage is done leave the live set (a final rebuild is not needed
+// after a polish or at it = 0, nor by FDPG-3)
 __global__ void an_retire(AnGeom g, AnBuffers bf) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= g.B) return;
     AnState &st = bf.st[b];
     st.pol_accept = 0;
-    if (st.status == kLive && (st.stage == kStDone || (st.stage == kStFinal && bf.img[b].mode == kAnFdpg3))) {
+    if (st.status == kLive &&
+        (st.stage == kStDone ||
+         (st.stage == kStFinal && (bf.img[b].mode == kAnFdpg3 || st.polished || st.it == 0)))) {
         st.status = st.gp <= bf.img[b].target ? kConverged : kNotConv;
         atomicSub(bf.live, 1);
     }
-}
-
-// a final rebuild is not needed after a polish or at it = 0: done
-__global__ void an_final_skip(AnGeom g, AnBuffers bf) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= g.B) return;
-    AnState &st = bf.st[b];
-    if (st.status == kLive && st.stage == kStFinal && (st.polished || st.it == 0)) st.stage = kStDone;
 }
 
 // ---------------------------------------------------------------------------
@@ -1689,7 +1890,6 @@ constexpr int kTileSmemMax = 200 * 1024;
 constexpr size_t kSmemPerSM = 228 * 1024;  // shared memory of an SM (sm_100)
 constexpr size_t kSmemReserve = 1024 + 512;  // per block: the system's and the kernels' static arrays
 constexpr int kSMs = 148;
-constexpr int kFibMany = 64;         // fibres per SM from which a piece pass has enough of them
 constexpr int kFibSmem = 72 * 1024;  // most shared memory of a block while it can hold fewer fibres
 
 // The tiled kernels may take up to kTileSmemMax of dynamic shared memory. Set
@@ -1781,21 +1981,23 @@ TileCfg tile_cfg(const AnGeom &g, const AnCall &c, int64_t nimg, size_t &smem) {
 
 // The pieces of a pass along axis a: P lanes per fibre and nf fibres per block.
 // Shorter pieces mean shorter chains but more work (each piece scans about a
-// segment twice): launches with many fibres per SM fill it with pieces of 48
-// entries or more, others take pieces down to 10. Measured, ms a solve at
-// P = 4, 8, 16, 32: 64 x 512^2 (221 fibres per SM) 85, 75, 77, 96; 16 x 256^2
-// weighted (28) 13.0, 11.7, 11.9, 13.5; 4 x 1024^2 weighted (28) 59, 40, 32, 30;
-// 2048^2 (14) 63, 45, 38, 38; 200 x 301 (2) 7.9, 6.6, 6.0, 6.2; 90^2 (0.6) 2.6,
-// 2.2, 2.2, 2.3. Blocks of 64, 128 and 256 threads run alike; a block keeps to
-// kFibSmem so that an SM holds several. 0 fibres when one does not fit.
+// segment twice): pieces have at most 64 entries, and fewer (down to 10) while
+// the fibres in flight (the launch's, or those an SM's shared memory holds)
+// would give an SM fewer than 8 warps. Measured, ms a solve at P = 4, 8, 16, 32:
+// 64 x 512^2 (221 fibres per SM) 85, 75, 77, 96; 16 x 256^2 weighted (28) 13.0,
+// 11.7, 11.9, 13.5; 4 x 1024^2 weighted (28) 59, 40, 32, 30; 2048^2 (14) 63,
+// 45, 38, 38; 200 x 301 (2) 7.9, 6.6, 6.0, 6.2; 90^2 (0.6) 2.6, 2.2, 2.2, 2.3.
+// Blocks of 64, 128 and 256 threads run alike; a block keeps to kFibSmem so
+// that an SM holds several. 0 fibres when one does not fit.
 template <class T>
 FibCfg fib_cfg(const AnGeom &g, int a, bool w, int64_t nimg, size_t &smem) {
     const int L = (int)g.L[a];
     const int64_t fibres = nimg * (g.N / g.L[a]);
     FibCfg c{};
-    const int piece = fibres >= (int64_t)kSMs * kFibMany ? 48 : 10;
     c.P = 1;
-    while (c.P < 32 && L / (2 * c.P) >= piece) c.P *= 2;
+    const int64_t one = (int64_t)(w ? 2 : 1) * L * (int64_t)sizeof(T) + L;  // a fibre's shared memory
+    const double flight = std::min((double)fibres / kSMs, (double)kSmemPerSM / (double)std::max<int64_t>(one, 1));
+    while (c.P < 32 && (L > 64 * c.P || (flight * c.P < 8 * 32 && L / (2 * c.P) >= 10))) c.P *= 2;
     c.len = ((L + c.P - 1) / c.P) | 1;
     c.pitch = L | 1;
     // at least a warp, and 8 fibres (a 32-byte sector of floats) across a strided axis
@@ -1826,13 +2028,14 @@ cudaError_t fib_pass(const AnGeom &g, const AnCall &c, const AnBuffers &bf, cons
 }
 
 template <class T>
-cudaError_t round_t(const AnGeom &g, const AnCall &c, const AnBuffers &bf, int64_t nimg, cudaStream_t s,
+cudaError_t round_t(const AnGeom &g, const AnCall &c, const AnBuffers &bf, int64_t nimg, bool tail, cudaStream_t s,
                    int64_t *launches) {
     if (nimg <= 0) return cudaSuccess;
     const unsigned B = (unsigned)nimg;
     int64_t nl = 0;
-    const int pb = an_pixel_blocks(g);
-    const dim3 pg(pb, B);
+    // blocks per image: enough for the SMs, no more than the image has chunks
+    const int64_t per = std::max<int64_t>(1, (int64_t)kSMs * 16 / B);
+    const dim3 pg((unsigned)std::min<int64_t>(an_pixel_blocks(g), per), B);
     // the iteration: ADBPG's two passes, or FDPG-3's three
     int64_t nf[3] = {1, 1, 1};
     for (int a = 0; a < g.k; ++a) nf[a] = g.N / g.L[a];
@@ -1898,8 +2101,10 @@ cudaError_t round_t(const AnGeom &g, const AnCall &c, const AnBuffers &bf, int64
         }
         nl += 2;
     }
-    an_restart_copy<T><<<pg, kThreads, 0, s>>>(g, bf);
-    ++nl;
+    if (!pieces) {  // the piece passes read y in place of the extrapolation after a restart
+        an_restart_copy<T><<<pg, kThreads, 0, s>>>(g, bf);
+        ++nl;
+    }
     if (c.warm && c.has_adbpg) {
         // a warm start's pass (run by the first pass above) and its dual
         an_warm_z<T><<<pg, kThreads, 0, s>>>(g, bf);
@@ -1913,21 +2118,32 @@ cudaError_t round_t(const AnGeom &g, const AnCall &c, const AnBuffers &bf, int64
     }
     an_gap<T><<<pg, kThreads, 0, s>>>(g, c, bf, kStCheck);
     ++nl;
-    // polish
-    an_dual<T><<<pg, kThreads, 0, s>>>(g, bf, kStPolish);
-    for (int a = 0; a < g.k; ++a) an_mark<T><<<dim3((unsigned)((nf[a] + 127) / 128), B), 128, 0, s>>>(g, c, bf, a);
-    an_union<<<pg, kThreads, 0, s>>>(g, bf);
-    an_region_sum<T><<<pg, kThreads, 0, s>>>(g, bf);
-    an_polish_gap<T><<<pg, kThreads, 0, s>>>(g, c, bf);
-    an_polish_write<T><<<pg, kThreads, 0, s>>>(g, bf);
-    nl += 5 + g.k;
-    // final rebuild, then retirement (over every image)
-    const unsigned BA = (unsigned)g.B;
-    an_final_skip<<<(BA + 127) / 128, 128, 0, s>>>(g, bf);
-    an_dual<T><<<pg, kThreads, 0, s>>>(g, bf, kStFinal);
-    an_gap<T><<<pg, kThreads, 0, s>>>(g, c, bf, kStFinal);
-    an_retire<<<(BA + 127) / 128, 128, 0, s>>>(g, bf);
-    nl += 4;
+    if (tail) {
+        // polish
+        an_dual<T><<<pg, kThreads, 0, s>>>(g, bf, kStPolish);
+        for (int a = 0; a < g.k; ++a) {
+            if (!(c.w[a] > 0.0 && g.L[a] > 1)) continue;
+            if (g.S[a] == 1) {
+                const int64_t bl = (nf[a] + kThreads / 32 - 1) / (kThreads / 32);
+                an_mark_rows<T><<<dim3((unsigned)std::min(bl, per), B), kThreads, 0, s>>>(g, c, bf, a);
+            } else {
+                const int64_t bl = (nf[a] + kMarkCols - 1) / kMarkCols;
+                an_mark_cols<T>
+                    <<<dim3((unsigned)std::min(bl, per), B), kMarkCols * kMarkParts, 0, s>>>(g, c, bf, a);
+            }
+            ++nl;
+        }
+        an_union<<<pg, kThreads, 0, s>>>(g, bf);
+        an_region_sum<T><<<pg, kThreads, 0, s>>>(g, bf);
+        an_polish_gap<T><<<pg, kThreads, 0, s>>>(g, c, bf);
+        an_polish_write<T><<<pg, kThreads, 0, s>>>(g, bf);
+        // final rebuild, then retirement (over every image)
+        const unsigned BA = (unsigned)g.B;
+        an_dual<T><<<pg, kThreads, 0, s>>>(g, bf, kStFinal);
+        an_gap<T><<<pg, kThreads, 0, s>>>(g, c, bf, kStFinal);
+        an_retire<<<(BA + 127) / 128, 128, 0, s>>>(g, bf);
+        nl += 8;
+    }
     if (launches) *launches += nl;
     return cudaGetLastError();
 }
@@ -1959,10 +2175,7 @@ bool aniso_pieces_enabled() {
     return on;
 }
 
-int an_pixel_blocks(const AnGeom &g) {
-    int64_t nb = (g.N + kThreads * 4 - 1) / (kThreads * 4);
-    return (int)std::max<int64_t>(1, std::min<int64_t>(nb, 256));
-}
+int an_pixel_blocks(const AnGeom &g) { return pixel_chunks(g.N); }
 
 cudaError_t aniso_setup(int dtype, const AnGeom &g, const AnCall &c, const AnBuffers &bf, const void *x,
                         cudaStream_t s) {
@@ -1978,9 +2191,10 @@ void aniso_prepare(int dtype) {
     else tile_attributes<double>();
 }
 
-cudaError_t aniso_round(int dtype, const AnGeom &g, const AnCall &c, const AnBuffers &bf, int64_t nimg,
+cudaError_t aniso_round(int dtype, const AnGeom &g, const AnCall &c, const AnBuffers &bf, int64_t nimg, bool tail,
                         cudaStream_t s, int64_t *launches) {
-    return dtype == 1 ? round_t<float>(g, c, bf, nimg, s, launches) : round_t<double>(g, c, bf, nimg, s, launches);
+    return dtype == 1 ? round_t<float>(g, c, bf, nimg, tail, s, launches)
+                      : round_t<double>(g, c, bf, nimg, tail, s, launches);
 }
 
 cudaError_t aniso_live_list(const AnState *st, int64_t B, int *lmap, int *lcnt, cudaStream_t s) {
