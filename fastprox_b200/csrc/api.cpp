@@ -1051,7 +1051,7 @@ fp_status run_iso(fp_workspace *ws, const fp_op *op, const void *xsrc, void *zds
         }
     }
     if (pairs || quads) {
-        e = iso_redo(ws->dtype, g, c, bf, s, quads);
+        e = iso_redo(ws->dtype, g, c, bf, s, quads, true);
         ws->kernel_launches += quads ? 3 : 2;
     }
     if (e == cudaSuccess) e = iso_finalize(ws->dtype, g, c, bf, zdst, s);

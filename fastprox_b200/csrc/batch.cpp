@@ -46,6 +46,7 @@ struct SlotHost {
     void *out = nullptr;  // the caller's z (device)
     int first_item = 0, n_items = 0, vec = 1;
     bool quad = false;  // the slot may take quad launches (its redo)
+    bool fresh = false; // admitted since the last chunk
 };
 
 template <class F>
@@ -76,24 +77,25 @@ struct fp_b200_batch {
     unsigned *ticket = nullptr;
     int *live = nullptr, *err = nullptr;
     RagSlot *slots = nullptr;
-    RagItem *items[3] = {nullptr, nullptr, nullptr};  // [0] vec 4 (or 2 for double), [1] vec 1, [2] quad tiles
-    int *n_items = nullptr;                           // 3 counts
+    // [0] vec 4 (or 2 for double), [1] vec 1, [2] quad tiles of rows of a multiple of 4 pixels, [3] of other rows
+    RagItem *items[4] = {nullptr, nullptr, nullptr, nullptr};
+    int *n_items = nullptr;  // 4 counts
     std::vector<void *> allocs, pinned;
     // host
     std::vector<Range> free_list;
     std::vector<SlotHost> sh;
     RagSlot *h_slots = nullptr;
-    RagItem *h_items[3] = {nullptr, nullptr, nullptr};
+    RagItem *h_items[4] = {nullptr, nullptr, nullptr, nullptr};
     int *h_n = nullptr;
     IsoState *h_st = nullptr;
     IsoImage *h_img = nullptr;
     int *h_live = nullptr;
     bool items_dirty = true;
-    int grid[3] = {0, 0, 0};
-    // graphs of `chunk` steps, keyed by (grid0, grid1, grid2, chunk)
-    std::map<std::tuple<int, int, int, int>, cudaGraphExec_t> graphs;
+    int grid[4] = {0, 0, 0, 0};
+    // graphs of `chunk` steps, keyed by the grids, the chunk and its mode
+    std::map<std::tuple<int, int, int, int, int, int>, cudaGraphExec_t> graphs;
     int rows_hint = 0;
-    bool quads = true;  // quad tiles for the float rows of a multiple of 4 pixels (admitted from now on)
+    bool quads = true;  // quad tiles for the float rows (admitted from now on)
     int quad_rows = 32;
     bool use_graphs = true;
     int64_t steps_run = 0, kernel_launches = 0;
@@ -235,7 +237,7 @@ IsoCall call_for(fp_b200_batch *bt, const SlotHost &s, double tol, int max_iter)
 
 // the work lists from the slots in use
 void rebuild_items(fp_b200_batch *bt) {
-    int n[3] = {0, 0, 0};
+    int n[4] = {0, 0, 0, 0};
     const int vfull = bt->dtype == FP_F32 ? 4 : 2;
     for (size_t i = 0; i < bt->sh.size(); ++i) {
         SlotHost &s = bt->sh[i];
@@ -251,10 +253,11 @@ void rebuild_items(fp_b200_batch *bt) {
             }
         if (rs.nquad > 0) {  // quad tiles: qrows rows x iso_quad_warps() strips
             const int ns = iso_quad_strips(s.W), qw = iso_quad_warps();
+            const int list = s.W % 4 == 0 ? 2 : 3;
             int qb = 0;
             for (int r0 = 0; r0 < s.H; r0 += rs.qrows)
                 for (int st0 = 0; st0 < ns; st0 += qw) {
-                    if (n[2] < bt->max_items) bt->h_items[2][n[2]++] = RagItem{(int)i, qb, r0, st0};
+                    if (n[list] < bt->max_items) bt->h_items[list][n[list]++] = RagItem{(int)i, qb, r0, st0};
                     ++qb;
                 }
         }
@@ -262,7 +265,8 @@ void rebuild_items(fp_b200_batch *bt) {
     bt->h_n[0] = n[0];
     bt->h_n[1] = n[1];
     bt->h_n[2] = n[2];
-    for (int l = 0; l < 3; ++l) {
+    bt->h_n[3] = n[3];
+    for (int l = 0; l < 4; ++l) {
         // a size class (a power of two) keeps captured graphs valid while the lists change within it
         int gcls = 0;
         if (n[l] > 0) {
@@ -273,35 +277,65 @@ void rebuild_items(fp_b200_batch *bt) {
         if (n[l]) cudaMemcpyAsync(bt->items[l], bt->h_items[l], (size_t)n[l] * sizeof(RagItem), cudaMemcpyHostToDevice,
                                   bt->stream);
     }
-    cudaMemcpyAsync(bt->n_items, bt->h_n, 3 * sizeof(int), cudaMemcpyHostToDevice, bt->stream);
+    cudaMemcpyAsync(bt->n_items, bt->h_n, 4 * sizeof(int), cudaMemcpyHostToDevice, bt->stream);
     bt->items_dirty = false;
 }
 
-cudaError_t launch_steps(fp_b200_batch *bt, int steps) {
+// What a chunk of steps launches beside the quads: a steady image (quad tiles,
+// past its first iteration, max_iter further than the chunk reaches) takes its
+// quad every step and leaves the single-step and pair launches alone, so they
+// are left out where every live image is steady (kQuadsOnly), and run in the
+// first step only where the others have just been admitted (kStart: their first
+// iteration, then quads). Three launches that exit at once cost 6 us a step
+// beside a quad launch of 30.
+enum ChunkMode : int { kAll = 0, kStart = 1, kQuadsOnly = 2 };
+
+ChunkMode chunk_mode(const fp_b200_batch *bt, int steps) {
+    ChunkMode m = kQuadsOnly;
+    for (size_t i = 0; i < bt->sh.size(); ++i) {
+        const SlotHost &s = bt->sh[i];
+        if (!s.used) continue;
+        const int max_iter = bt->h_slots[i].max_iter;
+        // the state as last polled; an image admitted since has it = 0
+        const int64_t it = s.fresh ? 0 : bt->h_st[i].it;
+        if (!s.fresh && bt->h_st[i].status != kLive) continue;
+        if (!s.quad || it + 4 * (int64_t)(steps + 1) >= max_iter || (it != 0 && (it & 3) != 1)) return kAll;
+        if (it == 0) m = kStart;
+    }
+    return m;
+}
+
+cudaError_t launch_steps(fp_b200_batch *bt, int steps, ChunkMode mode) {
     const IsoBuffers bf = buffers(bt);
     IsoCall c{};
     c.has_alpha = 0;
     const int vfull = bt->dtype == FP_F32 ? 4 : 2;
     for (int k = 0; k < steps; ++k) {
-        cudaError_t e = iso_ragged_step(bt->dtype, vfull, bt->items[0], bt->n_items, bt->grid[0], bt->slots, c, bf,
-                                        bt->stream);
-        if (e == cudaSuccess)
-            e = iso_ragged_step(bt->dtype, 1, bt->items[1], bt->n_items + 1, bt->grid[1], bt->slots, c, bf, bt->stream);
-        if (e == cudaSuccess)
-            e = iso_ragged_quad_step(bt->items[2], bt->n_items + 2, bt->grid[2], bt->slots, bf, bt->stream);
+        cudaError_t e = cudaSuccess;
+        if (mode == kAll || (mode == kStart && k == 0)) {
+            e = iso_ragged_step(bt->dtype, vfull, bt->items[0], bt->n_items, bt->grid[0], bt->slots, c, bf, bt->stream);
+            if (e == cudaSuccess)
+                e = iso_ragged_step(bt->dtype, 1, bt->items[1], bt->n_items + 1, bt->grid[1], bt->slots, c, bf,
+                                    bt->stream);
+        }
+        for (int l = 2; l < 4; ++l)
+            if (e == cudaSuccess)
+                e = iso_ragged_quad_step(l == 3, bt->items[l], bt->n_items + l, bt->grid[l], bt->slots, bf, bt->stream);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
-// kernels one step launches: the single steps on each non-empty list, the
-// two pair variants on the 4-wide float list
-int launches_per_step(const fp_b200_batch *bt) {
-    int n = 0;
-    if (bt->grid[0] > 0) n += 1 + (iso_ragged_pairs(bt->dtype, 4) ? 2 : 0);
-    if (bt->grid[1] > 0) n += 1;
-    if (bt->grid[2] > 0) n += 1;
-    return n;
+// kernels a chunk launches: the quads on each non-empty list, and where the mode
+// asks for them the single steps and, on the 4-wide float list, the two pair
+// variants
+int64_t chunk_launches(const fp_b200_batch *bt, int steps, ChunkMode mode) {
+    int all = 0, quads = 0;
+    if (bt->grid[0] > 0) all += 1 + (iso_ragged_pairs(bt->dtype, 4) ? 2 : 0);
+    if (bt->grid[1] > 0) all += 1;
+    if (bt->grid[2] > 0) quads += 1;
+    if (bt->grid[3] > 0) quads += 1;
+    return (int64_t)steps * quads + (mode == kAll ? (int64_t)steps * all : mode == kStart ? all : 0);
 }
 
 void trace(const char *what, cudaError_t e) {
@@ -310,8 +344,10 @@ void trace(const char *what, cudaError_t e) {
 }
 
 cudaError_t run_chunk(fp_b200_batch *bt, int steps) {
-    if (!bt->use_graphs) return launch_steps(bt, steps);
-    const auto key = std::make_tuple(bt->grid[0], bt->grid[1], bt->grid[2], steps);
+    const ChunkMode mode = chunk_mode(bt, steps);
+    bt->kernel_launches += chunk_launches(bt, steps, mode);
+    if (!bt->use_graphs) return launch_steps(bt, steps, mode);
+    const auto key = std::make_tuple(bt->grid[0], bt->grid[1], bt->grid[2], bt->grid[3], steps, (int)mode);
     auto it = bt->graphs.find(key);
     if (it == bt->graphs.end()) {
         cudaGraph_t graph = nullptr;
@@ -321,7 +357,7 @@ cudaError_t run_chunk(fp_b200_batch *bt, int steps) {
         bt->stream = cap;
         cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            e = launch_steps(bt, steps);
+            e = launch_steps(bt, steps, mode);
             cudaError_t e2 = cudaStreamEndCapture(cap, &graph);
             if (e == cudaSuccess) e = e2;
         }
@@ -334,7 +370,7 @@ cudaError_t run_chunk(fp_b200_batch *bt, int steps) {
             cudaGetLastError();
             if (graph) cudaGraphDestroy(graph);
             bt->use_graphs = false;
-            return launch_steps(bt, steps);
+            return launch_steps(bt, steps, mode);
         }
         cudaGraphExec_t exec = nullptr;
         e = cudaGraphInstantiate(&exec, graph, 0);
@@ -343,7 +379,7 @@ cudaError_t run_chunk(fp_b200_batch *bt, int steps) {
             trace("graph instantiate", e);
             cudaGetLastError();
             bt->use_graphs = false;
-            return launch_steps(bt, steps);
+            return launch_steps(bt, steps, mode);
         }
         it = bt->graphs.emplace(key, exec).first;
     }
@@ -400,11 +436,13 @@ FP_API fp_status fp_b200_batch_create(const fp_op *op, int64_t max_images, int64
         A((void **)&bt->items[0], (size_t)bt->max_items * sizeof(RagItem));
         A((void **)&bt->items[1], (size_t)bt->max_items * sizeof(RagItem));
         A((void **)&bt->items[2], (size_t)bt->max_items * sizeof(RagItem));
+        A((void **)&bt->items[3], (size_t)bt->max_items * sizeof(RagItem));
         A((void **)&bt->n_items, 16);
         Hh((void **)&bt->h_slots, S * sizeof(RagSlot));
         Hh((void **)&bt->h_items[0], (size_t)bt->max_items * sizeof(RagItem));
         Hh((void **)&bt->h_items[1], (size_t)bt->max_items * sizeof(RagItem));
         Hh((void **)&bt->h_items[2], (size_t)bt->max_items * sizeof(RagItem));
+        Hh((void **)&bt->h_items[3], (size_t)bt->max_items * sizeof(RagItem));
         Hh((void **)&bt->h_n, 16);
         Hh((void **)&bt->h_st, S * sizeof(IsoState));
         Hh((void **)&bt->h_img, S * sizeof(IsoImage));
@@ -513,10 +551,10 @@ FP_API fp_status fp_b200_batch_admit(fp_b200_batch *bt, const void *x, int64_t h
         }
         rs.max_iter = max_iter;
         rs.vec = s.vec;
-        // quad tiles: float rows of a multiple of 4 pixels, two rows or more
+        // quad tiles: float rows of a multiple of 4 pixels or of 32 or more, two rows or more
         rs.qrows = bt->quad_rows;
         rs.nquad = 0;
-        if (bt->quads && iso_ragged_pairs(bt->dtype, s.vec) && width % 4 == 0 && height >= 2) {
+        if (bt->quads && iso_ragged_pairs(bt->dtype, 4) && (width % 4 == 0 || width >= 32) && height >= 2) {
             const int64_t nq = ((height + rs.qrows - 1) / rs.qrows) *
                                ((iso_quad_strips((int)width) + iso_quad_warps() - 1) / iso_quad_warps());
             if (nq <= bt->max_part) rs.nquad = (int)nq;
@@ -547,6 +585,7 @@ FP_API fp_status fp_b200_batch_admit(fp_b200_batch *bt, const void *x, int64_t h
             return e == cudaErrorMemoryAllocation ? FP_ENOMEM : FP_EDEVICE;
         }
         bt->kernel_launches += 4;
+        s.fresh = true;
         bt->items_dirty = true;
         *slot_out = slot;
         return FP_OK;
@@ -576,12 +615,12 @@ FP_API fp_status fp_b200_batch_run(fp_b200_batch *bt, int steps, int max_chunks,
             trace("run", e);
             if (e != cudaSuccess) return FP_EDEVICE;
             bt->steps_run += steps;
-            bt->kernel_launches += (int64_t)steps * launches_per_step(bt);
             e = cudaMemcpyAsync(bt->h_st, bt->st, S * sizeof(IsoState), cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess) e = cudaMemcpyAsync(bt->h_live, bt->live, sizeof(int), cudaMemcpyDeviceToHost, st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
             trace("poll", e);
             if (e != cudaSuccess) return FP_EDEVICE;
+            for (size_t i = 0; i < S; ++i) bt->sh[i].fresh = false;
             for (size_t i = 0; i < S; ++i)
                 if (bt->sh[i].used && bt->h_st[i].status != kLive) done.push_back((int)i);
             if (!done.empty() || *bt->h_live == 0) break;

@@ -52,7 +52,7 @@ __device__ __forceinline__ double sqrt_t(double v) { return sqrt(v); }
 template <class T>
 __global__ void __launch_bounds__(kScanThreads) scan1_kernel(const T *__restrict__ x, T *__restrict__ d, Geometry g,
                                                              IsoCall c, IsoBuffers bf) {
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     __shared__ int flag;
     const int b = blockIdx.y;
     const int64_t N = g.N;
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kScanThreads) scan1_kernel(const T *__restrict
 // Pass 2: d *= 2^-e, sum d and sum d^2 (mean and the stopping target).
 template <class T>
 __global__ void __launch_bounds__(kScanThreads) scan2_kernel(T *__restrict__ d, Geometry g, IsoCall c, IsoBuffers bf) {
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     __shared__ int flag;
     const int b = blockIdx.y;
     const int mode = bf.img[b].mode;
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kScanThreads) scan2_kernel(T *__restrict__ d, 
 template <class T>
 __global__ void __launch_bounds__(kScanThreads) scan3_kernel(const T *__restrict__ d, Geometry g, IsoCall c,
                                                              IsoBuffers bf, int warm) {
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     __shared__ int flag;
     const int b = blockIdx.y;
     if (bf.img[b].mode != kModeFdpg) return;
@@ -586,7 +586,7 @@ __device__ __forceinline__ void lean_rows(const T *__restrict__ D, const T *__re
 // a single call never has) is flagged as an error rather than solved wrongly.
 template <class T, int VEC, bool ALPHA, bool GAP, bool ZIN>
 __global__ void __launch_bounds__(128, 5) iso2d_lean_kernel(StepArgs A, IsoCall c, IsoBuffers bf) {
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     __shared__ int flag;
     // launched as a programmatic dependent of the previous step: nothing of
     // its output (states, iterates, live list) is read before it completes
@@ -653,8 +653,10 @@ __global__ void __launch_bounds__(128, 5) iso2d_lean_kernel(StepArgs A, IsoCall 
         }
     }
     if (!arrive_last(bf.ticket + b, nblk, &flag)) return;
-    const double gap = GAP ? sum_partials(part, nslot, 2, 0, sh) : 0.0;
-    const double dot = test ? sum_partials(part, nslot, 2, 1, sh) : 0.0;
+    double gap = 0.0, dot = 0.0;
+    if (GAP || test) sum_pairs(part, nslot, sh, gap, dot);
+    if (!GAP) gap = 0.0;
+    if (!test) dot = 0.0;
     if (threadIdx.x != 0) return;
     bf.ticket[b] = 0;
     IsoState s2 = st;
@@ -1162,7 +1164,7 @@ __device__ __forceinline__ void pair_pass(const PairTile<T> &p, double *rowp, do
 template <class T, bool ALPHA, bool GAP2, bool WIDE>
 __global__ void __launch_bounds__(128, GAP2 ? 3 : 4) iso2d_pair_kernel(StepArgs A, IsoCall c, IsoBuffers bf) {
     __shared__ double rowp[GAP2 ? kLeanRowsMax * 8 : 1];
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     __shared__ int flag;
     asm volatile("griddepcontrol.wait;" ::: "memory");  // a programmatic dependent of the previous step
     const int b = step_image(bf, blockIdx.z);
@@ -1220,8 +1222,8 @@ __global__ void __launch_bounds__(128, GAP2 ? 3 : 4) iso2d_pair_kernel(StepArgs 
     }
     if (!arrive_last(bf.ticket + b, gridDim.x * gridDim.y, &flag)) return;
     const int nslot = H * (int)gridDim.x;
-    const double gap = GAP2 ? sum_partials(part, nslot, 2, 0, sh) : 0.0;
-    const double dot = GAP2 ? sum_partials(part, nslot, 2, 1, sh) : 0.0;
+    double gap = 0.0, dot = 0.0;
+    if (GAP2) sum_pairs(part, nslot, sh, gap, dot);
     if (threadIdx.x != 0) return;
     bf.ticket[b] = 0;
     IsoState s2 = st;
@@ -1325,13 +1327,21 @@ __global__ void iso2d_redo_state(IsoState *st, int64_t B) {
 // depend on: r0 - (4 - l) .. r1 + (4 - l).
 // The per-pixel arithmetic is the lean step's (the same expressions), so the
 // iterates are those of four single steps while the restart decisions agree;
-// the gap and restart-test sums are formed per row and strip (a lane's two
-// columns, then the warp's tree) into H x strips slots, summed in order by the
-// image's last block: a fixed order of its own (an image gives the same bits
-// alone and in any batch).
+// the gap and restart-test sums are formed per four rows and strip (a lane's
+// columns, then the warp's tree) into slots, summed in order by the image's last
+// block: a fixed order of its own (an image gives the same bits alone and in
+// any batch). The gap that is reported is formed once more by the redo variant,
+// row by row.
 // Traffic per pixel and four iterations: d, u, v, alpha read once (rows of a
 // block's halo again, from L2 mostly), u, v written once: about 40 B against
 // 4 x 40 B for four single steps.
+// What bounds it: with 16 warps per SM (128 registers) a step of a warp is 300
+// instructions over four dependent levels; 58 % of the issue slots, 27 % of the
+// DRAM sectors. 436 instructions a step (84 of them register moves, 78 integer
+// address work, 27 shuffles) took 227 us a launch on 64 x 512^2; pairs held in
+// 64-bit registers, four steps unrolled with fixed ring slots, the sums of four
+// rows at a time, momenta in shared memory and a square root without branches
+// made it 170 us (64 x 512^2 with pixel weights 48.8 -> 35.1 ms a solve).
 // ---------------------------------------------------------------------------
 constexpr int kQuadWin = 64;                        // window columns of a warp: two per lane
 constexpr int kQuadHalo = 4;                        // one column per iteration on each side
@@ -1343,15 +1353,16 @@ constexpr int kQuadSlotsD = 8;                      // ring rows of d and the ra
 constexpr int kQuadRingFloats = kQuadSlotsUV * 4 * kQuadWin + kQuadSlotsD * 2 * kQuadWin;
 constexpr size_t kQuadSmem = (size_t)kQuadWarps * kQuadRingFloats * sizeof(float);
 
-// Strips of a row of W columns: one window when W <= 64 (its edges are the
-// image's, so it needs no halo); else a first window at column 0 writing
-// columns 0 .. 59 (no halo on the image's edge), windows at 56 k writing
+// Strips of a row of W columns, W rounded up to a multiple of 4 (a window
+// starts on 16 bytes; columns past W are zero): one window when W <= 64 (its
+// edges are the image's, so it needs no halo); else a first window at column 0
+// writing columns 0 .. 59 (no halo on the image's edge), windows at 56 k writing
 // 56 k + 4 .. 56 k + 59, and a last window ending at column W writing the rest
 // (9 strips for a row of 512, against 10 with a halo on every side).
 __host__ __device__ constexpr int quad_strips(int W) {
     return W <= kQuadWin ? 1
                          : 2 + ((W - 2 * (kQuadWin - kQuadHalo) > 0)
-                                    ? (W - 2 * (kQuadWin - kQuadHalo) + kQuadOut - 1) / kQuadOut
+                                    ? ((W + 3) / 4 * 4 - 2 * (kQuadWin - kQuadHalo) + kQuadOut - 1) / kQuadOut
                                     : 0);
 }
 // Strip k's window (first column, a multiple of 4) and the columns it writes.
@@ -1364,14 +1375,20 @@ __host__ __device__ inline void quad_strip_cols(int W, int k, int &c0, int &lo, 
     } else if (k < n - 1) {
         c0 = k * kQuadOut, lo = c0 + kQuadHalo, hi = c0 + kQuadWin - kQuadHalo;
     } else {
-        c0 = W - kQuadWin, lo = (n - 2) * kQuadOut + kQuadWin - kQuadHalo, hi = W;
+        c0 = (W + 3) / 4 * 4 - kQuadWin, lo = (n - 2) * kQuadOut + kQuadWin - kQuadHalo, hi = W;
     }
 }
 
-__device__ __forceinline__ void cp_async16_zfill(void *dst, const void *src, unsigned n) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-                 "l"(src), "r"(n)
-                 : "memory");
+// Copies of N bytes (16, 8 or 4, aligned to N on both sides), n of them from
+// memory (N or 0) and the rest zero.
+template <int N>
+__device__ __forceinline__ void cp_async_zfill(uint32_t dst, const void *src, unsigned n) {
+    if constexpr (N == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+    else if constexpr (N == 8)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 
 // What one quad pass needs: an image's arrays (v = u when vsel), its
@@ -1399,35 +1416,46 @@ __device__ __forceinline__ void quad_betas(double tn, double beta0, float (&beta
     }
 }
 
-// Packed float pairs (a lane's two columns): sm_100's f32x2 arithmetic, each
-// half one IEEE float32 operation rounded to nearest (the same result as the
-// scalar operation; nothing is fused that the scalar steps do not fuse).
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) {  // a - b
-    float2 d;
-    asm("{.reg .b64 a, b, d;\n\t"
-        "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
-        "sub.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+// Packed float pairs (a lane's two columns) in 64-bit registers: sm_100's f32x2
+// arithmetic, each half one IEEE float32 operation rounded to nearest (the same
+// result as the scalar operation; nothing is fused that the scalar steps do not
+// fuse). Held as 64-bit values throughout: pairs packed from float2 around
+// every operation cost 84 register moves of 436 instructions per step.
+typedef unsigned long long F2;
+__device__ __forceinline__ F2 pk(float x, float y) {
+    F2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
     return d;
 }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {  // a b
-    float2 d;
-    asm("{.reg .b64 a, b, d;\n\t"
-        "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
-        "mul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+__device__ __forceinline__ float lo(F2 a) { return __uint_as_float((unsigned)a); }
+__device__ __forceinline__ float hi(F2 a) { return __uint_as_float((unsigned)(a >> 32)); }
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) {  // a - b
+    F2 d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {  // a b + c, one rounding
-    float2 d;
-    asm("{.reg .b64 a, b, c, d;\n\t"
-        "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
-        "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {  // a b
+    F2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {  // a b + c, one rounding
+    F2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+// sqrt of both halves (>= 0): s = x y from the hardware's reciprocal root y,
+// then one Newton step on s with its residual x - s^2 formed exactly by a fused
+// operation (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000", 1990): the error before the last rounding is about 2^-44 of s,
+// below sqrtf's half unit in all but about one case in 10^6. Without the
+// library call's branches (two per row and lane).
+__device__ __forceinline__ F2 sqrt2(F2 x) {
+    const F2 y = pk(rsqrt_t(lo(x)), rsqrt_t(hi(x)));
+    const F2 s = mul2(x, y);
+    const F2 e = pk(fmaf(-lo(s), lo(s), lo(x)), fmaf(-hi(s), hi(s), hi(x)));
+    return fma2(mul2(e, pk(0.5f, 0.5f)), y, s);
 }
 
 // One warp's march over a strip, rows [r0, r1) out. The pass's state: per
@@ -1436,17 +1464,30 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {  // a b +
 // is a lane's two columns.
 template <int LV>
 struct QuadCarry {
-    float2 cv0[LV], cv1[LV], cu0[LV], cu1[LV], cz[LV];
-    float2 czu;
+    F2 cv0[LV], cv1[LV], cu0[LV], cu1[LV], cz[LV];
+    F2 czu;
+    double gacc, dacc;  // the lane's gap and restart-test sums
+};
+// What a lane's two columns are, fixed over the march.
+struct QuadLane {
+    bool outx, outy;  // written columns
+    bool ledge;       // the first is the image's first: its left neighbour is the zero padding
+    F2 wr;            // the weights of their right differences (0 past the last column)
+    F2 rad;           // their radii without pixel weights (0 outside the image)
 };
 
-// One step s of the march: stage row s, then iteration l + 1 (l = 0 ..
-// LV - 1) updates row s - l - 1 from its input rows s - l - 1 (carried) and
-// s - l (the staged row for l = 0, else iteration l's output of this step).
-// OUT: the last level's row is an output row of the tile (stores, and the
-// check's sums); before that (the first 2 LV steps) the levels run on the rows
-// above the tile with the same arithmetic and nothing leaves the warp. Rows
-// outside the image have d = v = u = 0 and radius 0, so their updates give
+// One step of the march, row s: iteration l + 1 (l = 0 .. LV - 1) updates row
+// s - l - 1 from its input rows s - l - 1 (carried) and s - l (the staged row for
+// l = 0, else iteration l's output of this step).
+// The march is unrolled four steps deep: I is the step's place in its group, so
+// that the ring's slots are fixed offsets (uv's slot is I; d's rows lie in
+// halves of four slots, rdc this group's and rdo the last one's) and the carried
+// rows stay in the registers they were formed in. G >= 0: group G of the rows
+// above the tile (8 steps), where the levels whose rows do not feed an output
+// row's halo yet only keep their z and carried rows; G < 0: an output row (the
+// last level's row is stored, with its sums). EDGE: rows past the image may
+// occur (no vertical difference on its last row).
+// Rows outside the image have d = v = u = 0 and radius 0, so their updates give
 // u = v = 0 (the zero padding of the divergence) without a branch; a lane's
 // columns outside the image likewise. The left neighbour of a lane's first
 // column and the right one of its second come by shuffle; lane 0 and lane 31
@@ -1455,101 +1496,93 @@ struct QuadCarry {
 // The arithmetic per pixel is the single step's (iso2d_lean_kernel), operation
 // for operation, with each multiply-add the single step's compiler fuses
 // written as one fused operation here.
-template <bool ALPHA, bool REDO, bool ROWSUMS, bool OUT, int LV>
-__device__ __forceinline__ void quad_step(const QuadTile &p, QuadCarry<LV> &q, int s, int ustart, int strip,
-                                          float *ruv, float *rd, int wc, bool outcol, bool ledge, float wh1r1,
-                                          double &gsum, double &dsum, float *uo, float *vo) {
-    const int H = p.H, W = p.W;
-    const float2 W0 = make_float2(p.wh0, p.wh0), W1 = make_float2(p.wh1, p.wh1), WR = make_float2(p.wh1, wh1r1);
-    const float2 TAU = make_float2(p.tau, p.tau);
-    auto ld2 = [](const float *a) { return *reinterpret_cast<const float2 *>(a); };
-    const float *rs = ruv + (s & (kQuadSlotsUV - 1)) * 4 * kQuadWin + wc;
-    float2 nv0 = ld2(rs + 0 * kQuadWin), nv1 = ld2(rs + 1 * kQuadWin);
-    float2 nu0 = ld2(rs + 2 * kQuadWin), nu1 = ld2(rs + 3 * kQuadWin);
+template <int PC, bool REDO, int G, bool EDGE, int LV, int I>
+__device__ __forceinline__ void quad_step(const QuadTile &p, const QuadLane &ln, QuadCarry<LV> &q, int s,
+                                          const float *ruv, const float *rdc, const float *rdo, const F2 *qb,
+                                          float *uo, float *vo, unsigned oo) {
+    constexpr bool OUT = G < 0;
+    const F2 W0 = pk(p.wh0, p.wh0), W1 = pk(p.wh1, p.wh1), TAU = pk(p.tau, p.tau);
+    auto ld2 = [](const float *a) { return *reinterpret_cast<const F2 *>(a); };
+    const float *rs = ruv + I * 4 * kQuadWin;
+    F2 nv0 = ld2(rs), nv1 = ld2(rs + kQuadWin), nu0 = ld2(rs + 2 * kQuadWin), nu1 = ld2(rs + 3 * kQuadWin);
+    // z of a row pair: d + wh0 (a - above) + wh1 (b - b left)
+    auto zrow = [&](F2 d, F2 a, F2 above, F2 bb) {
+        const float sl = __shfl_up_sync(0xffffffffu, hi(bb), 1);
+        const float left = ln.ledge ? 0.f : sl;
+        // REDO: the difference in scalar operations. The row above the tile's first is
+        // used nowhere else there, and the assembler would fuse the product that
+        // forms it into a packed difference (one rounding less, another gap)
+        const F2 up = REDO ? pk(__fsub_rn(lo(a), lo(above)), __fsub_rn(hi(a), hi(above))) : sub2(a, above);
+        return fma2(W1, pk(lo(bb) - left, hi(bb) - lo(bb)), fma2(W0, up, d));
+    };
 #pragma unroll
     for (int l = 0; l < LV; ++l) {
-        const int rn = s - l, r = rn - 1;  // this level's new input row; the row it updates
-        const float2 dn = ld2(rd + (rn & (kQuadSlotsD - 1)) * 2 * kQuadWin + wc);
-        const float sl = __shfl_up_sync(0xffffffffu, nv1.y, 1);
-        const float left = ledge ? 0.f : sl;
-        // z = d + wh0 (v0 - v0 above) + wh1 (v1 - v1 left)
-        const float2 nz = fma2(W1, sub2(nv1, make_float2(left, nv1.x)), fma2(W0, sub2(nv0, q.cv0[l]), dn));
+        // this level's new input row s - l; the row it updates is the one above
+        const F2 dn = ld2((I - l >= 0 ? rdc + (I - l) * 2 * kQuadWin : rdo + (4 + I - l) * 2 * kQuadWin));
+        const F2 nz = zrow(dn, nv0, q.cv0[l], nv1);
         const bool last = l == LV - 1;
-        const bool check = !REDO && last;
-        float2 nzu = make_float2(0.f, 0.f);
-        if (check) {  // z of the third iterate's u on row rn
-            const float slu = __shfl_up_sync(0xffffffffu, nu1.y, 1);
-            const float lu = ledge ? 0.f : slu;
-            nzu = fma2(W1, sub2(nu1, make_float2(lu, nu1.x)), fma2(W0, sub2(nu0, q.cu0[l]), dn));
-        }
-        const float wh0n = rn < H ? p.wh0 : 0.f;  // no vertical difference on the image's last row
-        const float2 W0N = make_float2(wh0n, wh0n);
-        const float zr = __shfl_down_sync(0xffffffffu, q.cz[l].x, 1);
-        const float2 rp = ld2(rd + ((r & (kQuadSlotsD - 1)) * 2 + 1) * kQuadWin + wc);
-        float2 un0, un1, ov0, ov1;
-        // above the tile, level l's updates are first needed at step ustart + 2 l
-        // (their rows feed the output rows' halo); before it only its z and
-        // carried rows are kept, and its output is not read
-        if (OUT || s >= ustart + 2 * l) {
-            const float2 g0 = mul2(W0N, sub2(nz, q.cz[l]));
-            const float2 g1 = mul2(WR, sub2(make_float2(q.cz[l].y, zr), q.cz[l]));
-            const float2 a0 = fma2(TAU, g0, q.cv0[l]);
-            const float2 a1 = fma2(TAU, g1, q.cv1[l]);
-            const float2 nn = fma2(a0, a0, mul2(a1, a1));
-            const float2 rr = mul2(rp, rp);
-            const float2 pr = mul2(rp, make_float2(rsqrt_t(nn.x), rsqrt_t(nn.y)));
-            const float2 sc = make_float2(nn.x > rr.x ? pr.x : 1.f, nn.y > rr.y ? pr.y : 1.f);
-            un0 = mul2(a0, sc);
-            un1 = mul2(a1, sc);
-            const float2 B = make_float2(p.beta[l], p.beta[l]);
-            ov0 = fma2(B, sub2(un0, q.cu0[l]), un0);
-            ov1 = fma2(B, sub2(un1, q.cu1[l]), un1);
-        } else {
-            un0 = un1 = ov0 = ov1 = make_float2(0.f, 0.f);
-        }
-        if (OUT && last) {
-            if (check) {
+        F2 nzu = 0;
+        if (last) nzu = zrow(dn, nu0, q.cu0[l], nu1);  // z of the third iterate's u
+        F2 un0 = 0, un1 = 0, ov0 = 0, ov1 = 0;
+        // above the tile, level l's updates are first needed at step 2 + 2 l
+        if (OUT || 4 * G + I >= 2 + 2 * l) {
+            const F2 rp = ld2((I - l >= 1 ? rdc + (I - l - 1) * 2 * kQuadWin : rdo + (3 + I - l) * 2 * kQuadWin) +
+                              kQuadWin);
+            F2 W0N = W0;
+            if (EDGE) {
+                const float wh0n = s - l < p.H ? p.wh0 : 0.f;
+                W0N = pk(wh0n, wh0n);
+            }
+            if (!(REDO && last)) {
+                const float zr = __shfl_down_sync(0xffffffffu, lo(q.cz[l]), 1);
+                const F2 g0 = mul2(W0N, sub2(nz, q.cz[l]));
+                const F2 g1 = mul2(ln.wr, pk(hi(q.cz[l]) - lo(q.cz[l]), zr - hi(q.cz[l])));
+                const F2 a0 = fma2(TAU, g0, q.cv0[l]);
+                const F2 a1 = fma2(TAU, g1, q.cv1[l]);
+                const F2 nn = fma2(a0, a0, mul2(a1, a1));
+                const F2 rr = mul2(rp, rp);
+                const F2 pr = mul2(rp, pk(rsqrt_t(lo(nn)), rsqrt_t(hi(nn))));
+                const F2 sc = pk(lo(nn) > lo(rr) ? lo(pr) : 1.f, hi(nn) > hi(rr) ? hi(pr) : 1.f);
+                un0 = mul2(a0, sc);
+                un1 = mul2(a1, sc);
+                const F2 B = qb[l];
+                ov0 = fma2(B, sub2(un0, q.cu0[l]), un0);
+                ov1 = fma2(B, sub2(un1, q.cu1[l]), un1);
+            }
+            if (OUT && last) {
                 // the restart test's dot (v - u_new)(u_new - u) and the gap at
                 // the third iterate u with z of it
-                const float2 dd = fma2(sub2(q.cv0[l], un0), sub2(un0, q.cu0[l]),
+                const float zur = __shfl_down_sync(0xffffffffu, lo(q.czu), 1);
+                const F2 gu0 = mul2(W0N, sub2(nzu, q.czu));
+                const F2 gu1 = mul2(ln.wr, pk(hi(q.czu) - lo(q.czu), zur - hi(q.czu)));
+                const F2 gg = fma2(gu0, gu0, mul2(gu1, gu1));
+                const F2 in = fma2(gu0, q.cu0[l], mul2(gu1, q.cu1[l]));
+                const F2 sg = sqrt2(gg);
+                const float t0 = fmaf(lo(rp), lo(sg), -lo(in)), t1 = fmaf(hi(rp), hi(sg), -hi(in));
+                const double gx = (double)(ln.outx ? t0 : 0.f), gy = (double)(ln.outy ? t1 : 0.f);
+                q.gacc += gx + gy;
+                if (!REDO) {
+                    const F2 dd = fma2(sub2(q.cv0[l], un0), sub2(un0, q.cu0[l]),
                                        mul2(sub2(q.cv1[l], un1), sub2(un1, q.cu1[l])));
-                const float zur = __shfl_down_sync(0xffffffffu, q.czu.x, 1);
-                const float2 gu0 = mul2(W0N, sub2(nzu, q.czu));
-                const float2 gu1 = mul2(WR, sub2(make_float2(q.czu.y, zur), q.czu));
-                const float2 gg = fma2(gu0, gu0, mul2(gu1, gu1));
-                const float2 in = fma2(gu0, q.cu0[l], mul2(gu1, q.cu1[l]));
-                const float t0 = fmaf(rp.x, sqrtf(gg.x), -in.x), t1 = fmaf(rp.y, sqrtf(gg.y), -in.y);
-                double gacc = 0.0, dacc = 0.0;
-                if (outcol) {
-                    dacc = (double)dd.x;
-                    gacc = (double)t0;
-                    dacc += (double)dd.y;
-                    gacc += (double)t1;
-                }
-                if (ROWSUMS) {
-                    // this row's sums over the strip (a fixed tree) into its slot
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) {
-                        gacc += __shfl_down_sync(0xffffffffu, gacc, o);
-                        dacc += __shfl_down_sync(0xffffffffu, dacc, o);
-                    }
-                    if ((threadIdx.x & 31) == 0) {
-                        double *part = p.rowpart + ((int64_t)r * quad_strips(W) + strip) * 2;
-                        part[0] = gacc;
-                        part[1] = dacc;
-                    }
-                } else {
-                    gsum += gacc;
-                    dsum += dacc;
+                    const double dx = (double)(ln.outx ? lo(dd) : 0.f), dy = (double)(ln.outy ? hi(dd) : 0.f);
+                    q.dacc += dx + dy;
                 }
             }
-            if (outcol) {  // the pass's output row
-                const int64_t o = (int64_t)r * W;
-                *reinterpret_cast<float2 *>(uo + o) = un0;
-                *reinterpret_cast<float2 *>(uo + p.N + o) = un1;
+            if (OUT && last && ln.outx) {  // the pass's output row
+                auto store = [&](float *o, F2 v) {
+                    if (PC == 1) {
+                        o[0] = lo(v);
+                        if (ln.outy) o[1] = hi(v);
+                    } else {
+                        *reinterpret_cast<F2 *>(o) = v;
+                    }
+                };
+                const unsigned o1 = oo + (unsigned)p.N;  // N < 2^31
+                store(uo + oo, REDO ? q.cu0[l] : un0);
+                store(uo + o1, REDO ? q.cu1[l] : un1);
                 if (!REDO) {
-                    *reinterpret_cast<float2 *>(vo + o) = ov0;
-                    *reinterpret_cast<float2 *>(vo + p.N + o) = ov1;
+                    store(vo + oo, ov0);
+                    store(vo + o1, ov1);
                 }
             }
         }
@@ -1560,7 +1593,7 @@ __device__ __forceinline__ void quad_step(const QuadTile &p, QuadCarry<LV> &q, i
         q.cu0[l] = nu0;
         q.cu1[l] = nu1;
         q.cz[l] = nz;
-        if (check) q.czu = nzu;
+        if (last) q.czu = nzu;
         nv0 = ov0;
         nv1 = ov1;
         nu0 = un0;
@@ -1568,92 +1601,196 @@ __device__ __forceinline__ void quad_step(const QuadTile &p, QuadCarry<LV> &q, i
     }
 }
 
-// The march of one warp over strip `strip`, output rows [r0, r1): steps
-// r0 - LV .. r1 + LV - 1, a row staged per step (three ahead), the first 2 LV
-// steps before any output row. REDO: three iterations, the third's u written.
-// ROWSUMS: each output row's gap and restart-test sums over the strip into
-// p.rowpart[row x strips + strip] (the batched launch); else they accumulate
-// per lane in gsum, dsum (the ragged step's per-tile slot).
-template <bool ALPHA, bool REDO, bool ROWSUMS>
+// The march of one warp over strip `strip`, output rows [r0, r1): 8 steps of
+// rows above the tile, then a step per output row; row s is staged at its step,
+// its copies three steps before.
+// REDO: the third iterate's u is written, and the fourth level only forms its gap.
+// ROWSUMS: the sums over the strip go to p.rowpart: the gap and restart-test sums
+// of each four output rows to slot rows / 4 x strips + strip (r0 a multiple of 4:
+// the same groups in every tiling), or, REDO, each row's gap to slot row x strips +
+// strip. Else they accumulate per lane in gsum, dsum (the ragged step's per-tile
+// slot). (Summing every row in the march: 40.6 against 34.9 ms on 64 x 512^2.)
+// PC: columns per copy, 4 (rows of a multiple of 4 columns), 2 or 1: rows of any
+// width start on PC floats (3, 6 and 12 copies a row and lane). Single steps on
+// rows that are not a multiple of 4 (one column per thread) took 10.7 ms on a
+// 1531 x 1021 image, the quads take 4.2.
+template <int PC, bool ALPHA, bool REDO, bool ROWSUMS>
 __device__ __forceinline__ void quad_pass(const QuadTile &p, int strip, int r0, int r1, double &gsum,
                                           double &dsum) {
-    constexpr int LV = REDO ? 3 : 4;  // iterations of the pass
+    constexpr int LV = 4;  // iterations of the pass
     extern __shared__ __align__(16) float quad_ring[];
     const int H = p.H, W = p.W;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float *ring = quad_ring + warp * kQuadRingFloats;
-    float *ruv = ring;                                  // [slot][v0, v1, u0, u1][64]
-    float *rd = ring + kQuadSlotsUV * 4 * kQuadWin;     // [slot][d, radius][64]
-    int C0, lo, hi;  // the window's first column (a multiple of 4); the columns it writes
-    quad_strip_cols(W, strip, C0, lo, hi);
+    float *ruv = ring;  // [uv slot][v0, v1, u0, u1][64], then [d slot][d, radius][64]
+    int C0, lo_, hi_;  // the window's first column (a multiple of 4); the columns it writes
+    quad_strip_cols(W, strip, C0, lo_, hi_);
+    const int nstrips = quad_strips(W);
     const int wc = 2 * lane;                            // this lane's first window column
     const int col = C0 + wc;
-    const bool colin = col < W;                         // both columns (W and col are even)
-    const bool outcol = col >= lo && col < hi;          // written columns (lo, hi multiples of 4)
-    const bool ledge = C0 == 0 && lane == 0;            // column 0: its left neighbour is the zero padding
-    const float wh1r1 = col + 2 < W ? p.wh1 : 0.f;      // the second column's right difference
-    const float radl = colin ? p.rad : 0.f;             // the radius of this lane's columns (no pixel weights)
-    // the copies: 16-byte pieces of the window's rows, a piece per lane and
-    // array; pieces outside the image are zero-filled (from a valid address)
-    const int ch = lane & 15, half = lane >> 4;
-    const int cc = C0 + 4 * ch;
-    const bool colok = cc >= 0 && cc < W;
-    const int ccs = colok ? cc : 0;
-    const float *src_v = (half ? p.V0 + p.N : p.V0) + ccs;
-    const float *src_u = (half ? p.U0 + p.N : p.U0) + ccs;
-    const float *src_d = (half ? p.AL : p.D) + ccs;
-    float *dst_v = ruv + half * kQuadWin + 4 * ch;
-    float *dst_u = ruv + (2 + half) * kQuadWin + 4 * ch;
-    float *dst_d = rd + half * kQuadWin + 4 * ch;
-    const bool copy_d = ALPHA || half == 0;
-    auto issue = [&](int row, int se) {
-        if (row <= se) {
-            const bool rowin = (unsigned)row < (unsigned)H;
-            const int64_t ro = (int64_t)(rowin ? row : 0) * W;
-            const unsigned n = rowin && colok ? 16u : 0u;
-            cp_async16_zfill(dst_v + (row & (kQuadSlotsUV - 1)) * 4 * kQuadWin, src_v + ro, n);
-            cp_async16_zfill(dst_u + (row & (kQuadSlotsUV - 1)) * 4 * kQuadWin, src_u + ro, n);
-            if (copy_d) cp_async16_zfill(dst_d + (row & (kQuadSlotsD - 1)) * 2 * kQuadWin, src_d + ro, n);
+    const bool inx = col < W, iny = col + 1 < W;
+    QuadLane ln;
+    ln.outx = col >= lo_ && col < hi_;                  // lo_ is even; hi_ too, but for the last column of an odd W
+    ln.outy = ln.outx && col + 1 < hi_;
+    ln.ledge = C0 == 0 && lane == 0;
+    ln.wr = pk(iny ? p.wh1 : 0.f, col + 2 < W ? p.wh1 : 0.f);
+    ln.rad = pk(inx ? p.rad : 0.f, iny ? p.rad : 0.f);
+    // the copies of a row: pieces of PC columns of v and u (both components), d
+    // and alpha; pieces outside the image are zero-filled (from a valid address).
+    // PC = 4: a piece of one component per lane; 2: a piece of each per lane; 1:
+    // two columns of each per lane, 32 apart, so that a copy reads 32 columns
+    // side by side.
+    const int half = PC == 4 ? lane >> 4 : 0;
+    const int cl = PC == 4 ? 4 * (lane & 15) : (PC == 2 ? 2 * lane : lane);  // the window column this lane copies
+    const int cc = C0 + cl;
+    const bool okx = cc < W, oky = PC == 1 && cc + 32 < W;
+    const int ccx = okx ? cc : 0, sy = oky ? 32 : 0;
+    const uint32_t sm = (uint32_t)__cvta_generic_to_shared(ring) + (uint32_t)cl * 4u;
+    constexpr uint32_t kRow = kQuadWin * 4u, kD = kQuadSlotsUV * 4 * kRow;  // bytes of a ring row; of the uv ring
+    const unsigned rlast = (unsigned)min(r1 + LV - 1, H - 1);  // the last row copied
+    // offsets within an image's two planes fit 32 bits (N < 2^31)
+    const unsigned Nu = (unsigned)p.N, co = (unsigned)ccx + (PC == 4 && half ? Nu : 0u);
+    const float *sd = (PC == 4 && half ? p.AL : p.D) + ccx;
+    const uint32_t smv = sm + (PC == 4 ? half * kRow : 0u);
+    // row `row` into uv slot `slot` of the ring and the d slot at byte `ds`
+    auto issue = [&](int row, int slot, uint32_t ds) {
+        const bool rowin = (unsigned)row <= rlast;
+        const int ro = rowin ? row * W : 0;
+        const uint32_t du = smv + slot * 4 * kRow, dd = smv + kD + ds;
+        const unsigned o = (unsigned)ro + co;
+        if (PC == 4) {
+            const unsigned n = rowin && okx ? 16u : 0u;
+            cp_async_zfill<16>(du, p.V0 + o, n);
+            cp_async_zfill<16>(du + 2 * kRow, p.U0 + o, n);
+            if (ALPHA || half == 0) cp_async_zfill<16>(dd, sd + ro, n);
+        } else {
+            constexpr int NB = PC == 2 ? 8 : 4;
+            const unsigned nx = rowin && okx ? NB : 0u, ny = rowin && oky ? NB : 0u;
+            auto both = [&](uint32_t dst, const float *src) {
+                cp_async_zfill<NB>(dst, src, nx);
+                if (PC == 1) cp_async_zfill<NB>(dst + 128, src + sy, ny);
+            };
+            both(du, p.V0 + o);
+            both(du + kRow, p.V0 + (o + Nu));
+            both(du + 2 * kRow, p.U0 + o);
+            both(du + 3 * kRow, p.U0 + (o + Nu));
+            both(dd, sd + ro);
+            if (ALPHA) both(dd + kRow, p.AL + ccx + ro);
         }
         cp_async_commit();
     };
     QuadCarry<LV> q;
 #pragma unroll
-    for (int l = 0; l < LV; ++l) q.cv0[l] = q.cv1[l] = q.cu0[l] = q.cu1[l] = q.cz[l] = make_float2(0.f, 0.f);
-    q.czu = make_float2(0.f, 0.f);
-    float *uo = p.UO0 + (colin ? col : 0), *vo = p.VO0 + (colin ? col : 0);
-    const int sb = r0 - LV, se = r1 + LV - 1, ustart = r0 - LV + 2;
-    for (int k = 0; k < kQuadAhead; ++k) issue(sb + k, se);
-    // stage row s: wait for its copies, then the radius row in place (this
-    // lane's own entries): gamma alpha capped at the bound, 0 where alpha is 0
-    // or outside the image
-    auto stage = [&](int s) {
-        __syncwarp();  // every lane is past its reads of the slots refilled now
-        issue(s + kQuadAhead, se);
+    for (int l = 0; l < LV; ++l) q.cv0[l] = q.cv1[l] = q.cu0[l] = q.cu1[l] = q.cz[l] = 0;
+    q.czu = 0;
+    q.gacc = gsum;
+    q.dacc = dsum;
+    float *uo = p.UO0 + (inx ? col : 0), *vo = p.VO0 + (inx ? col : 0);
+    // the momenta as pairs in shared memory (broadcast reads, at a fixed address;
+    // the block's warps write the same): eight registers less
+    __shared__ F2 qb[5];
+    if (lane == 0) {
+        qb[4] = pk(p.rad, p.bnd);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) qb[l] = pk(p.beta[l], p.beta[l]);
+    }
+    __syncwarp();
+    const int sb = r0 - LV;
+    const int T = r1 - r0 + 8;
+    constexpr uint32_t kHalf = 4 * 2 * kRow;  // bytes of half the d ring
+    for (int k = 0; k < kQuadAhead; ++k) issue(sb + k, k, k * 2 * kRow);
+    // the halves of the d ring: this group's (hc) and the last one's, in bytes
+    uint32_t hc = 0;
+    const float *ruvl = ruv + wc;
+    // stage row s (step I of its group): wait for its copies, then the radius
+    // row in place (this lane's own entries): gamma alpha capped at the bound,
+    // 0 where alpha is 0 or outside the image
+    auto stage = [&](int s, int I) {
+        if (PC != 2) __syncwarp();  // every lane is past its reads of the slots refilled now
+        issue(s + kQuadAhead, (I + kQuadAhead) & 3, I == 0 ? hc + 3 * 2 * kRow : (hc ^ kHalf) + (I - 1) * 2 * kRow);
         cp_async_wait<kQuadAhead>();
-        __syncwarp();  // row s is in, from every lane's copies
-        float *ra = rd + ((s & (kQuadSlotsD - 1)) * 2 + 1) * kQuadWin + wc;
-        float rp[2];
+        if (PC != 2) __syncwarp();  // row s is in, from every lane's copies
+        float *ra = const_cast<float *>(ruvl) + (kD + hc) / 4 + (I * 2 + 1) * kQuadWin;
+        F2 rp;
         if (ALPHA) {
-            const float2 al = *reinterpret_cast<const float2 *>(ra);
-            const float r0f = p.rad * al.x, r1f = p.rad * al.y;
-            rp[0] = al.x == 0.f ? 0.f : (r0f <= p.bnd ? r0f : p.bnd);
-            rp[1] = al.y == 0.f ? 0.f : (r1f <= p.bnd ? r1f : p.bnd);
+            const F2 al = *reinterpret_cast<const F2 *>(ra);
+            const float rad = lo(qb[4]), bnd = hi(qb[4]);
+            const float r0f = rad * lo(al), r1f = rad * hi(al);
+            rp = pk(lo(al) == 0.f ? 0.f : (r0f <= bnd ? r0f : bnd), hi(al) == 0.f ? 0.f : (r1f <= bnd ? r1f : bnd));
         } else {
-            rp[0] = rp[1] = (unsigned)s < (unsigned)H ? radl : 0.f;
+            rp = (unsigned)s < (unsigned)H ? ln.rad : 0;
         }
-        *reinterpret_cast<float2 *>(ra) = make_float2(rp[0], rp[1]);
+        *reinterpret_cast<F2 *>(ra) = rp;
     };
-    int s = sb;
-    for (; s < r0 + LV; ++s) {  // the rows above the tile
-        stage(s);
-        quad_step<ALPHA, REDO, ROWSUMS, false, LV>(p, q, s, ustart, strip, ruv, rd, wc, outcol, ledge, wh1r1, gsum, dsum, uo, vo);
+    auto next_group = [&]() { hc ^= kHalf; };
+    // sums of four rows (a fixed tree) into their slots: after one exchange the
+    // lower half of the warp adds up the gaps and the upper half the dots
+    auto group_sums = [&](int row) {
+        if (!ROWSUMS || REDO) return;
+        double x = lane < 16 ? q.gacc : q.dacc;
+        x += __shfl_xor_sync(0xffffffffu, lane < 16 ? q.dacc : q.gacc, 16);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if ((lane & 15) == 0) p.rowpart[((int64_t)((row) >> 2) * nstrips + strip) * 2 + (lane >> 4)] = x;
+        q.gacc = q.dacc = 0.0;
+    };
+    auto row_gap = [&](int row) {
+        if (!ROWSUMS || !REDO) return;
+        const double x = warp_sum(q.gacc);
+        if (lane == 0 && p.rowpart) p.rowpart[((int64_t)row * nstrips + strip) * 2] = x;
+        q.gacc = 0.0;
+    };
+    // the rows above the tile
+#define FPB_QUAD_STEP(G, EDGE, I, S)                                                                            \
+    stage(S, I);                                                                                                 \
+    quad_step<PC, REDO, G, EDGE, LV, I>(p, ln, q, S, ruvl, ruvl + (kD + hc) / 4, ruvl + (kD + (hc ^ kHalf)) / 4, qb, uo, vo, (unsigned)(((S) - LV) * W))
+    FPB_QUAD_STEP(0, true, 0, sb);
+    FPB_QUAD_STEP(0, true, 1, sb + 1);
+    FPB_QUAD_STEP(0, true, 2, sb + 2);
+    FPB_QUAD_STEP(0, true, 3, sb + 3);
+    next_group();
+    FPB_QUAD_STEP(1, true, 0, sb + 4);
+    FPB_QUAD_STEP(1, true, 1, sb + 5);
+    FPB_QUAD_STEP(1, true, 2, sb + 6);
+    FPB_QUAD_STEP(1, true, 3, sb + 7);
+    next_group();
+    int t = 8;
+    // output rows, whole groups inside the image, then the rest
+    for (; t + 3 < T && sb + t + 3 < H; t += 4) {
+        const int s = sb + t;
+        FPB_QUAD_STEP(-1, false, 0, s);
+        row_gap(s - LV);
+        FPB_QUAD_STEP(-1, false, 1, s + 1);
+        row_gap(s - LV + 1);
+        FPB_QUAD_STEP(-1, false, 2, s + 2);
+        row_gap(s - LV + 2);
+        FPB_QUAD_STEP(-1, false, 3, s + 3);
+        row_gap(s - LV + 3);
+        group_sums(s - LV);
+        next_group();
     }
-    for (; s <= se; ++s) {  // output rows
-        stage(s);
-        quad_step<ALPHA, REDO, ROWSUMS, true, LV>(p, q, s, ustart, strip, ruv, rd, wc, outcol, ledge, wh1r1, gsum,
-                                                  dsum, uo, vo);
+    for (; t < T; t += 4) {
+        const int s = sb + t;
+        FPB_QUAD_STEP(-1, true, 0, s);
+        row_gap(s - LV);
+        if (t + 1 < T) {
+            FPB_QUAD_STEP(-1, true, 1, s + 1);
+            row_gap(s - LV + 1);
+        }
+        if (t + 2 < T) {
+            FPB_QUAD_STEP(-1, true, 2, s + 2);
+            row_gap(s - LV + 2);
+        }
+        if (t + 3 < T) {
+            FPB_QUAD_STEP(-1, true, 3, s + 3);
+            row_gap(s - LV + 3);
+        }
+        group_sums(s - LV);
+        next_group();
     }
+#undef FPB_QUAD_STEP
+    gsum = q.gacc;
+    dsum = q.dacc;
     cp_async_wait<0>();
 }
 
@@ -1678,14 +1815,14 @@ __device__ __forceinline__ void quad_control(const IsoState &st, const IsoImage 
 // REDO: the final iterate (the third's u) of images whose quad's check passed
 // (state redo == 3), from that quad's input buffers (fin_par, v = u when
 // redo_vsel) and momenta (redo_tn, redo_beta), into the other parity's u.
-template <bool ALPHA, bool REDO>
+template <int PC, bool ALPHA, bool REDO>
 __global__ void __launch_bounds__(32 * kQuadWarps, 4) iso2d_quad_kernel(StepArgs A, IsoCall c, IsoBuffers bf) {
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     __shared__ int flag;
     if (!REDO) asm volatile("griddepcontrol.wait;" ::: "memory");  // a programmatic dependent of the previous step
     const int b = REDO ? (int)blockIdx.z : step_image(bf, blockIdx.z);
     if (b < 0) return;
-    const IsoState st = bf.st[b];
+    const IsoState &st = bf.st[b];
     if (REDO) {
         if (st.redo != 3) return;
     } else {
@@ -1696,7 +1833,7 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 4) iso2d_quad_kernel(StepArgs
             return;
         }
     }
-    const IsoImage im = bf.img[b];
+    const IsoImage &im = bf.img[b];
     const int H = (int)A.g.L[0], W = (int)A.g.L[1];
     const int64_t N = A.g.N;
     const int pin = REDO ? st.fin_par : A.par, pout = pin ^ 1;
@@ -1717,7 +1854,7 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 4) iso2d_quad_kernel(StepArgs
     p.rad = (float)im.radius;
     p.bnd = (float)im.bound;
     quad_betas(REDO ? st.redo_tn : st.tn, REDO ? st.redo_beta : st.beta, p.beta);
-    p.rowpart = bf.part + (int64_t)b * bf.max_part * 2;
+    p.rowpart = REDO && !A.row_part ? nullptr : bf.part + (int64_t)b * bf.max_part * 2;
     // the block's warps take consecutive tiles (strip, band of A.rows rows) of
     // the image, strips fastest
     const int nstrips = quad_strips(W), nbands = (H + A.rows - 1) / A.rows;
@@ -1725,16 +1862,24 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 4) iso2d_quad_kernel(StepArgs
     double gs = 0.0, ds = 0.0;
     if (t < nstrips * nbands) {
         const int band = t / nstrips, r0 = band * A.rows;
-        quad_pass<ALPHA, REDO, true>(p, t - band * nstrips, r0, min(H, r0 + A.rows), gs, ds);
+        quad_pass<PC, ALPHA, REDO, true>(p, t - band * nstrips, r0, min(H, r0 + A.rows), gs, ds);
     }
-    if (REDO) return;
+    const double *part = bf.part + (int64_t)b * bf.max_part * 2;
+    if (REDO) {
+        // the gap that is reported: row by row, in order
+        if (!A.row_part || !arrive_last(bf.ticket + b, gridDim.x * gridDim.y, &flag)) return;
+        const double gap = sum_partials(part, H * nstrips, 2, 0, sh);
+        if (threadIdx.x != 0) return;
+        bf.ticket[b] = 0;
+        bf.st[b].gp = gap;
+        return;
+    }
     __syncthreads();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (!arrive_last(bf.ticket + b, gridDim.x * gridDim.y, &flag)) return;
-    const int nslot = H * nstrips;
-    const double *part = bf.part + (int64_t)b * bf.max_part * 2;
-    const double gap = sum_partials(part, nslot, 2, 0, sh);
-    const double dot = sum_partials(part, nslot, 2, 1, sh);
+    const int nslot = (H + 3) / 4 * nstrips;
+    double gap, dot;
+    sum_pairs(part, nslot, sh, gap, dot);
     if (threadIdx.x != 0) return;
     bf.ticket[b] = 0;
     IsoState s2;
@@ -1802,8 +1947,10 @@ __device__ __forceinline__ void ragged_single(const RagItem &item, const RagSlot
         part[item.blk * 2 + 1] = dsum;
     }
     if (!arrive_last(bf.ticket + b, sl.nblk, flag)) return;
-    const double gap = GAP ? sum_partials(part, sl.nblk, 2, 0, sh) : 0.0;
-    const double dot = test ? sum_partials(part, sl.nblk, 2, 1, sh) : 0.0;
+    double gap = 0.0, dot = 0.0;
+    if (GAP || test) sum_pairs(part, sl.nblk, sh, gap, dot);
+    if (!GAP) gap = 0.0;
+    if (!test) dot = 0.0;
     if (threadIdx.x != 0) return;
     bf.ticket[b] = 0;
     IsoState s2 = st;
@@ -1819,7 +1966,7 @@ __global__ void __launch_bounds__(128) iso2d_ragged_kernel(const RagItem *__rest
                                                            const int *__restrict__ n_items,
                                                            const RagSlot *__restrict__ slots, IsoBuffers bf,
                                                            int pairs) {
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     __shared__ int flag;
     if ((int)blockIdx.x >= *n_items) return;
     const RagItem item = items[blockIdx.x];
@@ -1844,7 +1991,7 @@ __global__ void __launch_bounds__(128, GAP2 ? 3 : 4) iso2d_ragged_pair_kernel(co
                                                                               const int *__restrict__ n_items,
                                                                               const RagSlot *__restrict__ slots,
                                                                               IsoBuffers bf) {
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     __shared__ int flag;
     if ((int)blockIdx.x >= *n_items) return;
     const RagItem item = items[blockIdx.x];
@@ -1886,8 +2033,8 @@ __global__ void __launch_bounds__(128, GAP2 ? 3 : 4) iso2d_ragged_pair_kernel(co
         }
     }
     if (!arrive_last(bf.ticket + b, sl.nblk, &flag)) return;
-    const double gap = GAP2 ? sum_partials(part, sl.nblk, 2, 0, sh) : 0.0;
-    const double dot = GAP2 ? sum_partials(part, sl.nblk, 2, 1, sh) : 0.0;
+    double gap = 0.0, dot = 0.0;
+    if (GAP2) sum_pairs(part, sl.nblk, sh, gap, dot);
     if (threadIdx.x != 0) return;
     bf.ticket[b] = 0;
     IsoState s2 = st;
@@ -1911,19 +2058,21 @@ __global__ void __launch_bounds__(128, GAP2 ? 3 : 4) iso2d_ragged_pair_kernel(co
 // the block's gap and restart-test sums (each lane's over the block's rows,
 // then the block's tree) go to the item's partial slot, summed in order by
 // the image's last block.
+// PC: columns per copy (quad_pass), 4 for rows of a multiple of 4 pixels.
+template <int PC>
 __global__ void __launch_bounds__(32 * kQuadWarps, 4) iso2d_ragged_quad_kernel(const RagItem *__restrict__ items,
                                                                               const int *__restrict__ n_items,
                                                                               const RagSlot *__restrict__ slots,
                                                                               IsoBuffers bf) {
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     __shared__ int flag;
     if ((int)blockIdx.x >= *n_items) return;
     const RagItem item = items[blockIdx.x];
     const int b = item.slot;
-    const RagSlot sl = slots[b];
-    const IsoState st = bf.st[b];
+    const RagSlot &sl = slots[b];
+    const IsoState &st = bf.st[b];
     if (st.status != kLive || !ragged_quad_ok(st, sl)) return;
-    const IsoImage im = bf.img[b];
+    const IsoImage &im = bf.img[b];
     const int pin = st.fin_par, pout = pin ^ 1;
     QuadTile p;
     p.D = static_cast<const float *>(bf.d) + sl.off;
@@ -1944,7 +2093,10 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 4) iso2d_ragged_quad_kernel(c
     p.rowpart = nullptr;
     const int strip = item.cs + (int)(threadIdx.x >> 5);
     double gs = 0.0, ds = 0.0;
-    if (strip < quad_strips(sl.W)) quad_pass<false, false, false>(p, strip, item.r0, min(sl.H, item.r0 + sl.qrows), gs, ds);
+    if (strip < quad_strips(sl.W)) {
+        const int r1 = min(sl.H, item.r0 + sl.qrows);
+        quad_pass<PC, false, false, false>(p, strip, item.r0, r1, gs, ds);
+    }
     const double gsum = block_sum(gs, sh);
     const double dsum = block_sum(ds, sh);
     double *part = bf.part + (int64_t)b * bf.max_part * 2;
@@ -1953,8 +2105,8 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 4) iso2d_ragged_quad_kernel(c
         part[item.blk * 2 + 1] = dsum;
     }
     if (!arrive_last(bf.ticket + b, sl.nquad, &flag)) return;
-    const double gap = sum_partials(part, sl.nquad, 2, 0, sh);
-    const double dot = sum_partials(part, sl.nquad, 2, 1, sh);
+    double gap, dot;
+    sum_pairs(part, sl.nquad, sh, gap, dot);
     if (threadIdx.x != 0) return;
     bf.ticket[b] = 0;
     IsoState s2;
@@ -1969,7 +2121,7 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 4) iso2d_ragged_quad_kernel(c
 
 template <class T, int K, bool ALPHA>
 __global__ void __launch_bounds__(256) iso_generic_kernel(StepArgs A, IsoCall c, IsoBuffers bf) {
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     __shared__ int flag;
     const int b = step_image(bf, blockIdx.y);
     if (b < 0) return;
@@ -2069,8 +2221,10 @@ __global__ void __launch_bounds__(256) iso_generic_kernel(StepArgs A, IsoCall c,
         part[blockIdx.x * 2 + 1] = dsum;
     }
     if (!arrive_last(bf.ticket + b, nblk, &flag)) return;
-    const double gap = do_gap ? sum_partials(part, nblk, 2, 0, sh) : 0.0;
-    const double dot = test ? sum_partials(part, nblk, 2, 1, sh) : 0.0;
+    double gap = 0.0, dot = 0.0;
+    if (do_gap || test) sum_pairs(part, nblk, sh, gap, dot);
+    if (!do_gap) gap = 0.0;
+    if (!test) dot = 0.0;
     if (threadIdx.x != 0) return;
     bf.ticket[b] = 0;
     IsoState s2 = st;
@@ -2104,7 +2258,7 @@ __device__ __forceinline__ double huber_h(double t, double dl) {
 
 template <class T, int K, bool SW, bool ANISO>
 __global__ void __launch_bounds__(256) huber_kernel(StepArgs A, IsoCall c, IsoBuffers bf) {
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     __shared__ int flag;
     const int b = step_image(bf, blockIdx.y);
     if (b < 0) return;
@@ -2295,7 +2449,7 @@ __global__ void __launch_bounds__(k3TX * k3TY) iso3d_kernel(StepArgs A, IsoCall 
     extern __shared__ __align__(16) unsigned char i3_smem[];
     T(*reg)[NA][k3R] = reinterpret_cast<T(*)[NA][k3R]>(i3_smem);
     T(*zs)[GAP ? 2 : 1][k3Z] = reinterpret_cast<T(*)[GAP ? 2 : 1][k3Z]>(i3_smem + k3Ring * NA * k3R * sizeof(T));
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     __shared__ int flag;
     asm volatile("griddepcontrol.wait;" ::: "memory");  // a programmatic dependent of the previous step
     const int b = step_image(bf, blockIdx.z);
@@ -2464,8 +2618,10 @@ __global__ void __launch_bounds__(k3TX * k3TY) iso3d_kernel(StepArgs A, IsoCall 
         part[blk * 2 + 1] = dsum;
     }
     if (!arrive_last(bf.ticket + b, nblk, &flag)) return;
-    const double gap = GAP ? sum_partials(part, nblk, 2, 0, sh) : 0.0;
-    const double dot = test ? sum_partials(part, nblk, 2, 1, sh) : 0.0;
+    double gap = 0.0, dot = 0.0;
+    if (GAP || test) sum_pairs(part, nblk, sh, gap, dot);
+    if (!GAP) gap = 0.0;
+    if (!test) dot = 0.0;
     if (threadIdx.x != 0) return;
     bf.ticket[b] = 0;
     IsoState s2 = st;
@@ -2508,7 +2664,7 @@ __global__ void __launch_bounds__(k3VX / 2 * k3VY, 4) iso3d_v2_kernel(StepArgs A
     extern __shared__ __align__(16) unsigned char i3v_smem[];
     T(*reg)[NA][k3VR] = reinterpret_cast<T(*)[NA][k3VR]>(i3v_smem);
     T(*zs)[GAP ? 2 : 1][k3VZ] = reinterpret_cast<T(*)[GAP ? 2 : 1][k3VZ]>(i3v_smem + k3Ring * NA * k3VR * sizeof(T));
-    __shared__ double sh[32];
+    __shared__ double sh[64];
     __shared__ int flag;
     asm volatile("griddepcontrol.wait;" ::: "memory");  // a programmatic dependent of the previous step
     const int b = step_image(bf, blockIdx.z);
@@ -2718,8 +2874,10 @@ __global__ void __launch_bounds__(k3VX / 2 * k3VY, 4) iso3d_v2_kernel(StepArgs A
         part[blk * 2 + 1] = dsum;
     }
     if (!arrive_last(bf.ticket + b, nblk, &flag)) return;
-    const double gap = GAP ? sum_partials(part, nblk, 2, 0, sh) : 0.0;
-    const double dot = test ? sum_partials(part, nblk, 2, 1, sh) : 0.0;
+    double gap = 0.0, dot = 0.0;
+    if (GAP || test) sum_pairs(part, nblk, sh, gap, dot);
+    if (!GAP) gap = 0.0;
+    if (!test) dot = 0.0;
     if (threadIdx.x != 0) return;
     bf.ticket[b] = 0;
     IsoState s2 = st;
@@ -3042,34 +3200,43 @@ void launch_3d_a(const StepShape &sh, StepArgs A, const IsoCall &c, const IsoBuf
     else launch_3d_v<T, ALPHA, false, false>(grid, A, c, bf, s);
 }
 
+// f(PC) for the columns per copy that rows of W columns allow.
+template <class F>
+void quad_kernels(int W, const F &f) {
+    if (W % 4 == 0) f(std::integral_constant<int, 4>{});
+    else if (W % 2 == 0) f(std::integral_constant<int, 2>{});
+    else f(std::integral_constant<int, 1>{});
+}
+
 // The quad launch: blocks of kQuadWarps tiles (a strip by `rows` rows). A
 // tile's march takes rows + 8 steps and the SMs hold a fixed number of
-// blocks at once, so the rows are chosen (8 to 64, in steps of 4) for the
+// blocks at once, so the rows are chosen (4 to 64, in steps of 4) for the
 // fewest waves of resident blocks times steps per tile: 48 on 64 images of
 // 512^2 (three waves of 56 steps, against five of 40 at 32 rows), 8 for one
-// image (a single wave of short tiles).
-void launch_quad(StepArgs A, const IsoCall &c, const IsoBuffers &bf, cudaStream_t s) {
+// image (a single wave of short tiles). Small launches take 4 rows (64^2: 0.58 ms
+// a solve against 0.64 at 8).
+int quad_rows(const Geometry &g, int64_t nimg) {
     static const int rows_hint = [] {  // tuning hint FASTPROX_B200_QUAD_ROWS
         const char *v = std::getenv("FASTPROX_B200_QUAD_ROWS");
         const int r = v ? std::atoi(v) : 0;
-        return (r >= 4 && r <= 256) ? r : 0;
+        return (r >= 4 && r <= 256) ? (r + 3) / 4 * 4 : 0;
     }();
     static const int64_t slots = [] {  // resident quad blocks on the device
         int dev = 0, sms = 148, per = 4;
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, iso2d_quad_kernel<true, false>, 32 * kQuadWarps,
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, iso2d_quad_kernel<4, true, false>, 32 * kQuadWarps,
                                                           kQuadSmem) != cudaSuccess || per < 1)
             per = 4;
         cudaGetLastError();
         return (int64_t)sms * per;
     }();
-    const int64_t H = A.g.L[0], ns = quad_strips((int)A.g.L[1]);
+    const int64_t H = g.L[0], ns = quad_strips((int)g.L[1]);
     auto blocks = [&](int rows) { return (ns * ((H + rows - 1) / rows) + kQuadWarps - 1) / kQuadWarps; };
     int rows = rows_hint;
     if (!rows) {
         double best = 0.0;
-        for (int r = 8; r <= 64; r += 4) {
-            const int64_t waves = (A.nimg * blocks(r) + slots - 1) / slots;
+        for (int r = 4; r <= 64; r += 4) {
+            const int64_t waves = (nimg * blocks(r) + slots - 1) / slots;
             const double cost = (double)waves * (double)(std::min<int64_t>(r, H) + 8);
             if (!rows || cost < best) {
                 rows = r;
@@ -3077,10 +3244,21 @@ void launch_quad(StepArgs A, const IsoCall &c, const IsoBuffers &bf, cudaStream_
             }
         }
     }
-    A.rows = rows;
-    const dim3 grid((unsigned)blocks(rows), 1, (unsigned)A.nimg);
-    if (c.has_alpha) launch_step(iso2d_quad_kernel<true, false>, grid, 32 * kQuadWarps, kQuadSmem, s, A, c, bf);
-    else launch_step(iso2d_quad_kernel<false, false>, grid, 32 * kQuadWarps, kQuadSmem, s, A, c, bf);
+    return rows;
+}
+dim3 quad_grid(const Geometry &g, int rows, int64_t nimg) {
+    const int64_t tiles = quad_strips((int)g.L[1]) * ((g.L[0] + rows - 1) / rows);
+    return dim3((unsigned)((tiles + kQuadWarps - 1) / kQuadWarps), 1, (unsigned)nimg);
+}
+
+void launch_quad(StepArgs A, const IsoCall &c, const IsoBuffers &bf, cudaStream_t s) {
+    A.rows = quad_rows(A.g, A.nimg);
+    const dim3 grid = quad_grid(A.g, A.rows, A.nimg);
+    quad_kernels((int)A.g.L[1], [&](auto pc) {
+        constexpr int PC = decltype(pc)::value;
+        if (c.has_alpha) launch_step(iso2d_quad_kernel<PC, true, false>, grid, 32 * kQuadWarps, kQuadSmem, s, A, c, bf);
+        else launch_step(iso2d_quad_kernel<PC, false, false>, grid, 32 * kQuadWarps, kQuadSmem, s, A, c, bf);
+    });
 }
 
 template <class T>
@@ -3218,10 +3396,11 @@ bool iso_ragged_pairs(int dtype, int vec) {
     return pairs_enabled() && dtype == 1 && vec == 4;
 }
 
-cudaError_t iso_ragged_quad_step(const RagItem *items, const int *n_items, int grid, const RagSlot *slots,
+cudaError_t iso_ragged_quad_step(bool odd, const RagItem *items, const int *n_items, int grid, const RagSlot *slots,
                                  const IsoBuffers &bf, cudaStream_t s) {
     if (grid <= 0) return cudaSuccess;
-    iso2d_ragged_quad_kernel<<<grid, 32 * kQuadWarps, kQuadSmem, s>>>(items, n_items, slots, bf);
+    if (odd) iso2d_ragged_quad_kernel<1><<<grid, 32 * kQuadWarps, kQuadSmem, s>>>(items, n_items, slots, bf);
+    else iso2d_ragged_quad_kernel<4><<<grid, 32 * kQuadWarps, kQuadSmem, s>>>(items, n_items, slots, bf);
     return cudaGetLastError();
 }
 
@@ -3329,7 +3508,7 @@ bool iso_quad_ok(int dtype, const Geometry &g, int max_part) {
         return !(v && v[0] == '0' && v[1] == 0);
     }();
     // rows narrower than 32 pixels keep the generic step (its gap terms in FP64)
-    return on && pairs_enabled() && dtype == 1 && g.k == 2 && g.L[1] >= 32 && g.L[1] % 4 == 0 && g.L[0] >= 2 &&
+    return on && pairs_enabled() && dtype == 1 && g.k == 2 && g.L[1] >= 32 && g.L[0] >= 2 &&
            g.L[0] * g.L[1] < (int64_t(1) << 31) && iso_quad_parts(g) <= max_part;
 }
 
@@ -3338,21 +3517,23 @@ int64_t iso_quad_parts(const Geometry &g) {
 }
 
 cudaError_t iso_redo(int dtype, const Geometry &g, const IsoCall &c, const IsoBuffers &bf, cudaStream_t s,
-                     bool quads) {
+                     bool quads, bool gaps) {
     if (g.k != 2 || g.B <= 0 || g.N <= 0) return cudaSuccess;
     if (quads && dtype == 1) {
-        // the quad's redo: three iterations over whole images, blocks of 32 rows
+        // the quad's redo: three iterations over whole images
         StepArgs A;
         A.g = g;
         A.max_iter = c.max_iter;
         A.par = 0;
-        A.rows = 32;
+        A.rows = quad_rows(g, g.B);
         A.nimg = g.B;
-        A.row_part = 0;
-        const int64_t tiles = quad_strips((int)g.L[1]) * ((g.L[0] + A.rows - 1) / A.rows);
-        const dim3 grid((unsigned)((tiles + kQuadWarps - 1) / kQuadWarps), 1, (unsigned)g.B);
-        if (c.has_alpha) iso2d_quad_kernel<true, true><<<grid, 32 * kQuadWarps, kQuadSmem, s>>>(A, c, bf);
-        else iso2d_quad_kernel<false, true><<<grid, 32 * kQuadWarps, kQuadSmem, s>>>(A, c, bf);
+        A.row_part = gaps && iso_quad_parts(g) <= bf.max_part ? 1 : 0;
+        const dim3 grid = quad_grid(g, A.rows, g.B);
+        quad_kernels((int)g.L[1], [&](auto pc) {
+            constexpr int PC = decltype(pc)::value;
+            if (c.has_alpha) iso2d_quad_kernel<PC, true, true><<<grid, 32 * kQuadWarps, kQuadSmem, s>>>(A, c, bf);
+            else iso2d_quad_kernel<PC, false, true><<<grid, 32 * kQuadWarps, kQuadSmem, s>>>(A, c, bf);
+        });
     }
     const dim3 grid((unsigned)std::min<int64_t>((g.N + 255) / 256, 1024), (unsigned)g.B);
     if (dtype == 1) {
