@@ -1988,7 +1988,7 @@ fp_status vjp_impl(const fp_op *op, fp_workspace *ws, const fp_array *ga, fp_arr
         return finish();
     }
     cudaError_t e = vjp_solve(ws->dtype, vg, bf, gsrc, gdst, ws->deriv_tol, ws->deriv_max_iter, ws->conj ? 1 : 0,
-                              params, s, ws->h_live, ws->ev[0], &nl);
+                              params, s, ws->h_live, ws->ev, &nl);
     if (e != cudaSuccess) return cuda_status(e);
     if (fp_status st = unstage_output(ws, gdst, gx)) return st;
     e = cudaMemcpyAsync(ws->h_ggam, ws->v_ggam, (size_t)g0.B * sizeof(double), cudaMemcpyDeviceToHost, s);
@@ -2121,7 +2121,7 @@ fp_status jvp_impl(const fp_op *op, fp_workspace *ws, const fp_array *dxa, doubl
         return cuda_status(e);
     }
     e = jvp_solve(ws->dtype, vg, bf, dsrc, ddst, dgamma, dir, dalpha, ws->deriv_tol, ws->deriv_max_iter,
-                  ws->conj ? 1 : 0, s, ws->h_live, ws->ev[0], &nl);
+                  ws->conj ? 1 : 0, s, ws->h_live, ws->ev, &nl);
     if (e != cudaSuccess) return cuda_status(e);
     if (fp_status st = unstage_output(ws, ddst, out)) return st;
     return read_cg(ws, nl);

@@ -142,15 +142,22 @@ __device__ __forceinline__ bool img_reduce(const VjpBuffers &bf, int b, unsigned
 }
 
 struct Px {  // a pixel's coordinates and its forward neighbours
-    int64_t co[3];
+    int co[3];
     bool has[3];
 };
 
 __device__ __forceinline__ Px pix_of(const VjpGeom &g, int64_t p) {
     Px x;
-    for (int a = 0; a < 3; ++a) {
-        x.co[a] = a < g.k ? (p / g.S[a]) % g.L[a] : 0;
-        x.has[a] = a < g.k && g.wa[a] != 0.0 && x.co[a] + 1 < g.L[a];
+    unsigned q = (unsigned)p;  // N < 2^31: 32-bit divisions, one fewer than axes
+#pragma unroll
+    for (int a = 2; a >= 0; --a) {
+        x.co[a] = 0;
+        if (a < g.k) {
+            const unsigned L = (unsigned)g.L[a], t = a > 0 ? q / L : 0u;
+            x.co[a] = (int)(q - t * L);
+            q = t;
+        }
+        x.has[a] = a < g.k && g.wa[a] != 0.0 && x.co[a] + 1 < (int)g.L[a];
     }
     return x;
 }
@@ -166,12 +173,12 @@ __device__ __forceinline__ double z_at(const VjpGeom &g, const VjpBuffers &bf, i
     if (mode != kModeFdpg) return (double)D[q];
     const T *U = static_cast<const T *>(bf.U[bf.st[b].fin_par]) + (int64_t)b * g.k * N;
     double z = (double)D[q];
+    const Px x = pix_of(g, q);
     for (int a = 0; a < g.k; ++a) {
         const double wh = g.wh[a];
         if (wh == 0.0) continue;
-        const int64_t co = (q / g.S[a]) % g.L[a];
         const double cur = (double)U[a * N + q];
-        const double prev = co > 0 ? (double)U[a * N + q - g.S[a]] : 0.0;
+        const double prev = x.co[a] > 0 ? (double)U[a * N + q - g.S[a]] : 0.0;
         z += wh * (cur - prev);
     }
     return z;
@@ -284,10 +291,10 @@ __device__ __forceinline__ double apply_y(const VjpGeom &g, const VjpBuffers &bf
     const double *PV = bf.pv + (int64_t)b * N;
     const double *Hh = bf.h + (int64_t)b * g.k * N;
     double y = PV[R[p]];
+    const Px x = pix_of(g, p);
     for (int a = 0; a < g.k; ++a) {
         if (g.wa[a] == 0.0) continue;
-        const int64_t co = (p / g.S[a]) % g.L[a];
-        const double prev = co > 0 ? Hh[a * N + p - g.S[a]] : 0.0;
+        const double prev = x.co[a] > 0 ? Hh[a * N + p - g.S[a]] : 0.0;
         y -= g.wa[a] * (Hh[a * N + p] - prev);
     }
     return y;
@@ -481,7 +488,32 @@ __global__ void __launch_bounds__(kT) cg_init(VjpGeom g, VjpBuffers bf, double t
     cs.max_iter = max_iter;
 }
 
-// h = H G pix with pix = pv[root] (tv_iso.cpp:870-877, 809-827)
+// (H G pix)_p of a pixel that is not flat, pix = pv[root] (tv_iso.cpp:870-877,
+// 809-827): c0 the pixel's value, cn its forward neighbours'. The roundings are
+// written out: conjugate gradients carry the last bit of one product into the
+// fifth digit of the result, which should not hang on how a loop is unrolled.
+template <class T>
+__device__ __forceinline__ void hg_at(const VjpGeom &g, const VjpBuffers &bf, const VjpImage &vi, int b, int64_t p,
+                                      const bool *has, double c0, const double *cn, const double *gz, double *out) {
+    double y[3] = {0.0, 0.0, 0.0}, nn = 0.0, dot = 0.0;
+    for (int a = 0; a < g.k; ++a) {
+        y[a] = has[a] ? __dmul_rn(g.wa[a], cn[a] - c0) : 0.0;
+        nn = __fma_rn(gz[a], gz[a], nn);
+    }
+    const double nr = sqrt(nn);
+    for (int a = 0; a < g.k; ++a) dot = __fma_rn(gz[a], y[a], dot);
+    double rp = vi.gs;
+    if (bf.alpha) {
+        const double al = (double)static_cast<const T *>(bf.alpha)[(int64_t)b * bf.alpha_stride + p];
+        rp = al == 0.0 ? 0.0 : __dmul_rn(vi.gs, al);
+    }
+    const double h = rp / fmax(nr, vi.mu);
+    for (int a = 0; a < g.k; ++a) {
+        const double na = gz[a] / nr;
+        out[a] = __dmul_rn(h, y[a] - __dmul_rn(na, dot) / nr);
+    }
+}
+
 template <class T>
 __global__ void __launch_bounds__(kT) cg_hg(VjpGeom g, VjpBuffers bf) {
     const int b = blockIdx.y;
@@ -494,54 +526,24 @@ __global__ void __launch_bounds__(kT) cg_hg(VjpGeom g, VjpBuffers bf) {
     double *Hh = bf.h + (int64_t)b * g.k * N;
     const VjpImage &vi = bf.vimg[b];
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += (int64_t)gridDim.x * blockDim.x) {
-        const Px x = pix_of(g, p);
-        if (F[p] & 1) {
-            for (int a = 0; a < g.k; ++a) Hh[a * N + p] = 0.0;
-            continue;
+        double hv[3] = {0.0, 0.0, 0.0};
+        if (!(F[p] & 1)) {
+            const Px x = pix_of(g, p);
+            double cn[3], gz[3];
+            for (int a = 0; a < g.k; ++a) {
+                cn[a] = x.has[a] ? PV[R[p + g.S[a]]] : 0.0;
+                gz[a] = GZ[a * N + p];
+            }
+            hg_at<T>(g, bf, vi, b, p, x.has, PV[R[p]], cn, gz, hv);
         }
-        const double c0 = PV[R[p]];
-        double y[3] = {0.0, 0.0, 0.0}, nn = 0.0, dot = 0.0;
-        for (int a = 0; a < g.k; ++a) {
-            y[a] = x.has[a] ? g.wa[a] * (PV[R[p + g.S[a]]] - c0) : 0.0;
-            nn += GZ[a * N + p] * GZ[a * N + p];
-        }
-        const double nr = sqrt(nn);
-        for (int a = 0; a < g.k; ++a) dot += GZ[a * N + p] * y[a];
-        double rp = vi.gs;
-        if (bf.alpha) {
-            const double al = (double)static_cast<const T *>(bf.alpha)[(int64_t)b * bf.alpha_stride + p];
-            rp = al == 0.0 ? 0.0 : vi.gs * al;
-        }
-        const double h = rp / fmax(nr, vi.mu);
-        for (int a = 0; a < g.k; ++a) {
-            const double na = GZ[a * N + p] / nr;
-            Hh[a * N + p] = h * (y[a] - na * dot / nr);
-        }
+        for (int a = 0; a < g.k; ++a) Hh[a * N + p] = hv[a];
     }
 }
 
-// after qv = A pv: alpha = rz / <pv, qv>
-__global__ void __launch_bounds__(kT) cg_alpha(VjpGeom g, VjpBuffers bf) {
-    __shared__ double sh[32];
-    __shared__ int flag;
-    const int b = blockIdx.y;
-    if (bf.cg[b].status != kCgLive) return;
-    const int64_t N = g.N;
-    const int *R = bf.root + (int64_t)b * N;
-    const double *PV = bf.pv + (int64_t)b * N, *QV = bf.qv + (int64_t)b * N;
-    double pq = 0.0;
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += (int64_t)gridDim.x * blockDim.x)
-        if (R[p] == p) pq += PV[p] * QV[p];
-    double t, unused;
-    if (!img_reduce(bf, b, blockIdx.x, gridDim.x, pq, 0.0, sh, &flag, t, unused, false)) return;
-    CgState &cs = bf.cg[b];
-    if (!(t > 0.0)) {
-        cs.status = kCgDone;
-        atomicSub(bf.live, 1);
-        return;
-    }
-    cs.alpha = cs.rz / t;
-}
+// A thread's entries in the kernels over region vectors go kU at a time, their
+// loads before the first store: one entry after another, each waiting for the
+// test whether it is a root, took 122 us for cg_read_alpha on 48 x 256^2.
+constexpr int kU = 4;
 
 // x += alpha pv, r -= alpha qv; beta, the residual and the stopping test
 __global__ void __launch_bounds__(kT) cg_step(VjpGeom g, VjpBuffers bf) {
@@ -556,13 +558,32 @@ __global__ void __launch_bounds__(kT) cg_step(VjpGeom g, VjpBuffers bf) {
     double *X = bf.x + (int64_t)b * N, *Rr = bf.r + (int64_t)b * N;
     const double *PV = bf.pv + (int64_t)b * N, *QV = bf.qv + (int64_t)b * N, *DI = bf.dinv + (int64_t)b * N;
     double rzn = 0.0, rn = 0.0;
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += (int64_t)gridDim.x * blockDim.x) {
-        if (R[p] != p) continue;
-        X[p] += al * PV[p];
-        const double r = Rr[p] - al * QV[p];
-        Rr[p] = r;
-        rzn += r * r * DI[p];
-        rn += r * r / (double)C[p];
+    const int64_t st = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t p0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p0 < N; p0 += kU * st) {
+        bool root[kU];
+        int c[kU];
+        double x[kU], r[kU], pv[kU], qv[kU], di[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int64_t p = p0 + u * st < N ? p0 + u * st : p0;
+            root[u] = R[p] == p && p0 + u * st < N;
+            c[u] = C[p];
+            x[u] = X[p];
+            r[u] = Rr[p];
+            pv[u] = PV[p];
+            qv[u] = QV[p];
+            di[u] = DI[p];
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            if (!root[u]) continue;
+            const int64_t p = p0 + u * st;
+            X[p] = __fma_rn(al, pv[u], x[u]);
+            const double rr = __fma_rn(-al, qv[u], r[u]);
+            Rr[p] = rr;
+            rzn = __fma_rn(__dmul_rn(rr, rr), di[u], rzn);
+            rn += __dmul_rn(rr, rr) / (double)c[u];
+        }
     }
     double t0, t1;
     if (!img_reduce(bf, b, blockIdx.x, gridDim.x, rzn, rn, sh, &flag, t0, t1, false)) return;
@@ -585,8 +606,258 @@ __global__ void cg_pv(VjpGeom g, VjpBuffers bf) {
     const int *R = bf.root + (int64_t)b * N;
     double *PV = bf.pv + (int64_t)b * N;
     const double *Rr = bf.r + (int64_t)b * N, *DI = bf.dinv + (int64_t)b * N;
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += (int64_t)gridDim.x * blockDim.x)
-        if (R[p] == p) PV[p] = Rr[p] * DI[p] + be * PV[p];
+    const int64_t st = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t p0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p0 < N; p0 += kU * st) {
+        bool root[kU];
+        double r[kU], di[kU], pv[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int64_t p = p0 + u * st < N ? p0 + u * st : p0;
+            root[u] = R[p] == p && p0 + u * st < N;
+            r[u] = Rr[p];
+            di[u] = DI[p];
+            pv[u] = PV[p];
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u)
+            if (root[u]) PV[p0 + u * st] = __fma_rn(r[u], di[u], __dmul_rn(be, pv[u]));
+    }
+}
+
+// ---- the iteration's product on 2D images ----------------------------------------
+//
+// cg_hg and the first pass of the region sums (rs_max) over tiles of an image in
+// one kernel: pix over the tile and one entry around it is gathered into shared
+// memory once, h formed there over the tile, the row above and the column on the
+// left, and y = pix + G^T h written from it, so h never goes to memory. What an
+// iteration does not change is formed once per solve (cg_prep2): |G z|, its
+// reciprocal and the scale of H, in the planes of h and b, which are free then.
+// As two kernels (a square root and five divisions per pixel, 64-bit divisions
+// for the coordinates) they took 118 of the 250 us of an iteration on 48 x 256^2;
+// this takes 55 (its arrays' 180 MB about 27 at the copy rate, the rest FP64).
+constexpr int kTileW = 32, kTileH = 32, kTileT = 512;
+
+// x / nr from yr = 1 / nr rounded: the quotient of the reciprocal corrected twice
+// by its residual, formed exactly by a fused operation (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000", 1990): the rounded quotient,
+// as the division gives it, while nothing underflows.
+__device__ __forceinline__ double div_by(double x, double nr, double yr) {
+    double q = __dmul_rn(x, yr);
+    q = __fma_rn(__fma_rn(-q, nr, x), yr, q);
+    return __fma_rn(__fma_rn(-q, nr, x), yr, q);
+}
+
+template <class T>
+__global__ void __launch_bounds__(kT) cg_prep2(VjpGeom g, VjpBuffers bf) {
+    const int b = blockIdx.y;
+    if (bf.cg[b].status != kCgLive) return;
+    const int64_t N = g.N, o = (int64_t)b * N;
+    const double *GZ = bf.gz + 2 * o;
+    const uint8_t *F = bf.flat + o;
+    double *NR = bf.h + 2 * o, *YR = NR + N, *HS = bf.b + o;
+    const VjpImage vi = bf.vimg[b];
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += (int64_t)gridDim.x * blockDim.x) {
+        if (F[p] & 1) continue;
+        const double nr = sqrt(__fma_rn(GZ[N + p], GZ[N + p], __dmul_rn(GZ[p], GZ[p])));
+        double rp = vi.gs;
+        if (bf.alpha) {
+            const double al = (double)static_cast<const T *>(bf.alpha)[(int64_t)b * bf.alpha_stride + p];
+            rp = al == 0.0 ? 0.0 : __dmul_rn(vi.gs, al);
+        }
+        NR[p] = nr;
+        YR[p] = 1.0 / nr;
+        HS[p] = rp / fmax(nr, vi.mu);
+    }
+}
+
+__global__ void __launch_bounds__(kTileT, 2) cg_y2(VjpGeom g, VjpBuffers bf) {
+    __shared__ double sv[kTileH + 2][kTileW + 2];                                // pix from (r0 - 1, c0 - 1)
+    __shared__ double sh0[kTileH + 1][kTileW + 1], sh1[kTileH + 1][kTileW + 1];  // h from there
+    __shared__ double sh[32];
+    __shared__ int flag;
+    const int b = blockIdx.y;
+    if (bf.cg[b].status != kCgLive) return;
+    const int H = (int)g.L[0], W = (int)g.L[1];
+    const int64_t N = g.N, o = (int64_t)b * N;
+    const int *R = bf.root + o;
+    const double *PV = bf.pv + o, *GZ = bf.gz + 2 * o, *NR = bf.h + 2 * o, *YR = NR + N, *HS = bf.b + o;
+    const uint8_t *F = bf.flat + o;
+    double *Y = bf.y + o;
+    const double w0 = g.wa[0], w1 = g.wa[1];
+    const int tw = (W + kTileW - 1) / kTileW, th = (H + kTileH - 1) / kTileH;
+    double m = 0.0;
+    for (int tile = blockIdx.x; tile < tw * th; tile += gridDim.x) {
+        const int r0 = tile / tw * kTileH, c0 = tile % tw * kTileW;
+        // every load of the tile is issued before the first is used
+        constexpr int kP = ((kTileH + 1) * (kTileW + 1) + kTileT - 1) / kTileT;  // entries of h per thread
+        constexpr int kV = ((kTileH + 2) * (kTileW + 2) + kTileT - 1) / kTileT;  // entries of pix per thread
+        int root[kV];
+#pragma unroll
+        for (int k = 0; k < kV; ++k) {
+            const int i = threadIdx.x + k * kTileT, lr = i / (kTileW + 2), lc = i - lr * (kTileW + 2);
+            const int r = r0 - 1 + lr, c = c0 - 1 + lc;
+            root[k] = lr < kTileH + 2 && r >= 0 && r < H && c >= 0 && c < W ? R[r * W + c] : -1;
+        }
+        double gz0[kP], gz1[kP], nr[kP], yr[kP], hs[kP];
+        bool go[kP];
+#pragma unroll
+        for (int k = 0; k < kP; ++k) {
+            const int i = threadIdx.x + k * kTileT, lr = i / (kTileW + 1), lc = i - lr * (kTileW + 1);
+            const int r = r0 - 1 + lr, c = c0 - 1 + lc;
+            const bool in = lr < kTileH + 1 && r >= 0 && r < H && c >= 0 && c < W;
+            const int p = in ? r * W + c : 0;
+            go[k] = in && !(F[p] & 1);
+        }
+#pragma unroll
+        for (int k = 0; k < kP; ++k) {  // (flat entries come in stretches: their sectors are not read)
+            const int i = threadIdx.x + k * kTileT, lr = i / (kTileW + 1), lc = i - lr * (kTileW + 1);
+            const int p = go[k] ? (r0 - 1 + lr) * W + c0 - 1 + lc : 0;
+            gz0[k] = GZ[p];
+            gz1[k] = GZ[N + p];
+            nr[k] = NR[p];
+            yr[k] = YR[p];
+            hs[k] = HS[p];
+        }
+        double pix[kV];
+#pragma unroll
+        for (int k = 0; k < kV; ++k) pix[k] = root[k] >= 0 ? PV[root[k]] : 0.0;
+#pragma unroll
+        for (int k = 0; k < kV; ++k) {
+            const int i = threadIdx.x + k * kTileT, lr = i / (kTileW + 2);
+            if (lr < kTileH + 2) sv[lr][i - lr * (kTileW + 2)] = pix[k];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kP; ++k) {
+            const int i = threadIdx.x + k * kTileT, lr = i / (kTileW + 1), lc = i - lr * (kTileW + 1);
+            if (lr > kTileH) continue;
+            const int r = r0 - 1 + lr, c = c0 - 1 + lc;
+            double h0 = 0.0, h1 = 0.0;
+            if (go[k]) {  // hg_at, its divisions by nr from yr
+                const double v = sv[lr][lc];
+                const double y0 = w0 != 0.0 && r + 1 < H ? __dmul_rn(w0, sv[lr + 1][lc] - v) : 0.0;
+                const double y1 = w1 != 0.0 && c + 1 < W ? __dmul_rn(w1, sv[lr][lc + 1] - v) : 0.0;
+                const double dot = __fma_rn(gz1[k], y1, __dmul_rn(gz0[k], y0));
+                const double n0 = div_by(gz0[k], nr[k], yr[k]), n1 = div_by(gz1[k], nr[k], yr[k]);
+                h0 = __dmul_rn(hs[k], y0 - div_by(__dmul_rn(n0, dot), nr[k], yr[k]));
+                h1 = __dmul_rn(hs[k], y1 - div_by(__dmul_rn(n1, dot), nr[k], yr[k]));
+            }
+            sh0[lr][lc] = h0;
+            sh1[lr][lc] = h1;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < kTileH * kTileW; i += kTileT) {
+            const int lr = i / kTileW + 1, lc = i % kTileW + 1, r = r0 - 1 + lr, c = c0 - 1 + lc;
+            if (r >= H || c >= W) continue;
+            double y = sv[lr][lc];
+            if (w0 != 0.0) y = __fma_rn(-w0, sh0[lr][lc] - sh0[lr - 1][lc], y);
+            if (w1 != 0.0) y = __fma_rn(-w1, sh1[lr][lc] - sh1[lr][lc - 1], y);
+            Y[(int64_t)r * W + c] = y;
+            m = fmax(m, fabs(y));
+        }
+        __syncthreads();
+    }
+    double mx, unused;
+    if (!img_reduce(bf, b, blockIdx.x, gridDim.x, m, 0.0, sh, &flag, mx, unused, true)) return;
+    bf.cg[b].fx = fixed_exp(mx, N);
+}
+
+// The region sums of y: added up run by run within a warp (equal roots side by
+// side) with an atomic pair per run; a region of one pixel takes none, its value
+// goes to qv at once. (An atomic pair per pixel took 43 us on 48 x 256^2.)
+__global__ void __launch_bounds__(kT) cg_add(VjpGeom g, VjpBuffers bf) {
+    const int b = blockIdx.y;
+    if (bf.cg[b].status != kCgLive) return;
+    const int N = (int)g.N, s = bf.cg[b].fx, lane = threadIdx.x & 31;
+    const int64_t o = (int64_t)b * N;
+    const int *R = bf.root + o, *C = bf.cnt + o;
+    const double *Y = bf.y + o;
+    double *QV = bf.qv + o;
+    unsigned long long *A = bf.acc + 2 * o;
+    for (int64_t p0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; p0 < N;
+         p0 += (int64_t)gridDim.x * blockDim.x) {
+        const int p = (int)p0 + lane;
+        const int r = p < N ? R[p] : -1;
+        const bool sum = r >= 0 && C[r] > 1;
+        I128 x = r >= 0 ? to_fixed(Y[p], s) : I128{0ull, 0ll};
+        if (r >= 0 && !sum) QV[p] = from_fixed(x.lo, x.hi, s);
+        if (!__any_sync(0xffffffffu, sum)) continue;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            I128 u;
+            u.lo = __shfl_up_sync(0xffffffffu, x.lo, d);
+            u.hi = __shfl_up_sync(0xffffffffu, x.hi, d);
+            if (lane >= d) x = add128(x, u);
+        }
+        const int rl = __shfl_up_sync(0xffffffffu, r, 1), rn = __shfl_down_sync(0xffffffffu, r, 1);
+        const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || r != rl);
+        const int first = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+        I128 u;  // the scan before the run's first entry
+        u.lo = __shfl_sync(0xffffffffu, x.lo, first > 0 ? first - 1 : 0);
+        u.hi = __shfl_sync(0xffffffffu, x.hi, first > 0 ? first - 1 : 0);
+        if (sum && (lane == 31 || r != rn)) {
+            if (first > 0) {
+                const unsigned long long lo = x.lo - u.lo;
+                x.hi -= u.hi + (x.lo < u.lo ? 1 : 0);
+                x.lo = lo;
+            }
+            const unsigned long long old = atomicAdd(A + 2 * (int64_t)r, x.lo);
+            const unsigned long long carry = old + x.lo < old ? 1ull : 0ull;
+            atomicAdd(A + 2 * (int64_t)r + 1, (unsigned long long)x.hi + carry);
+        }
+    }
+}
+
+// The read-out of cg_add at the roots (the words cleared), and
+// alpha = rz / <pv, qv>.
+__global__ void __launch_bounds__(kT) cg_read_alpha(VjpGeom g, VjpBuffers bf) {
+    __shared__ double sh[32];
+    __shared__ int flag;
+    const int b = blockIdx.y;
+    if (bf.cg[b].status != kCgLive) return;
+    const int s = bf.cg[b].fx;
+    const int64_t N = g.N, o = (int64_t)b * N;
+    const int *R = bf.root + o, *C = bf.cnt + o;
+    const double *PV = bf.pv + o;
+    double *QV = bf.qv + o;
+    ulonglong2 *A = reinterpret_cast<ulonglong2 *>(bf.acc + 2 * o);
+    double pq = 0.0;
+    const int64_t st = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t p0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p0 < N; p0 += kU * st) {
+        bool root[kU], sum[kU];
+        double pv[kU], q[kU];
+        ulonglong2 x[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int64_t p = p0 + u * st < N ? p0 + u * st : p0;
+            root[u] = R[p] == p && p0 + u * st < N;
+            sum[u] = C[p] > 1;
+            pv[u] = PV[p];
+            q[u] = QV[p];
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u)
+            if (root[u] && sum[u]) x[u] = A[p0 + u * st];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            if (!root[u]) continue;
+            if (sum[u]) {
+                q[u] = from_fixed(x[u].x, (long long)x[u].y, s);
+                A[p0 + u * st] = make_ulonglong2(0ull, 0ull);
+                QV[p0 + u * st] = q[u];
+            }
+            pq = __fma_rn(pv[u], q[u], pq);
+        }
+    }
+    double t, unused;
+    if (!img_reduce(bf, b, blockIdx.x, gridDim.x, pq, 0.0, sh, &flag, t, unused, false)) return;
+    CgState &cs = bf.cg[b];
+    if (!(t > 0.0)) {
+        cs.status = kCgDone;
+        atomicSub(bf.live, 1);
+        return;
+    }
+    cs.alpha = cs.rz / t;
 }
 
 // ---- outputs (tv_iso.cpp:1014-1057) --------------------------------------------
@@ -823,10 +1094,10 @@ __global__ void __launch_bounds__(kT) jvp_rhs(VjpGeom g, VjpBuffers bf) {
     double *Y = bf.y + (int64_t)b * N;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += (int64_t)gridDim.x * blockDim.x) {
         double t = Y[p];
+        const Px x = pix_of(g, p);
         for (int a = 0; a < g.k; ++a) {
             if (g.wa[a] == 0.0) continue;
-            const int64_t co = (p / g.S[a]) % g.L[a];
-            const double prev = co > 0 ? Hh[a * N + p - g.S[a]] : 0.0;
+            const double prev = x.co[a] > 0 ? Hh[a * N + p - g.S[a]] : 0.0;
             t += g.wa[a] * (Hh[a * N + p] - prev);
         }
         Y[p] = t;
@@ -1323,7 +1594,7 @@ cudaError_t structure_t(const VjpGeom &g, const VjpBuffers &bf, cudaStream_t s) 
 // gradients in chunks of 8 iterations until every image has stopped.
 template <class T>
 cudaError_t solve_system(const VjpGeom &g, const VjpBuffers &bf, int kind, const T *gin, double tol, int max_iter,
-                         cudaStream_t s, int *h_live, cudaEvent_t ev, int64_t &nl) {
+                         cudaStream_t s, int *h_live, const cudaEvent_t *ev, int64_t &nl) {
     const dim3 grid(pblocks(g), (unsigned)g.B);
     rs_max<T><<<grid, kT, 0, s>>>(g, bf, kind, gin);
     rs_add<T><<<grid, kT, 0, s>>>(g, bf, kind, gin);
@@ -1337,29 +1608,43 @@ cudaError_t solve_system(const VjpGeom &g, const VjpBuffers &bf, int kind, const
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const int chunk = 8;
+    const int64_t tiles = ((g.L[0] + kTileH - 1) / kTileH) * ((g.L[1] + kTileW - 1) / kTileW);
+    const dim3 tgrid((unsigned)std::min<int64_t>(tiles, 512), (unsigned)g.B);
+    if (g.k == 2) {
+        cg_prep2<T><<<grid, kT, 0, s>>>(g, bf);
+        ++nl;
+    }
     for (int it = 0; it < max_iter + chunk; it += chunk) {
         for (int j = 0; j < chunk; ++j) {
-            cg_hg<T><<<grid, kT, 0, s>>>(g, bf);
-            rs_max<T><<<grid, kT, 0, s>>>(g, bf, 1, gin);
-            rs_add<T><<<grid, kT, 0, s>>>(g, bf, 1, gin);
-            rs_read<<<grid, kT, 0, s>>>(g, bf, 1, bf.qv);
-            cg_alpha<<<grid, kT, 0, s>>>(g, bf);
+            if (g.k == 2) {
+                cg_y2<<<tgrid, kTileT, 0, s>>>(g, bf);
+            } else {
+                cg_hg<T><<<grid, kT, 0, s>>>(g, bf);
+                rs_max<T><<<grid, kT, 0, s>>>(g, bf, 1, gin);
+            }
+            cg_add<<<grid, kT, 0, s>>>(g, bf);
+            cg_read_alpha<<<grid, kT, 0, s>>>(g, bf);
             cg_step<<<grid, kT, 0, s>>>(g, bf);
             cg_pv<<<grid, kT, 0, s>>>(g, bf);
-            nl += 7;
+            nl += (g.k == 2 ? 1 : 2) + 4;
         }
-        e = cudaMemcpyAsync(h_live, bf.live, sizeof(int), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaEventRecord(ev, s);
-        if (e == cudaSuccess) e = cudaEventSynchronize(ev);
+        // the live count is read one chunk behind, so that the device has the next
+        // chunk when the host waits (its launches exit at once after the last)
+        const int slot = (it / chunk) & 1;
+        e = cudaMemcpyAsync(h_live + slot, bf.live, sizeof(int), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaEventRecord(ev[slot], s);
+        if (e == cudaSuccess && it > 0) {
+            e = cudaEventSynchronize(ev[slot ^ 1]);
+            if (e == cudaSuccess && h_live[slot ^ 1] == 0) break;
+        }
         if (e != cudaSuccess) return e;
-        if (*h_live == 0) break;
     }
     return cudaSuccess;
 }
 
 template <class T>
 cudaError_t vjp_t(const VjpGeom &g, const VjpBuffers &bf, const void *gin, void *gx, double tol, int max_iter, int conj,
-                  bool params, cudaStream_t s, int *h_live, cudaEvent_t ev, int64_t *launches) {
+                  bool params, cudaStream_t s, int *h_live, const cudaEvent_t *ev, int64_t *launches) {
     const dim3 grid(pblocks(g), (unsigned)g.B);
     const T *gi = static_cast<const T *>(gin);
     int64_t nl = 0;
@@ -1389,7 +1674,7 @@ cudaError_t vjp_t(const VjpGeom &g, const VjpBuffers &bf, const void *gin, void 
 template <class T>
 cudaError_t jvp_t(const VjpGeom &g, const VjpBuffers &bf, const void *dx, void *dz, double dgamma, const JvpDir &dir,
                   const double *dalpha, double tol, int max_iter, int conj, cudaStream_t s, int *h_live,
-                  cudaEvent_t ev, int64_t *launches) {
+                  const cudaEvent_t *ev, int64_t *launches) {
     const dim3 grid(pblocks(g), (unsigned)g.B);
     const T *dxi = static_cast<const T *>(dx);
     int64_t nl = 0;
@@ -1487,7 +1772,7 @@ cudaError_t vjp_structure(int dtype, const VjpGeom &g, const VjpBuffers &bf, cud
 }
 
 cudaError_t vjp_solve(int dtype, const VjpGeom &g, const VjpBuffers &bf, const void *gin, void *gx, double tol,
-                      int max_iter, int conj, bool params, cudaStream_t s, int *h_live, cudaEvent_t ev,
+                      int max_iter, int conj, bool params, cudaStream_t s, int *h_live, const cudaEvent_t *ev,
                       int64_t *launches) {
     return dtype == 1 ? vjp_t<float>(g, bf, gin, gx, tol, max_iter, conj, params, s, h_live, ev, launches)
                       : vjp_t<double>(g, bf, gin, gx, tol, max_iter, conj, params, s, h_live, ev, launches);
@@ -1495,7 +1780,7 @@ cudaError_t vjp_solve(int dtype, const VjpGeom &g, const VjpBuffers &bf, const v
 
 cudaError_t jvp_solve(int dtype, const VjpGeom &g, const VjpBuffers &bf, const void *dx, void *dz, double dgamma,
                       const JvpDir &dir, const double *dalpha, double tol, int max_iter, int conj, cudaStream_t s,
-                      int *h_live, cudaEvent_t ev, int64_t *launches) {
+                      int *h_live, const cudaEvent_t *ev, int64_t *launches) {
     return dtype == 1 ? jvp_t<float>(g, bf, dx, dz, dgamma, dir, dalpha, tol, max_iter, conj, s, h_live, ev, launches)
                       : jvp_t<double>(g, bf, dx, dz, dgamma, dir, dalpha, tol, max_iter, conj, s, h_live, ev,
                                       launches);

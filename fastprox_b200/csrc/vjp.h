@@ -121,12 +121,12 @@ cudaError_t an_jvp_solve(int dtype, const VjpGeom &g, const VjpBuffers &bf, cons
 // the axis weights' into gw and the pixel weights' (summed over the images)
 // into qv[0, N).
 cudaError_t vjp_solve(int dtype, const VjpGeom &g, const VjpBuffers &bf, const void *gin, void *gx, double tol,
-                      int max_iter, int conj, bool params, cudaStream_t s, int *h_live, cudaEvent_t ev,
+                      int max_iter, int conj, bool params, cudaStream_t s, int *h_live, const cudaEvent_t *ev,
                       int64_t *launches);
 // dz = J_x dx + (dz/dgamma) dgamma + (dz/dw) dw + (dz/dalpha) dalpha per image;
 // dx and dalpha (N doubles on the device, outside x, r, y and h) may be null.
 cudaError_t jvp_solve(int dtype, const VjpGeom &g, const VjpBuffers &bf, const void *dx, void *dz, double dgamma,
                       const JvpDir &dir, const double *dalpha, double tol, int max_iter, int conj, cudaStream_t s,
-                      int *h_live, cudaEvent_t ev, int64_t *launches);
+                      int *h_live, const cudaEvent_t *ev, int64_t *launches);
 
 }  // namespace fpb
