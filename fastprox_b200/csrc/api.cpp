@@ -557,8 +557,8 @@ fp_status fpb_workspace_build(const fp_op *op, const Arr &x, const fp_options &o
     ws->max_part = std::max(ws->max_part, 4096);
     if (ws->shape_.kind == 4)  // per-row partial sums of the lean 2D step
         ws->max_part = (int)std::max<int64_t>(ws->max_part, (int64_t)ws->shape_.gx * g.L[0]);
-    if (x.dtype == FP_F32 && g.k == 2 && !op->huber)  // per-row, per-strip partial sums of the quad launch
-        ws->max_part = (int)std::max<int64_t>(ws->max_part, iso_quad_parts(g));
+    if (g.k == 2 && !op->huber)  // per-row, per-strip partial sums of the quad launch
+        ws->max_part = (int)std::max<int64_t>(ws->max_part, iso_quad_parts(x.dtype, g));
     if (op->kind == kAniso && !op->huber) {
         // the untiled fibre passes: a block of 128 fibres per partial, three
         // axes in one launch for FDPG-3

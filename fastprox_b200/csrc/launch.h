@@ -75,14 +75,14 @@ inline int iso_variant(int64_t k, int max_iter, bool warm) {
     return (k % 4 == 0 || k == max_iter) ? 2 : 0;
 }
 // Iterations k .. k + 3 in one launch (the quad), for k = 1 mod 4 and
-// k + 3 < max_iter where iso_quad_ok (2D float32 rows of 32 pixels or more):
+// k + 3 < max_iter where iso_quad_ok (2D rows of 32 pixels or more):
 // the fourth carries the gap check of the third iterate and the restart test;
 // when the check passes, the final u is the third iterate, formed again by
 // iso_redo.
 constexpr int kVariantQuad = 5;
 bool iso_quad_ok(int dtype, const Geometry &g, int max_part);
 // Partial-sum slots per image the quad needs (one per row and warp strip).
-int64_t iso_quad_parts(const Geometry &g);
+int64_t iso_quad_parts(int dtype, const Geometry &g);
 inline int iso_quad_at(int64_t k, int max_iter) {
     return (k > 0 && (k & 3) == 1 && k + 3 < max_iter) ? kVariantQuad : -1;
 }

@@ -1342,40 +1342,46 @@ __global__ void iso2d_redo_state(IsoState *st, int64_t B) {
 // 64-bit registers, four steps unrolled with fixed ring slots, the sums of four
 // rows at a time, momenta in shared memory and a square root without branches
 // made it 170 us (64 x 512^2 with pixel weights 48.8 -> 35.1 ms a solve).
+// Float64: one column per lane (windows of 32, 24 written), the same ring in bytes;
+// bound by the four dependent levels of a step (FP64 latency, 0.25 us each at three
+// blocks per SM) more than by FP64 rate. Four 384 x 320 images at 1e-8: 26.4 ms in
+// single steps of 15 us, 11.4 in quads.
 // ---------------------------------------------------------------------------
-constexpr int kQuadWin = 64;                        // window columns of a warp: two per lane
+// A lane's columns: two floats (one packed pair) or one double; a window is 32
+// lanes wide, a ring row 256 bytes.
+template <class T>
+constexpr int kQuadCols = 8 / (int)sizeof(T);
 constexpr int kQuadHalo = 4;                        // one column per iteration on each side
-constexpr int kQuadOut = kQuadWin - 2 * kQuadHalo;  // columns a warp writes
 constexpr int kQuadWarps = 4;                       // strips side by side per block
 constexpr int kQuadAhead = 3;                       // rows in flight beyond the row being read
 constexpr int kQuadSlotsUV = 4;                     // ring rows of v0, v1, u0, u1 (read at their own step)
 constexpr int kQuadSlotsD = 8;                      // ring rows of d and the radii (read by all four iterations)
-constexpr int kQuadRingFloats = kQuadSlotsUV * 4 * kQuadWin + kQuadSlotsD * 2 * kQuadWin;
-constexpr size_t kQuadSmem = (size_t)kQuadWarps * kQuadRingFloats * sizeof(float);
+constexpr int kQuadRow = 256;                       // bytes of a ring row
+constexpr int kQuadRingBytes = (kQuadSlotsUV * 4 + kQuadSlotsD * 2) * kQuadRow;
+constexpr size_t kQuadSmem = (size_t)kQuadWarps * kQuadRingBytes;
 
-// Strips of a row of W columns, W rounded up to a multiple of 4 (a window
-// starts on 16 bytes; columns past W are zero): one window when W <= 64 (its
-// edges are the image's, so it needs no halo); else a first window at column 0
-// writing columns 0 .. 59 (no halo on the image's edge), windows at 56 k writing
-// 56 k + 4 .. 56 k + 59, and a last window ending at column W writing the rest
-// (9 strips for a row of 512, against 10 with a halo on every side).
-__host__ __device__ constexpr int quad_strips(int W) {
-    return W <= kQuadWin ? 1
-                         : 2 + ((W - 2 * (kQuadWin - kQuadHalo) > 0)
-                                    ? ((W + 3) / 4 * 4 - 2 * (kQuadWin - kQuadHalo) + kQuadOut - 1) / kQuadOut
-                                    : 0);
+// Strips of a row of W columns, nc columns per lane, W rounded up to whole
+// 16-byte pieces (a window starts on 16 bytes; columns past W are zero). For
+// float: one window when W <= 64 (its edges are the image's, so it needs no
+// halo); else a first window at column 0 writing columns 0 .. 59 (no halo on the
+// image's edge), windows at 56 k writing 56 k + 4 .. 56 k + 59, and a last window
+// ending at column W writing the rest (9 strips for a row of 512, against 10 with
+// a halo on every side).
+__host__ __device__ constexpr int quad_strips(int W, int nc) {
+    const int win = 32 * nc, edge = win - kQuadHalo, out = win - 2 * kQuadHalo, pc = 2 * nc;
+    return W <= win ? 1 : 2 + (W - 2 * edge > 0 ? ((W + pc - 1) / pc * pc - 2 * edge + out - 1) / out : 0);
 }
-// Strip k's window (first column, a multiple of 4) and the columns it writes.
-__host__ __device__ inline void quad_strip_cols(int W, int k, int &c0, int &lo, int &hi) {
-    const int n = quad_strips(W);
+// Strip k's window (first column, on 16 bytes) and the columns it writes.
+__host__ __device__ inline void quad_strip_cols(int W, int nc, int k, int &c0, int &lo, int &hi) {
+    const int win = 32 * nc, out = win - 2 * kQuadHalo, pc = 2 * nc, n = quad_strips(W, nc);
     if (n == 1) {
         c0 = 0, lo = 0, hi = W;
     } else if (k == 0) {
-        c0 = 0, lo = 0, hi = kQuadWin - kQuadHalo;
+        c0 = 0, lo = 0, hi = win - kQuadHalo;
     } else if (k < n - 1) {
-        c0 = k * kQuadOut, lo = c0 + kQuadHalo, hi = c0 + kQuadWin - kQuadHalo;
+        c0 = k * out, lo = c0 + kQuadHalo, hi = c0 + win - kQuadHalo;
     } else {
-        c0 = (W + 3) / 4 * 4 - kQuadWin, lo = (n - 2) * kQuadOut + kQuadWin - kQuadHalo, hi = W;
+        c0 = (W + pc - 1) / pc * pc - win, lo = (n - 2) * out + win - kQuadHalo, hi = W;
     }
 }
 
@@ -1394,24 +1400,26 @@ __device__ __forceinline__ void cp_async_zfill(uint32_t dst, const void *src, un
 // What one quad pass needs: an image's arrays (v = u when vsel), its
 // geometry, the step's constants, the momenta of the four iterations, and
 // where the per-row sums go.
+template <class T>
 struct QuadTile {
-    const float *D, *U0, *V0, *AL;
-    float *UO0, *VO0;
+    const T *D, *U0, *V0, *AL;
+    T *UO0, *VO0;
     int64_t N;
     int H, W;
-    float wh0, wh1, tau, rad, bnd;
-    float beta[4];
+    T wh0, wh1, tau, rad, bnd;
+    T beta[4];
     double *rowpart;  // ROWSUMS: the image's per-row, per-strip slots
 };
 
 // The momenta of four iterations from the state's tn and beta, as the
 // control would set them.
-__device__ __forceinline__ void quad_betas(double tn, double beta0, float (&beta)[4]) {
-    beta[0] = (float)beta0;
+template <class T>
+__device__ __forceinline__ void quad_betas(double tn, double beta0, T (&beta)[4]) {
+    beta[0] = (T)beta0;
 #pragma unroll
     for (int l = 1; l < 4; ++l) {
         const double t2 = fista_t(tn);
-        beta[l] = (float)((tn - 1.0) / t2);
+        beta[l] = (T)((tn - 1.0) / t2);
         tn = t2;
     }
 }
@@ -1458,22 +1466,87 @@ __device__ __forceinline__ F2 sqrt2(F2 x) {
     return fma2(mul2(e, pk(0.5f, 0.5f)), y, s);
 }
 
+// A lane's columns: the operations of a step on float pairs and on one double
+// (roundings written out, so that nothing is fused that the steps do not fuse).
+template <class T>
+struct QuadOps;
+template <>
+struct QuadOps<float> {
+    using V = F2;
+    static __device__ __forceinline__ V dup(float x) { return pk(x, x); }
+    static __device__ __forceinline__ V two(float x, float y) { return pk(x, y); }
+    static __device__ __forceinline__ float first(V a) { return lo(a); }
+    static __device__ __forceinline__ float last(V a) { return hi(a); }
+    static __device__ __forceinline__ V sub(V a, V b) { return sub2(a, b); }
+    // the same in scalar operations (see zrow)
+    static __device__ __forceinline__ V sub_apart(V a, V b) {
+        return pk(__fsub_rn(lo(a), lo(b)), __fsub_rn(hi(a), hi(b)));
+    }
+    static __device__ __forceinline__ V mul(V a, V b) { return mul2(a, b); }
+    static __device__ __forceinline__ V fma(V a, V b, V c) { return fma2(a, b, c); }
+    static __device__ __forceinline__ V fms(V a, V b, V c) {  // a b - c
+        return pk(fmaf(lo(a), lo(b), -lo(c)), fmaf(hi(a), hi(b), -hi(c)));
+    }
+    static __device__ __forceinline__ V sqrt(V a) { return sqrt2(a); }
+    // each column less its left neighbour, the first's given; its right one less it, the last's given
+    static __device__ __forceinline__ V less_left(V a, float left) { return pk(lo(a) - left, hi(a) - lo(a)); }
+    static __device__ __forceinline__ V right_less(V a, float right) { return pk(hi(a) - lo(a), right - hi(a)); }
+    // the projection's scale: rp / sqrt(nn) where nn > rp^2, else 1
+    static __device__ __forceinline__ V scale(V nn, V rp) {
+        const V rr = mul2(rp, rp), pr = mul2(rp, pk(rsqrt_t(lo(nn)), rsqrt_t(hi(nn))));
+        return pk(lo(nn) > lo(rr) ? lo(pr) : 1.f, hi(nn) > hi(rr) ? hi(pr) : 1.f);
+    }
+    // gamma alpha capped at the bound, 0 where alpha is 0
+    static __device__ __forceinline__ V radius(V al, float rad, float bnd) {
+        const float r0 = rad * lo(al), r1 = rad * hi(al);
+        return pk(lo(al) == 0.f ? 0.f : (r0 <= bnd ? r0 : bnd), hi(al) == 0.f ? 0.f : (r1 <= bnd ? r1 : bnd));
+    }
+    static __device__ __forceinline__ double sum(V a, bool x, bool y) {
+        return (double)(x ? lo(a) : 0.f) + (double)(y ? hi(a) : 0.f);
+    }
+};
+template <>
+struct QuadOps<double> {
+    using V = double;
+    static __device__ __forceinline__ V dup(double x) { return x; }
+    static __device__ __forceinline__ V two(double x, double) { return x; }
+    static __device__ __forceinline__ double first(V a) { return a; }
+    static __device__ __forceinline__ double last(V a) { return a; }
+    static __device__ __forceinline__ V sub(V a, V b) { return __dsub_rn(a, b); }
+    static __device__ __forceinline__ V sub_apart(V a, V b) { return __dsub_rn(a, b); }
+    static __device__ __forceinline__ V mul(V a, V b) { return __dmul_rn(a, b); }
+    static __device__ __forceinline__ V fma(V a, V b, V c) { return __fma_rn(a, b, c); }
+    static __device__ __forceinline__ V fms(V a, V b, V c) { return __fma_rn(a, b, -c); }
+    static __device__ __forceinline__ V sqrt(V a) { return ::sqrt(a); }
+    static __device__ __forceinline__ V less_left(V a, double left) { return __dsub_rn(a, left); }
+    static __device__ __forceinline__ V right_less(V a, double right) { return __dsub_rn(right, a); }
+    static __device__ __forceinline__ V scale(V nn, V rp) {
+        return nn > __dmul_rn(rp, rp) ? __dmul_rn(rp, rsqrt_t(nn)) : 1.0;
+    }
+    static __device__ __forceinline__ V radius(V al, double rad, double bnd) {
+        const double r = __dmul_rn(rad, al);
+        return al == 0.0 ? 0.0 : (r <= bnd ? r : bnd);
+    }
+    static __device__ __forceinline__ double sum(V a, bool x, bool) { return x ? a : 0.0; }
+};
+
 // One warp's march over a strip, rows [r0, r1) out. The pass's state: per
 // level l, the input row above the one it takes next (v, u of it and z of
 // v), carried from step to step; the check's z of u on that row. Each entry
-// is a lane's two columns.
-template <int LV>
+// is a lane's columns.
+template <class V, int LV>
 struct QuadCarry {
-    F2 cv0[LV], cv1[LV], cu0[LV], cu1[LV], cz[LV];
-    F2 czu;
+    V cv0[LV], cv1[LV], cu0[LV], cu1[LV], cz[LV];
+    V czu;
     double gacc, dacc;  // the lane's gap and restart-test sums
 };
-// What a lane's two columns are, fixed over the march.
+// What a lane's columns are, fixed over the march.
+template <class V>
 struct QuadLane {
     bool outx, outy;  // written columns
     bool ledge;       // the first is the image's first: its left neighbour is the zero padding
-    F2 wr;            // the weights of their right differences (0 past the last column)
-    F2 rad;           // their radii without pixel weights (0 outside the image)
+    V wr;             // the weights of their right differences (0 past the last column)
+    V rad;            // their radii without pixel weights (0 outside the image)
 };
 
 // One step of the march, row s: iteration l + 1 (l = 0 .. LV - 1) updates row
@@ -1496,85 +1569,77 @@ struct QuadLane {
 // The arithmetic per pixel is the single step's (iso2d_lean_kernel), operation
 // for operation, with each multiply-add the single step's compiler fuses
 // written as one fused operation here.
-template <int PC, bool REDO, int G, bool EDGE, int LV, int I>
-__device__ __forceinline__ void quad_step(const QuadTile &p, const QuadLane &ln, QuadCarry<LV> &q, int s,
-                                          const float *ruv, const float *rdc, const float *rdo, const F2 *qb,
-                                          float *uo, float *vo, unsigned oo) {
+template <class T, int PB, bool REDO, int G, bool EDGE, int LV, int I>
+__device__ __forceinline__ void quad_step(const QuadTile<T> &p, const QuadLane<typename QuadOps<T>::V> &ln,
+                                          QuadCarry<typename QuadOps<T>::V, LV> &q, int s, const char *ruv,
+                                          const char *rdc, const char *rdo, const typename QuadOps<T>::V *qb, T *uo,
+                                          T *vo, unsigned oo) {
+    using O = QuadOps<T>;
+    using V = typename O::V;
     constexpr bool OUT = G < 0;
-    const F2 W0 = pk(p.wh0, p.wh0), W1 = pk(p.wh1, p.wh1), TAU = pk(p.tau, p.tau);
-    auto ld2 = [](const float *a) { return *reinterpret_cast<const F2 *>(a); };
-    const float *rs = ruv + I * 4 * kQuadWin;
-    F2 nv0 = ld2(rs), nv1 = ld2(rs + kQuadWin), nu0 = ld2(rs + 2 * kQuadWin), nu1 = ld2(rs + 3 * kQuadWin);
+    const V W0 = O::dup(p.wh0), W1 = O::dup(p.wh1), TAU = O::dup(p.tau);
+    auto ld = [](const char *a) { return *reinterpret_cast<const V *>(a); };
+    const char *rs = ruv + I * 4 * kQuadRow;
+    V nv0 = ld(rs), nv1 = ld(rs + kQuadRow), nu0 = ld(rs + 2 * kQuadRow), nu1 = ld(rs + 3 * kQuadRow);
     // z of a row pair: d + wh0 (a - above) + wh1 (b - b left)
-    auto zrow = [&](F2 d, F2 a, F2 above, F2 bb) {
-        const float sl = __shfl_up_sync(0xffffffffu, hi(bb), 1);
-        const float left = ln.ledge ? 0.f : sl;
+    auto zrow = [&](V d, V a, V above, V bb) {
+        const T sl = __shfl_up_sync(0xffffffffu, O::last(bb), 1);
+        const T left = ln.ledge ? T(0) : sl;
         // REDO: the difference in scalar operations. The row above the tile's first is
         // used nowhere else there, and the assembler would fuse the product that
         // forms it into a packed difference (one rounding less, another gap)
-        const F2 up = REDO ? pk(__fsub_rn(lo(a), lo(above)), __fsub_rn(hi(a), hi(above))) : sub2(a, above);
-        return fma2(W1, pk(lo(bb) - left, hi(bb) - lo(bb)), fma2(W0, up, d));
+        const V up = REDO ? O::sub_apart(a, above) : O::sub(a, above);
+        return O::fma(W1, O::less_left(bb, left), O::fma(W0, up, d));
     };
 #pragma unroll
     for (int l = 0; l < LV; ++l) {
         // this level's new input row s - l; the row it updates is the one above
-        const F2 dn = ld2((I - l >= 0 ? rdc + (I - l) * 2 * kQuadWin : rdo + (4 + I - l) * 2 * kQuadWin));
-        const F2 nz = zrow(dn, nv0, q.cv0[l], nv1);
+        const V dn = ld((I - l >= 0 ? rdc + (I - l) * 2 * kQuadRow : rdo + (4 + I - l) * 2 * kQuadRow));
+        const V nz = zrow(dn, nv0, q.cv0[l], nv1);
         const bool last = l == LV - 1;
-        F2 nzu = 0;
+        V nzu = 0;
         if (last) nzu = zrow(dn, nu0, q.cu0[l], nu1);  // z of the third iterate's u
-        F2 un0 = 0, un1 = 0, ov0 = 0, ov1 = 0;
+        V un0 = 0, un1 = 0, ov0 = 0, ov1 = 0;
         // above the tile, level l's updates are first needed at step 2 + 2 l
         if (OUT || 4 * G + I >= 2 + 2 * l) {
-            const F2 rp = ld2((I - l >= 1 ? rdc + (I - l - 1) * 2 * kQuadWin : rdo + (3 + I - l) * 2 * kQuadWin) +
-                              kQuadWin);
-            F2 W0N = W0;
-            if (EDGE) {
-                const float wh0n = s - l < p.H ? p.wh0 : 0.f;
-                W0N = pk(wh0n, wh0n);
-            }
+            const V rp = ld((I - l >= 1 ? rdc + (I - l - 1) * 2 * kQuadRow : rdo + (3 + I - l) * 2 * kQuadRow) +
+                            kQuadRow);
+            const V W0N = EDGE ? O::dup(s - l < p.H ? p.wh0 : T(0)) : W0;
             if (!(REDO && last)) {
-                const float zr = __shfl_down_sync(0xffffffffu, lo(q.cz[l]), 1);
-                const F2 g0 = mul2(W0N, sub2(nz, q.cz[l]));
-                const F2 g1 = mul2(ln.wr, pk(hi(q.cz[l]) - lo(q.cz[l]), zr - hi(q.cz[l])));
-                const F2 a0 = fma2(TAU, g0, q.cv0[l]);
-                const F2 a1 = fma2(TAU, g1, q.cv1[l]);
-                const F2 nn = fma2(a0, a0, mul2(a1, a1));
-                const F2 rr = mul2(rp, rp);
-                const F2 pr = mul2(rp, pk(rsqrt_t(lo(nn)), rsqrt_t(hi(nn))));
-                const F2 sc = pk(lo(nn) > lo(rr) ? lo(pr) : 1.f, hi(nn) > hi(rr) ? hi(pr) : 1.f);
-                un0 = mul2(a0, sc);
-                un1 = mul2(a1, sc);
-                const F2 B = qb[l];
-                ov0 = fma2(B, sub2(un0, q.cu0[l]), un0);
-                ov1 = fma2(B, sub2(un1, q.cu1[l]), un1);
+                const T zr = __shfl_down_sync(0xffffffffu, O::first(q.cz[l]), 1);
+                const V g0 = O::mul(W0N, O::sub(nz, q.cz[l]));
+                const V g1 = O::mul(ln.wr, O::right_less(q.cz[l], zr));
+                const V a0 = O::fma(TAU, g0, q.cv0[l]);
+                const V a1 = O::fma(TAU, g1, q.cv1[l]);
+                const V nn = O::fma(a0, a0, O::mul(a1, a1));
+                const V sc = O::scale(nn, rp);
+                un0 = O::mul(a0, sc);
+                un1 = O::mul(a1, sc);
+                const V B = qb[l];
+                ov0 = O::fma(B, O::sub(un0, q.cu0[l]), un0);
+                ov1 = O::fma(B, O::sub(un1, q.cu1[l]), un1);
             }
             if (OUT && last) {
                 // the restart test's dot (v - u_new)(u_new - u) and the gap at
                 // the third iterate u with z of it
-                const float zur = __shfl_down_sync(0xffffffffu, lo(q.czu), 1);
-                const F2 gu0 = mul2(W0N, sub2(nzu, q.czu));
-                const F2 gu1 = mul2(ln.wr, pk(hi(q.czu) - lo(q.czu), zur - hi(q.czu)));
-                const F2 gg = fma2(gu0, gu0, mul2(gu1, gu1));
-                const F2 in = fma2(gu0, q.cu0[l], mul2(gu1, q.cu1[l]));
-                const F2 sg = sqrt2(gg);
-                const float t0 = fmaf(lo(rp), lo(sg), -lo(in)), t1 = fmaf(hi(rp), hi(sg), -hi(in));
-                const double gx = (double)(ln.outx ? t0 : 0.f), gy = (double)(ln.outy ? t1 : 0.f);
-                q.gacc += gx + gy;
-                if (!REDO) {
-                    const F2 dd = fma2(sub2(q.cv0[l], un0), sub2(un0, q.cu0[l]),
-                                       mul2(sub2(q.cv1[l], un1), sub2(un1, q.cu1[l])));
-                    const double dx = (double)(ln.outx ? lo(dd) : 0.f), dy = (double)(ln.outy ? hi(dd) : 0.f);
-                    q.dacc += dx + dy;
-                }
+                const T zur = __shfl_down_sync(0xffffffffu, O::first(q.czu), 1);
+                const V gu0 = O::mul(W0N, O::sub(nzu, q.czu));
+                const V gu1 = O::mul(ln.wr, O::right_less(q.czu, zur));
+                const V gg = O::fma(gu0, gu0, O::mul(gu1, gu1));
+                const V in = O::fma(gu0, q.cu0[l], O::mul(gu1, q.cu1[l]));
+                q.gacc += O::sum(O::fms(rp, O::sqrt(gg), in), ln.outx, ln.outy);
+                if (!REDO)
+                    q.dacc += O::sum(O::fma(O::sub(q.cv0[l], un0), O::sub(un0, q.cu0[l]),
+                                            O::mul(O::sub(q.cv1[l], un1), O::sub(un1, q.cu1[l]))),
+                                     ln.outx, ln.outy);
             }
             if (OUT && last && ln.outx) {  // the pass's output row
-                auto store = [&](float *o, F2 v) {
-                    if (PC == 1) {
-                        o[0] = lo(v);
-                        if (ln.outy) o[1] = hi(v);
+                auto store = [&](T *o, V v) {
+                    if (PB == 4) {
+                        o[0] = O::first(v);
+                        if (ln.outy) o[1] = O::last(v);
                     } else {
-                        *reinterpret_cast<F2 *>(o) = v;
+                        *reinterpret_cast<V *>(o) = v;
                     }
                 };
                 const unsigned o1 = oo + (unsigned)p.N;  // N < 2^31
@@ -1610,65 +1675,65 @@ __device__ __forceinline__ void quad_step(const QuadTile &p, const QuadLane &ln,
 // the same groups in every tiling), or, REDO, each row's gap to slot row x strips +
 // strip. Else they accumulate per lane in gsum, dsum (the ragged step's per-tile
 // slot). (Summing every row in the march: 40.6 against 34.9 ms on 64 x 512^2.)
-// PC: columns per copy, 4 (rows of a multiple of 4 columns), 2 or 1: rows of any
-// width start on PC floats (3, 6 and 12 copies a row and lane). Single steps on
-// rows that are not a multiple of 4 (one column per thread) took 10.7 ms on a
-// 1531 x 1021 image, the quads take 4.2.
-template <int PC, bool ALPHA, bool REDO, bool ROWSUMS>
-__device__ __forceinline__ void quad_pass(const QuadTile &p, int strip, int r0, int r1, double &gsum,
+// PB: bytes per copy, 16 (rows of whole 16-byte pieces), 8 or 4: rows of any
+// width start on PB bytes (3, 6 and 12 copies a row and lane). Single steps on
+// float rows that are not a multiple of 4 (one column per thread) took 10.7 ms on
+// a 1531 x 1021 image, the quads take 4.2.
+template <class T, int PB, bool ALPHA, bool REDO, bool ROWSUMS>
+__device__ __forceinline__ void quad_pass(const QuadTile<T> &p, int strip, int r0, int r1, double &gsum,
                                           double &dsum) {
+    using O = QuadOps<T>;
+    using V = typename O::V;
     constexpr int LV = 4;  // iterations of the pass
-    extern __shared__ __align__(16) float quad_ring[];
+    constexpr int NC = kQuadCols<T>;
+    extern __shared__ __align__(16) char quad_ring[];
     const int H = p.H, W = p.W;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float *ring = quad_ring + warp * kQuadRingFloats;
-    float *ruv = ring;  // [uv slot][v0, v1, u0, u1][64], then [d slot][d, radius][64]
-    int C0, lo_, hi_;  // the window's first column (a multiple of 4); the columns it writes
-    quad_strip_cols(W, strip, C0, lo_, hi_);
-    const int nstrips = quad_strips(W);
-    const int wc = 2 * lane;                            // this lane's first window column
-    const int col = C0 + wc;
-    const bool inx = col < W, iny = col + 1 < W;
-    QuadLane ln;
+    char *ring = quad_ring + warp * kQuadRingBytes;  // [uv slot][v0, v1, u0, u1], then [d slot][d, radius]
+    int C0, lo_, hi_;  // the window's first column (on 16 bytes); the columns it writes
+    quad_strip_cols(W, NC, strip, C0, lo_, hi_);
+    const int nstrips = quad_strips(W, NC);
+    const int col = C0 + NC * lane;                     // this lane's first column
+    const bool inx = col < W, iny = NC > 1 && col + 1 < W;
+    QuadLane<V> ln;
     ln.outx = col >= lo_ && col < hi_;                  // lo_ is even; hi_ too, but for the last column of an odd W
-    ln.outy = ln.outx && col + 1 < hi_;
+    ln.outy = NC > 1 && ln.outx && col + 1 < hi_;
     ln.ledge = C0 == 0 && lane == 0;
-    ln.wr = pk(iny ? p.wh1 : 0.f, col + 2 < W ? p.wh1 : 0.f);
-    ln.rad = pk(inx ? p.rad : 0.f, iny ? p.rad : 0.f);
-    // the copies of a row: pieces of PC columns of v and u (both components), d
+    ln.wr = O::two(col + 1 < W ? p.wh1 : T(0), col + 2 < W ? p.wh1 : T(0));
+    ln.rad = O::two(inx ? p.rad : T(0), iny ? p.rad : T(0));
+    // the copies of a row: pieces of PB bytes of v and u (both components), d
     // and alpha; pieces outside the image are zero-filled (from a valid address).
-    // PC = 4: a piece of one component per lane; 2: a piece of each per lane; 1:
+    // PB = 16: a piece of one component per lane; 8: a piece of each per lane; 4:
     // two columns of each per lane, 32 apart, so that a copy reads 32 columns
     // side by side.
-    const int half = PC == 4 ? lane >> 4 : 0;
-    const int cl = PC == 4 ? 4 * (lane & 15) : (PC == 2 ? 2 * lane : lane);  // the window column this lane copies
+    constexpr int PE = PB / (int)sizeof(T);
+    const int half = PB == 16 ? lane >> 4 : 0;
+    const int cl = PB == 16 ? PE * (lane & 15) : PE * lane;  // the window column this lane copies
     const int cc = C0 + cl;
-    const bool okx = cc < W, oky = PC == 1 && cc + 32 < W;
+    const bool okx = cc < W, oky = PB == 4 && cc + 32 < W;
     const int ccx = okx ? cc : 0, sy = oky ? 32 : 0;
-    const uint32_t sm = (uint32_t)__cvta_generic_to_shared(ring) + (uint32_t)cl * 4u;
-    constexpr uint32_t kRow = kQuadWin * 4u, kD = kQuadSlotsUV * 4 * kRow;  // bytes of a ring row; of the uv ring
+    constexpr uint32_t kRow = kQuadRow, kD = kQuadSlotsUV * 4 * kRow;  // bytes of a ring row; of the uv ring
+    const uint32_t smv = (uint32_t)__cvta_generic_to_shared(ring) + (uint32_t)cl * (uint32_t)sizeof(T) +
+                         (PB == 16 ? half * kRow : 0u);
     const unsigned rlast = (unsigned)min(r1 + LV - 1, H - 1);  // the last row copied
     // offsets within an image's two planes fit 32 bits (N < 2^31)
-    const unsigned Nu = (unsigned)p.N, co = (unsigned)ccx + (PC == 4 && half ? Nu : 0u);
-    const float *sd = (PC == 4 && half ? p.AL : p.D) + ccx;
-    const uint32_t smv = sm + (PC == 4 ? half * kRow : 0u);
+    const unsigned Nu = (unsigned)p.N, co = (unsigned)ccx + (PB == 16 && half ? Nu : 0u);
+    const T *sd = (PB == 16 && half ? p.AL : p.D) + ccx;
     // row `row` into uv slot `slot` of the ring and the d slot at byte `ds`
     auto issue = [&](int row, int slot, uint32_t ds) {
         const bool rowin = (unsigned)row <= rlast;
         const int ro = rowin ? row * W : 0;
         const uint32_t du = smv + slot * 4 * kRow, dd = smv + kD + ds;
         const unsigned o = (unsigned)ro + co;
-        if (PC == 4) {
-            const unsigned n = rowin && okx ? 16u : 0u;
-            cp_async_zfill<16>(du, p.V0 + o, n);
-            cp_async_zfill<16>(du + 2 * kRow, p.U0 + o, n);
-            if (ALPHA || half == 0) cp_async_zfill<16>(dd, sd + ro, n);
+        const unsigned nx = rowin && okx ? PB : 0u, ny = rowin && oky ? PB : 0u;
+        if (PB == 16) {
+            cp_async_zfill<PB>(du, p.V0 + o, nx);
+            cp_async_zfill<PB>(du + 2 * kRow, p.U0 + o, nx);
+            if (ALPHA || half == 0) cp_async_zfill<PB>(dd, sd + ro, nx);
         } else {
-            constexpr int NB = PC == 2 ? 8 : 4;
-            const unsigned nx = rowin && okx ? NB : 0u, ny = rowin && oky ? NB : 0u;
-            auto both = [&](uint32_t dst, const float *src) {
-                cp_async_zfill<NB>(dst, src, nx);
-                if (PC == 1) cp_async_zfill<NB>(dst + 128, src + sy, ny);
+            auto both = [&](uint32_t dst, const T *src) {
+                cp_async_zfill<PB>(dst, src, nx);
+                if (PB == 4) cp_async_zfill<PB>(dst + 128, src + sy, ny);
             };
             both(du, p.V0 + o);
             both(du + kRow, p.V0 + (o + Nu));
@@ -1679,48 +1744,41 @@ __device__ __forceinline__ void quad_pass(const QuadTile &p, int strip, int r0, 
         }
         cp_async_commit();
     };
-    QuadCarry<LV> q;
+    QuadCarry<V, LV> q;
 #pragma unroll
     for (int l = 0; l < LV; ++l) q.cv0[l] = q.cv1[l] = q.cu0[l] = q.cu1[l] = q.cz[l] = 0;
     q.czu = 0;
     q.gacc = gsum;
     q.dacc = dsum;
-    float *uo = p.UO0 + (inx ? col : 0), *vo = p.VO0 + (inx ? col : 0);
-    // the momenta as pairs in shared memory (broadcast reads, at a fixed address;
-    // the block's warps write the same): eight registers less
-    __shared__ F2 qb[5];
+    T *uo = p.UO0 + (inx ? col : 0), *vo = p.VO0 + (inx ? col : 0);
+    // the momenta in shared memory (broadcast reads, at a fixed address; the
+    // block's warps write the same): eight registers less
+    __shared__ V qb[6];
     if (lane == 0) {
-        qb[4] = pk(p.rad, p.bnd);
+        qb[4] = O::two(p.rad, p.bnd);
+        if (NC == 1) qb[5] = O::two(p.bnd, p.bnd);
 #pragma unroll
-        for (int l = 0; l < 4; ++l) qb[l] = pk(p.beta[l], p.beta[l]);
+        for (int l = 0; l < 4; ++l) qb[l] = O::dup(p.beta[l]);
     }
     __syncwarp();
     const int sb = r0 - LV;
-    const int T = r1 - r0 + 8;
+    const int T_ = r1 - r0 + 8;
     constexpr uint32_t kHalf = 4 * 2 * kRow;  // bytes of half the d ring
     for (int k = 0; k < kQuadAhead; ++k) issue(sb + k, k, k * 2 * kRow);
     // the halves of the d ring: this group's (hc) and the last one's, in bytes
     uint32_t hc = 0;
-    const float *ruvl = ruv + wc;
+    char *rl = ring + 8 * lane;
     // stage row s (step I of its group): wait for its copies, then the radius
     // row in place (this lane's own entries): gamma alpha capped at the bound,
     // 0 where alpha is 0 or outside the image
     auto stage = [&](int s, int I) {
-        if (PC != 2) __syncwarp();  // every lane is past its reads of the slots refilled now
+        if (PB != 8) __syncwarp();  // every lane is past its reads of the slots refilled now
         issue(s + kQuadAhead, (I + kQuadAhead) & 3, I == 0 ? hc + 3 * 2 * kRow : (hc ^ kHalf) + (I - 1) * 2 * kRow);
         cp_async_wait<kQuadAhead>();
-        if (PC != 2) __syncwarp();  // row s is in, from every lane's copies
-        float *ra = const_cast<float *>(ruvl) + (kD + hc) / 4 + (I * 2 + 1) * kQuadWin;
-        F2 rp;
-        if (ALPHA) {
-            const F2 al = *reinterpret_cast<const F2 *>(ra);
-            const float rad = lo(qb[4]), bnd = hi(qb[4]);
-            const float r0f = rad * lo(al), r1f = rad * hi(al);
-            rp = pk(lo(al) == 0.f ? 0.f : (r0f <= bnd ? r0f : bnd), hi(al) == 0.f ? 0.f : (r1f <= bnd ? r1f : bnd));
-        } else {
-            rp = (unsigned)s < (unsigned)H ? ln.rad : 0;
-        }
-        *reinterpret_cast<F2 *>(ra) = rp;
+        if (PB != 8) __syncwarp();  // row s is in, from every lane's copies
+        V *ra = reinterpret_cast<V *>(rl + (kD + hc) + (I * 2 + 1) * kRow);
+        if (ALPHA) *ra = O::radius(*ra, O::first(qb[4]), NC > 1 ? O::last(qb[4]) : O::first(qb[5]));
+        else *ra = (unsigned)s < (unsigned)H ? ln.rad : V(0);
     };
     auto next_group = [&]() { hc ^= kHalf; };
     // sums of four rows (a fixed tree) into their slots: after one exchange the
@@ -1743,7 +1801,8 @@ __device__ __forceinline__ void quad_pass(const QuadTile &p, int strip, int r0, 
     // the rows above the tile
 #define FPB_QUAD_STEP(G, EDGE, I, S)                                                                            \
     stage(S, I);                                                                                                 \
-    quad_step<PC, REDO, G, EDGE, LV, I>(p, ln, q, S, ruvl, ruvl + (kD + hc) / 4, ruvl + (kD + (hc ^ kHalf)) / 4, qb, uo, vo, (unsigned)(((S) - LV) * W))
+    quad_step<T, PB, REDO, G, EDGE, LV, I>(p, ln, q, S, rl, rl + (kD + hc), rl + (kD + (hc ^ kHalf)), qb, uo, vo,   \
+                                           (unsigned)(((S) - LV) * W))
     FPB_QUAD_STEP(0, true, 0, sb);
     FPB_QUAD_STEP(0, true, 1, sb + 1);
     FPB_QUAD_STEP(0, true, 2, sb + 2);
@@ -1756,7 +1815,7 @@ __device__ __forceinline__ void quad_pass(const QuadTile &p, int strip, int r0, 
     next_group();
     int t = 8;
     // output rows, whole groups inside the image, then the rest
-    for (; t + 3 < T && sb + t + 3 < H; t += 4) {
+    for (; t + 3 < T_ && sb + t + 3 < H; t += 4) {
         const int s = sb + t;
         FPB_QUAD_STEP(-1, false, 0, s);
         row_gap(s - LV);
@@ -1769,19 +1828,19 @@ __device__ __forceinline__ void quad_pass(const QuadTile &p, int strip, int r0, 
         group_sums(s - LV);
         next_group();
     }
-    for (; t < T; t += 4) {
+    for (; t < T_; t += 4) {
         const int s = sb + t;
         FPB_QUAD_STEP(-1, true, 0, s);
         row_gap(s - LV);
-        if (t + 1 < T) {
+        if (t + 1 < T_) {
             FPB_QUAD_STEP(-1, true, 1, s + 1);
             row_gap(s - LV + 1);
         }
-        if (t + 2 < T) {
+        if (t + 2 < T_) {
             FPB_QUAD_STEP(-1, true, 2, s + 2);
             row_gap(s - LV + 2);
         }
-        if (t + 3 < T) {
+        if (t + 3 < T_) {
             FPB_QUAD_STEP(-1, true, 3, s + 3);
             row_gap(s - LV + 3);
         }
@@ -1815,8 +1874,11 @@ __device__ __forceinline__ void quad_control(const IsoState &st, const IsoImage 
 // REDO: the final iterate (the third's u) of images whose quad's check passed
 // (state redo == 3), from that quad's input buffers (fin_par, v = u when
 // redo_vsel) and momenta (redo_tn, redo_beta), into the other parity's u.
-template <int PC, bool ALPHA, bool REDO>
-__global__ void __launch_bounds__(32 * kQuadWarps, 4) iso2d_quad_kernel(StepArgs A, IsoCall c, IsoBuffers bf) {
+// Blocks resident per SM: four of float (128 registers), three of double (168;
+// at 128 it spills: 12.4 ms against 11.9 on four 384 x 320 images at 1e-8).
+template <class T, int PB, bool ALPHA, bool REDO>
+__global__ void __launch_bounds__(32 * kQuadWarps, sizeof(T) == 8 ? 3 : 4)
+iso2d_quad_kernel(StepArgs A, IsoCall c, IsoBuffers bf) {
     __shared__ double sh[64];
     __shared__ int flag;
     if (!REDO) asm volatile("griddepcontrol.wait;" ::: "memory");  // a programmatic dependent of the previous step
@@ -1838,31 +1900,31 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 4) iso2d_quad_kernel(StepArgs
     const int64_t N = A.g.N;
     const int pin = REDO ? st.fin_par : A.par, pout = pin ^ 1;
     const bool vsel = REDO ? st.redo_vsel != 0 : st.vsel != 0;
-    QuadTile p;
-    p.D = static_cast<const float *>(bf.d) + (int64_t)b * N;
-    p.U0 = static_cast<const float *>(bf.U[pin]) + (int64_t)b * 2 * N;
-    p.V0 = vsel ? p.U0 : static_cast<const float *>(bf.V[pin]) + (int64_t)b * 2 * N;
-    p.AL = ALPHA ? static_cast<const float *>(bf.alpha) + (int64_t)b * c.alpha_stride : nullptr;
-    p.UO0 = static_cast<float *>(bf.U[pout]) + (int64_t)b * 2 * N;
-    p.VO0 = static_cast<float *>(bf.V[pout]) + (int64_t)b * 2 * N;
+    QuadTile<T> p;
+    p.D = static_cast<const T *>(bf.d) + (int64_t)b * N;
+    p.U0 = static_cast<const T *>(bf.U[pin]) + (int64_t)b * 2 * N;
+    p.V0 = vsel ? p.U0 : static_cast<const T *>(bf.V[pin]) + (int64_t)b * 2 * N;
+    p.AL = ALPHA ? static_cast<const T *>(bf.alpha) + (int64_t)b * c.alpha_stride : nullptr;
+    p.UO0 = static_cast<T *>(bf.U[pout]) + (int64_t)b * 2 * N;
+    p.VO0 = static_cast<T *>(bf.V[pout]) + (int64_t)b * 2 * N;
     p.N = N;
     p.H = H;
     p.W = W;
-    p.wh0 = (float)c.wh[0];
-    p.wh1 = (float)c.wh[1];
-    p.tau = (float)c.tau;
-    p.rad = (float)im.radius;
-    p.bnd = (float)im.bound;
+    p.wh0 = (T)c.wh[0];
+    p.wh1 = (T)c.wh[1];
+    p.tau = (T)c.tau;
+    p.rad = (T)im.radius;
+    p.bnd = (T)im.bound;
     quad_betas(REDO ? st.redo_tn : st.tn, REDO ? st.redo_beta : st.beta, p.beta);
     p.rowpart = REDO && !A.row_part ? nullptr : bf.part + (int64_t)b * bf.max_part * 2;
     // the block's warps take consecutive tiles (strip, band of A.rows rows) of
     // the image, strips fastest
-    const int nstrips = quad_strips(W), nbands = (H + A.rows - 1) / A.rows;
+    const int nstrips = quad_strips(W, kQuadCols<T>), nbands = (H + A.rows - 1) / A.rows;
     const int t = (int)blockIdx.x * kQuadWarps + (int)(threadIdx.x >> 5);
     double gs = 0.0, ds = 0.0;
     if (t < nstrips * nbands) {
         const int band = t / nstrips, r0 = band * A.rows;
-        quad_pass<PC, ALPHA, REDO, true>(p, t - band * nstrips, r0, min(H, r0 + A.rows), gs, ds);
+        quad_pass<T, PB, ALPHA, REDO, true>(p, t - band * nstrips, r0, min(H, r0 + A.rows), gs, ds);
     }
     const double *part = bf.part + (int64_t)b * bf.max_part * 2;
     if (REDO) {
@@ -2058,8 +2120,8 @@ __global__ void __launch_bounds__(128, GAP2 ? 3 : 4) iso2d_ragged_pair_kernel(co
 // the block's gap and restart-test sums (each lane's over the block's rows,
 // then the block's tree) go to the item's partial slot, summed in order by
 // the image's last block.
-// PC: columns per copy (quad_pass), 4 for rows of a multiple of 4 pixels.
-template <int PC>
+// PB: bytes per copy (quad_pass), 16 for rows of a multiple of 4 pixels.
+template <int PB>
 __global__ void __launch_bounds__(32 * kQuadWarps, 4) iso2d_ragged_quad_kernel(const RagItem *__restrict__ items,
                                                                               const int *__restrict__ n_items,
                                                                               const RagSlot *__restrict__ slots,
@@ -2074,7 +2136,7 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 4) iso2d_ragged_quad_kernel(c
     if (st.status != kLive || !ragged_quad_ok(st, sl)) return;
     const IsoImage &im = bf.img[b];
     const int pin = st.fin_par, pout = pin ^ 1;
-    QuadTile p;
+    QuadTile<float> p;
     p.D = static_cast<const float *>(bf.d) + sl.off;
     p.U0 = static_cast<const float *>(bf.U[pin]) + 2 * sl.off;
     p.V0 = st.vsel ? p.U0 : static_cast<const float *>(bf.V[pin]) + 2 * sl.off;
@@ -2093,9 +2155,9 @@ __global__ void __launch_bounds__(32 * kQuadWarps, 4) iso2d_ragged_quad_kernel(c
     p.rowpart = nullptr;
     const int strip = item.cs + (int)(threadIdx.x >> 5);
     double gs = 0.0, ds = 0.0;
-    if (strip < quad_strips(sl.W)) {
+    if (strip < quad_strips(sl.W, kQuadCols<float>)) {
         const int r1 = min(sl.H, item.r0 + sl.qrows);
-        quad_pass<PC, false, false, false>(p, strip, item.r0, r1, gs, ds);
+        quad_pass<float, PB, false, false, false>(p, strip, item.r0, r1, gs, ds);
     }
     const double gsum = block_sum(gs, sh);
     const double dsum = block_sum(ds, sh);
@@ -3200,12 +3262,13 @@ void launch_3d_a(const StepShape &sh, StepArgs A, const IsoCall &c, const IsoBuf
     else launch_3d_v<T, ALPHA, false, false>(grid, A, c, bf, s);
 }
 
-// f(PC) for the columns per copy that rows of W columns allow.
-template <class F>
+// f(PB) for the bytes per copy that rows of W columns allow.
+template <class T, class F>
 void quad_kernels(int W, const F &f) {
-    if (W % 4 == 0) f(std::integral_constant<int, 4>{});
-    else if (W % 2 == 0) f(std::integral_constant<int, 2>{});
-    else f(std::integral_constant<int, 1>{});
+    const int b = W * (int)sizeof(T) % 16;
+    if (b == 0) f(std::integral_constant<int, 16>{});
+    else if (b == 8) f(std::integral_constant<int, 8>{});
+    else if constexpr (sizeof(T) == 4) f(std::integral_constant<int, 4>{});
 }
 
 // The quad launch: blocks of kQuadWarps tiles (a strip by `rows` rows). A
@@ -3215,6 +3278,7 @@ void quad_kernels(int W, const F &f) {
 // 512^2 (three waves of 56 steps, against five of 40 at 32 rows), 8 for one
 // image (a single wave of short tiles). Small launches take 4 rows (64^2: 0.58 ms
 // a solve against 0.64 at 8).
+template <class T>
 int quad_rows(const Geometry &g, int64_t nimg) {
     static const int rows_hint = [] {  // tuning hint FASTPROX_B200_QUAD_ROWS
         const char *v = std::getenv("FASTPROX_B200_QUAD_ROWS");
@@ -3224,13 +3288,13 @@ int quad_rows(const Geometry &g, int64_t nimg) {
     static const int64_t slots = [] {  // resident quad blocks on the device
         int dev = 0, sms = 148, per = 4;
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, iso2d_quad_kernel<4, true, false>, 32 * kQuadWarps,
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, iso2d_quad_kernel<T, 16, true, false>, 32 * kQuadWarps,
                                                           kQuadSmem) != cudaSuccess || per < 1)
             per = 4;
         cudaGetLastError();
         return (int64_t)sms * per;
     }();
-    const int64_t H = g.L[0], ns = quad_strips((int)g.L[1]);
+    const int64_t H = g.L[0], ns = quad_strips((int)g.L[1], kQuadCols<T>);
     auto blocks = [&](int rows) { return (ns * ((H + rows - 1) / rows) + kQuadWarps - 1) / kQuadWarps; };
     int rows = rows_hint;
     if (!rows) {
@@ -3246,18 +3310,38 @@ int quad_rows(const Geometry &g, int64_t nimg) {
     }
     return rows;
 }
+template <class T>
 dim3 quad_grid(const Geometry &g, int rows, int64_t nimg) {
-    const int64_t tiles = quad_strips((int)g.L[1]) * ((g.L[0] + rows - 1) / rows);
+    const int64_t tiles = quad_strips((int)g.L[1], kQuadCols<T>) * ((g.L[0] + rows - 1) / rows);
     return dim3((unsigned)((tiles + kQuadWarps - 1) / kQuadWarps), 1, (unsigned)nimg);
 }
 
+template <class T>
 void launch_quad(StepArgs A, const IsoCall &c, const IsoBuffers &bf, cudaStream_t s) {
-    A.rows = quad_rows(A.g, A.nimg);
-    const dim3 grid = quad_grid(A.g, A.rows, A.nimg);
-    quad_kernels((int)A.g.L[1], [&](auto pc) {
-        constexpr int PC = decltype(pc)::value;
-        if (c.has_alpha) launch_step(iso2d_quad_kernel<PC, true, false>, grid, 32 * kQuadWarps, kQuadSmem, s, A, c, bf);
-        else launch_step(iso2d_quad_kernel<PC, false, false>, grid, 32 * kQuadWarps, kQuadSmem, s, A, c, bf);
+    A.rows = quad_rows<T>(A.g, A.nimg);
+    const dim3 grid = quad_grid<T>(A.g, A.rows, A.nimg);
+    quad_kernels<T>((int)A.g.L[1], [&](auto pb) {
+        constexpr int PB = decltype(pb)::value;
+        if (c.has_alpha) launch_step(iso2d_quad_kernel<T, PB, true, false>, grid, 32 * kQuadWarps, kQuadSmem, s, A, c, bf);
+        else launch_step(iso2d_quad_kernel<T, PB, false, false>, grid, 32 * kQuadWarps, kQuadSmem, s, A, c, bf);
+    });
+}
+
+// The quad's redo: three iterations over whole images.
+template <class T>
+void quad_redo(const Geometry &g, const IsoCall &c, const IsoBuffers &bf, bool gaps, cudaStream_t s) {
+    StepArgs A;
+    A.g = g;
+    A.max_iter = c.max_iter;
+    A.par = 0;
+    A.rows = quad_rows<T>(g, g.B);
+    A.nimg = g.B;
+    A.row_part = gaps && iso_quad_parts(sizeof(T) == 4 ? 1 : 2, g) <= bf.max_part ? 1 : 0;
+    const dim3 grid = quad_grid<T>(g, A.rows, g.B);
+    quad_kernels<T>((int)g.L[1], [&](auto pb) {
+        constexpr int PB = decltype(pb)::value;
+        if (c.has_alpha) iso2d_quad_kernel<T, PB, true, true><<<grid, 32 * kQuadWarps, kQuadSmem, s>>>(A, c, bf);
+        else iso2d_quad_kernel<T, PB, false, true><<<grid, 32 * kQuadWarps, kQuadSmem, s>>>(A, c, bf);
     });
 }
 
@@ -3295,11 +3379,8 @@ cudaError_t step_t(const Geometry &g, const IsoCall &c, const IsoBuffers &bf, co
         return cudaGetLastError();
     }
     if (variant == kVariantQuad) {
-        if constexpr (std::is_same<T, float>::value) {
-            launch_quad(A, c, bf, s);
-            return cudaGetLastError();
-        }
-        return cudaErrorInvalidValue;
+        launch_quad<T>(A, c, bf, s);
+        return cudaGetLastError();
     }
     if (variant == kVariantPair || variant == kVariantPairGap) {
         launch_pair<T>(sh, A, c, bf, s, variant == kVariantPairGap);
@@ -3399,12 +3480,12 @@ bool iso_ragged_pairs(int dtype, int vec) {
 cudaError_t iso_ragged_quad_step(bool odd, const RagItem *items, const int *n_items, int grid, const RagSlot *slots,
                                  const IsoBuffers &bf, cudaStream_t s) {
     if (grid <= 0) return cudaSuccess;
-    if (odd) iso2d_ragged_quad_kernel<1><<<grid, 32 * kQuadWarps, kQuadSmem, s>>>(items, n_items, slots, bf);
-    else iso2d_ragged_quad_kernel<4><<<grid, 32 * kQuadWarps, kQuadSmem, s>>>(items, n_items, slots, bf);
+    if (odd) iso2d_ragged_quad_kernel<4><<<grid, 32 * kQuadWarps, kQuadSmem, s>>>(items, n_items, slots, bf);
+    else iso2d_ragged_quad_kernel<16><<<grid, 32 * kQuadWarps, kQuadSmem, s>>>(items, n_items, slots, bf);
     return cudaGetLastError();
 }
 
-int iso_quad_strips(int W) { return quad_strips(W); }
+int iso_quad_strips(int W) { return quad_strips(W, kQuadCols<float>); }
 int iso_quad_warps() { return kQuadWarps; }
 
 int iso_setup_blocks(const Geometry &g) {
@@ -3508,32 +3589,21 @@ bool iso_quad_ok(int dtype, const Geometry &g, int max_part) {
         return !(v && v[0] == '0' && v[1] == 0);
     }();
     // rows narrower than 32 pixels keep the generic step (its gap terms in FP64)
-    return on && pairs_enabled() && dtype == 1 && g.k == 2 && g.L[1] >= 32 && g.L[0] >= 2 &&
-           g.L[0] * g.L[1] < (int64_t(1) << 31) && iso_quad_parts(g) <= max_part;
+    return on && pairs_enabled() && g.k == 2 && g.L[1] >= 32 && g.L[0] >= 2 &&
+           g.L[0] * g.L[1] < (int64_t(1) << 31) && iso_quad_parts(dtype, g) <= max_part;
 }
 
-int64_t iso_quad_parts(const Geometry &g) {
-    return g.k == 2 ? g.L[0] * (int64_t)quad_strips((int)std::min<int64_t>(g.L[1], 1 << 30)) : 0;
+int64_t iso_quad_parts(int dtype, const Geometry &g) {
+    const int W = (int)std::min<int64_t>(g.L[1], 1 << 30);
+    return g.k == 2 ? g.L[0] * (int64_t)quad_strips(W, dtype == 1 ? kQuadCols<float> : kQuadCols<double>) : 0;
 }
 
 cudaError_t iso_redo(int dtype, const Geometry &g, const IsoCall &c, const IsoBuffers &bf, cudaStream_t s,
                      bool quads, bool gaps) {
     if (g.k != 2 || g.B <= 0 || g.N <= 0) return cudaSuccess;
-    if (quads && dtype == 1) {
-        // the quad's redo: three iterations over whole images
-        StepArgs A;
-        A.g = g;
-        A.max_iter = c.max_iter;
-        A.par = 0;
-        A.rows = quad_rows(g, g.B);
-        A.nimg = g.B;
-        A.row_part = gaps && iso_quad_parts(g) <= bf.max_part ? 1 : 0;
-        const dim3 grid = quad_grid(g, A.rows, g.B);
-        quad_kernels((int)g.L[1], [&](auto pc) {
-            constexpr int PC = decltype(pc)::value;
-            if (c.has_alpha) iso2d_quad_kernel<PC, true, true><<<grid, 32 * kQuadWarps, kQuadSmem, s>>>(A, c, bf);
-            else iso2d_quad_kernel<PC, false, true><<<grid, 32 * kQuadWarps, kQuadSmem, s>>>(A, c, bf);
-        });
+    if (quads) {
+        if (dtype == 1) quad_redo<float>(g, c, bf, gaps, s);
+        else quad_redo<double>(g, c, bf, gaps, s);
     }
     const dim3 grid((unsigned)std::min<int64_t>((g.N + 255) / 256, 1024), (unsigned)g.B);
     if (dtype == 1) {
