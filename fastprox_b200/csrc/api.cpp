@@ -559,6 +559,8 @@ fp_status fpb_workspace_build(const fp_op *op, const Arr &x, const fp_options &o
         ws->max_part = (int)std::max<int64_t>(ws->max_part, (int64_t)ws->shape_.gx * g.L[0]);
     if (g.k == 2 && !op->huber)  // per-row, per-strip partial sums of the quad launch
         ws->max_part = (int)std::max<int64_t>(ws->max_part, iso_quad_parts(x.dtype, g));
+    if (ws->shape_.kind == 5)  // per-block partial sums of the 3D pair launch
+        ws->max_part = (int)std::max<int64_t>(ws->max_part, iso_pair3d_parts(x.dtype, g));
     if (op->kind == kAniso && !op->huber) {
         // the untiled fibre passes: a block of 128 fibres per partial, three
         // axes in one launch for FDPG-3
@@ -975,11 +977,19 @@ fp_status run_iso(fp_workspace *ws, const fp_op *op, const void *xsrc, void *zds
     // count was read holds every image still live): the tail of a batch, where
     // a few slow images remain, launches only their blocks.
     // Iterations 1 and 2 mod 4 (no check in either), and 3 and 4 mod 4 (the
-    // second with the check) run as one launch each where the lean 2D step
-    // applies (iso_pair_ok).
+    // second with the check) run as one launch each where iso_pair_ok (the lean
+    // 2D step, float32 volumes).
     const int chunk = ws->chunk > 0 ? ws->chunk : 8;
-    const bool pairs = iso_pair_ok(g, ws->shape_, ws->max_part);
+    const bool pairs = !c.huber && iso_pair_ok(ws->dtype, g, ws->shape_, ws->max_part);
     const bool quads = !c.huber && iso_quad_ok(ws->dtype, g, ws->max_part);
+    // Float64 and 3D take their first eight iterations in single steps: a solve
+    // that stops in a quad or pair forms its final iterate again, another pass,
+    // which float64 quads (0.5-0.7 of four steps on 0.5 M pixels) and 3D pairs
+    // (0.76) earn back in two or three launches only. Noise at small steps stops
+    // after 4 or 8 iterations: 610 x 1087 float64 took 440 us against 367.
+    // They are one chunk, so such a solve is known to need no redo.
+    const int first = (pairs || quads) && (ws->dtype == FP_F64 || g.k == 3) ? 9 : 1;
+    bool fused = false, fused_by[2] = {false, false};  // quads or pairs launched, by the end of a slot's chunk
     int par = 0, slot = 0, inflight = 0;
     int64_t launched = 0, steps = 0, lists = 0, nimg = g.B;
     const int64_t cap = (int64_t)max_iter + 1 + 2 * chunk;
@@ -992,9 +1002,10 @@ fp_status run_iso(fp_workspace *ws, const fp_op *op, const void *xsrc, void *zds
     }
     bool done = false;
     while (!done) {
-        for (int j = 0; j < chunk; ++j) {
-            int pv = quads ? iso_quad_at(launched, max_iter) : -1;
-            if (pv < 0 && pairs) pv = iso_pair_at(launched, max_iter);
+        const int n = launched == 0 ? std::max(chunk, first) : chunk;
+        for (int j = 0; j < n; ++j) {
+            int pv = quads && launched >= first ? iso_quad_at(launched, max_iter) : -1;
+            if (pv < 0 && pairs && launched >= first) pv = iso_pair_at(launched, max_iter);
             const bool timed = ws->time_steps && tkind.size() < kTimed;
             if (timed) {
                 while (ws->tev.size() < 2 * (tkind.size() + 1)) {
@@ -1011,6 +1022,7 @@ fp_status run_iso(fp_workspace *ws, const fp_op *op, const void *xsrc, void *zds
                 if ((e = cudaEventRecord(ws->tev[2 * tkind.size() + 1], s)) != cudaSuccess) return cuda_status(e);
                 tkind.push_back(pv == kVariantQuad ? 3 : pv == kVariantPairGap ? 2 : (pv == kVariantPair ? 1 : 0));
             }
+            fused = fused || pv >= 0;
             par ^= 1;
             launched += pv == kVariantQuad ? 4 : pv >= 0 ? 2 : 1;
             ++steps;
@@ -1018,6 +1030,7 @@ fp_status run_iso(fp_workspace *ws, const fp_op *op, const void *xsrc, void *zds
         e = cudaMemcpyAsync(ws->h_live + slot, ws->live, sizeof(int), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaEventRecord(ws->ev[slot], s);
         if (e != cudaSuccess) return cuda_status(e);
+        fused_by[slot] = fused;
         slot ^= 1;
         ++inflight;
         if (inflight == 2) {
@@ -1027,6 +1040,7 @@ fp_status run_iso(fp_workspace *ws, const fp_op *op, const void *xsrc, void *zds
             const int live = ws->h_live[slot];
             if (live == 0) {
                 done = true;
+                fused = fused_by[slot];
             } else if (live < nimg) {
                 e = iso_live_list(ws->st, g.B, ws->lmap, ws->lcnt, s);
                 if (e != cudaSuccess) return cuda_status(e);
@@ -1050,7 +1064,7 @@ fp_status run_iso(fp_workspace *ws, const fp_op *op, const void *xsrc, void *zds
             ws->tcount[tkind[k]] += 1;
         }
     }
-    if (pairs || quads) {
+    if (fused) {
         e = iso_redo(ws->dtype, g, c, bf, s, quads, true);
         ws->kernel_launches += quads ? 3 : 2;
     }

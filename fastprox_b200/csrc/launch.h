@@ -63,7 +63,8 @@ cudaError_t iso_step(int dtype, const Geometry &g, const IsoCall &c, const IsoBu
 // it passes, the final u is the first iterate, formed again by iso_redo).
 constexpr int kVariantPair = 3;
 constexpr int kVariantPairGap = 4;
-bool iso_pair_ok(const Geometry &g, const StepShape &sh, int max_part);
+// 3D float32 volumes have pairs of their own.
+bool iso_pair_ok(int dtype, const Geometry &g, const StepShape &sh, int max_part);
 inline int iso_pair_at(int64_t k, int max_iter) {
     if (k <= 0 || k + 1 >= max_iter) return -1;
     if ((k & 3) == 1) return kVariantPair;
@@ -83,6 +84,8 @@ constexpr int kVariantQuad = 5;
 bool iso_quad_ok(int dtype, const Geometry &g, int max_part);
 // Partial-sum slots per image the quad needs (one per row and warp strip).
 int64_t iso_quad_parts(int dtype, const Geometry &g);
+// Partial-sum slots per volume the 3D pair needs (one per block).
+int64_t iso_pair3d_parts(int dtype, const Geometry &g);
 inline int iso_quad_at(int64_t k, int max_iter) {
     return (k > 0 && (k & 3) == 1 && k + 3 < max_iter) ? kVariantQuad : -1;
 }

@@ -2948,6 +2948,358 @@ __global__ void __launch_bounds__(k3VX / 2 * k3VY, 4) iso3d_v2_kernel(StepArgs A
 }
 
 // ---------------------------------------------------------------------------
+// Two 3D iterations in one pass (float32; the launches a 2D pair makes:
+// kVariantPair, kVariantPairGap). A single 3D step moves 52 bytes a voxel (d, v
+// and u in, v and u out) and is bound by that; here they move once for two
+// iterations. A block owns a window of 32 columns (axis 2) by 2 k3PW rows (axis
+// 1) and marches along axis 0; a lane holds one column and two adjacent rows, the
+// rows a packed pair (f32x2), so the window is nearly square and its halo (2
+// columns on each side, 1 row above and 2 below, none on the volume's edges)
+// costs least: 35 % more voxels than are written on a plane of 128 x 128, against
+// 75 to 95 % with windows of 64 or 128 columns of as many voxels. Everything but
+// the outermost rows of a warp's neighbours stays in registers: rows of z and v
+// cross between warps through shared memory one slice later than they are formed
+// (the second iteration runs two slices behind the first), so a slice takes one
+// barrier. The entries of slice s + 3 are copied (cp.async) while slice s is
+// worked on. Step s, of the first iteration: z(s), then u', v' of slice
+// s - 1; of the second: z'(s - 2) of v', then u'', v'' of slice s - 3, and for the
+// check the gap at u' and the restart test's dot there. Arithmetic per voxel as
+// the single steps', every fused operation written out.
+// What bounds it: 16 warps per SM (128 registers) issue in 49 % of the cycles (272
+// instructions per warp and step, two dependent iterations, a barrier), with 54 B of
+// DRAM traffic a voxel per two iterations at 3.6 TB/s. Four iterations of 8 x 128^3:
+// 730 us in single steps (three of 166, one of 230), 554 in two pairs; 5 volumes
+// live: 473 and 365; 2: 223 and 182. A solve of 8 to 1e-5: 110.9 -> 86.4 ms.
+// ---------------------------------------------------------------------------
+constexpr int k3PW = 8;               // warps per block
+constexpr int k3PRows = 2 * k3PW;     // window rows
+constexpr int k3PLeft = 2, k3PRight = 2, k3PTop = 1, k3PBot = 2;  // halos
+constexpr int k3PAhead = 3;           // slices in flight beyond the one being read
+constexpr int k3PSlots = 4;           // ring slots per warp (k3PAhead + 1)
+template <bool ALPHA>
+constexpr int k3PSlot = (ALPHA ? 17 : 15) * 128;  // bytes of a warp's ring slot: rows of 32 floats, v0 (first row,
+                                                  // second), v1, v2, u0, u1, u2, d, v1 of the row above, alpha
+template <bool ALPHA>
+constexpr size_t k3PSmem = (size_t)k3PW * k3PSlots * k3PSlot<ALPHA>;
+
+// Windows of w entries over an extent of n with halos a before and b after.
+__host__ __device__ inline int win_count(int n, int w, int a, int b) {
+    if (n <= w) return 1;
+    const int out = w - a - b, rest = n - (w - a) - (w - b);
+    return 2 + (rest > 0 ? (rest + out - 1) / out : 0);
+}
+// Window k's first entry and the entries it writes.
+__device__ inline void win_range(int n, int w, int a, int b, int k, int &c0, int &lo, int &hi) {
+    const int out = w - a - b, cnt = win_count(n, w, a, b);
+    if (cnt == 1) {
+        c0 = 0, lo = 0, hi = n;
+    } else if (k == 0) {
+        c0 = 0, lo = 0, hi = w - b;
+    } else if (k < cnt - 1) {
+        c0 = k * out, lo = c0 + a, hi = c0 + w - b;
+    } else {
+        c0 = n - w, lo = (cnt - 1) * out + a, hi = n;
+    }
+}
+
+template <bool ALPHA, bool GAP, bool V16>
+__global__ void __launch_bounds__(32 * k3PW, 2) iso3d_pair_kernel(StepArgs A, IsoCall c, IsoBuffers bf) {
+    using O = QuadOps<float>;
+    extern __shared__ __align__(16) char i3p_ring[];
+    // rows exchanged between warps, by the parity of the step: the first row of z
+    // (first iteration; row w, read by warp w - 1), the last row of v1' (row w + 1,
+    // read by warp w + 1), the first row of z'; for the check the same of u1', z of u'
+    __shared__ float xz0[2][k3PW + 1][32], xv1[2][k3PW + 1][32], xz1[2][k3PW + 1][32];
+    __shared__ float xu1[GAP ? 2 : 1][k3PW + 1][32], xzu[GAP ? 2 : 1][k3PW + 1][32];
+    __shared__ F2 qb[2];
+    __shared__ double sh[64];
+    __shared__ int flag;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // a programmatic dependent of the previous step
+    const int b = step_image(bf, blockIdx.z);
+    if (b < 0) return;
+    const IsoState st = bf.st[b];
+    if (st.status != kLive) return;
+    const int it = st.it;
+    if (it <= 0 || (it & 3) != (GAP ? 3 : 1) || it + 1 >= A.max_iter || st.zero_in) {
+        if (threadIdx.x == 0) atomicExch(bf.err, 3);
+        return;
+    }
+    const IsoImage im = bf.img[b];
+    const int D0 = (int)A.g.L[0], D1 = (int)A.g.L[1], D2 = (int)A.g.L[2];
+    const int64_t N = A.g.N;
+    const int S0 = D1 * D2;
+    const int pin = A.par, pout = A.par ^ 1;
+    const float *D = static_cast<const float *>(bf.d) + (int64_t)b * N;
+    const float *U = static_cast<const float *>(bf.U[pin]) + (int64_t)b * 3 * N;
+    const float *V = st.vsel ? U : static_cast<const float *>(bf.V[pin]) + (int64_t)b * 3 * N;
+    float *UO = static_cast<float *>(bf.U[pout]) + (int64_t)b * 3 * N;
+    float *VO = static_cast<float *>(bf.V[pout]) + (int64_t)b * 3 * N;
+    const float *AL = ALPHA ? static_cast<const float *>(bf.alpha) + (int64_t)b * c.alpha_stride : D;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int nx = win_count(D2, 32, k3PLeft, k3PRight), ny = win_count(D1, k3PRows, k3PTop, k3PBot);
+    int X0, xlo, xhi, Y0, ylo, yhi;
+    const int tile = (int)blockIdx.x, chunk = tile / (nx * ny), txy = tile - chunk * (nx * ny);
+    win_range(D2, 32, k3PLeft, k3PRight, txy % nx, X0, xlo, xhi);
+    win_range(D1, k3PRows, k3PTop, k3PBot, txy / nx, Y0, ylo, yhi);
+    const int r0 = chunk * A.rows, r1 = min(D0, r0 + A.rows);
+    const int x = X0 + lane, y = Y0 + 2 * w;  // this lane's column and first row
+    const bool inx = x < D2, ina = inx && y < D1, inb = inx && y + 1 < D1, inr = inx && y > 0 && y - 1 < D1;
+    const bool outx = x >= xlo && x < xhi, outa = outx && y >= ylo && y < yhi, outb = outx && y + 1 >= ylo && y + 1 < yhi;
+    const bool ledge = x == 0;
+    const float wh0 = (float)c.wh[0];
+    const F2 W0 = O::dup(wh0), W1 = O::dup((float)c.wh[1]), W2 = O::dup((float)c.wh[2]);
+    const F2 wf1 = pk(y + 1 < D1 ? (float)c.wh[1] : 0.f, y + 2 < D1 ? (float)c.wh[1] : 0.f);  // forward, zero at the edge
+    const float wf2 = x + 1 < D2 ? (float)c.wh[2] : 0.f;
+    const F2 TAU = O::dup((float)c.tau);
+    const float rad = (float)im.radius, bnd = (float)im.bound;
+    const F2 radin = pk(ina ? rad : 0.f, inb ? rad : 0.f);
+    if (threadIdx.x < 32) {
+        if (threadIdx.x == 0) {
+            qb[0] = O::dup((float)st.beta);
+            qb[1] = O::dup((float)((st.tn - 1.0) / fista_t(st.tn)));
+        }
+        for (int q = 0; q < 2; ++q) {  // the rows beyond the window
+            xz0[q][k3PW][lane] = xv1[q][0][lane] = xz1[q][k3PW][lane] = 0.f;
+            if (GAP) xu1[GAP ? q : 0][0][lane] = xzu[GAP ? q : 0][k3PW][lane] = 0.f;
+        }
+    }
+    for (int q = 0; q < 2; ++q) {  // what the first step reads
+        xz0[q][w][lane] = xv1[q][w + 1][lane] = xz1[q][w][lane] = 0.f;
+        if (GAP) xu1[GAP ? q : 0][w + 1][lane] = xzu[GAP ? q : 0][w][lane] = 0.f;
+    }
+    // copies of slice sl into ring slot `slot` (zeros outside the volume). Rows of a
+    // multiple of 4 columns (V16): 16-byte pieces, eight lanes a row, four rows a
+    // copy (4 copies a lane and slice instead of 15; 272 instructions a step against
+    // 298). Offsets fit 32 bits (4 N < 2^32) on bases the block shares.
+    char *ring = i3p_ring + (size_t)w * k3PSlots * k3PSlot<ALPHA>;
+    const uint32_t rs = (uint32_t)__cvta_generic_to_shared(ring) + (V16 ? 16u : 4u) * (uint32_t)lane;
+    const unsigned oa = ina ? 4u * (unsigned)(y * D2 + x) : 0u, sbytes = 4u * (unsigned)S0;
+    constexpr int NC = V16 ? (ALPHA ? 5 : 4) : (ALPHA ? 17 : 15);
+    const char *src[V16 ? NC : 1];
+    unsigned okm = 0;
+    if (V16) {
+        const int q = lane >> 3, px = X0 + 4 * (lane & 7);
+#pragma unroll
+        for (int e = 0; e < NC; ++e) {
+            const int r = 4 * e + q;  // the row of the slot
+            const float *base = r < 6 ? V + (r >> 1) * N : r < 12 ? U + ((r >> 1) - 3) * N : r < 14 ? D : r == 14 ? V + N : AL;
+            const int py = r == 14 ? y - 1 : r < 14 ? y + (r & 1) : y + (r - 15);
+            const bool ok = r < (ALPHA ? 17 : 15) && px < D2 && py >= 0 && py < D1;
+            src[V16 ? e : 0] = reinterpret_cast<const char *>(base + (ok ? py * D2 + px : 0));
+            okm |= (ok ? 1u : 0u) << e;
+        }
+    } else {
+        okm = (ina ? 1u : 0u) | (inb ? 2u : 0u) | (inr ? 4u : 0u);
+    }
+    auto issue = [&](int sl, int slot) {
+        const bool in = (unsigned)sl < (unsigned)D0 && sl <= r1 + 1;  // the last slice any output reads
+        const unsigned so = in ? (unsigned)sl * sbytes : 0u;
+        const uint32_t d = rs + (uint32_t)slot * k3PSlot<ALPHA>;
+        if (V16) {
+#pragma unroll
+            for (int e = 0; e < NC; ++e)
+                if (e < 3 || e * 4 + 3 < (ALPHA ? 17 : 15) || lane < 8 * ((ALPHA ? 17 : 15) - 4 * e))
+                    cp_async_zfill<16>(d + e * 512, src[V16 ? e : 0] + so, in && (okm >> e & 1) ? 16u : 0u);
+        } else {
+            const unsigned n[3] = {in && ina ? 4u : 0u, in && inb ? 4u : 0u, in && inr ? 4u : 0u};
+#pragma unroll
+            for (int r = 0; r < NC; ++r) {
+                const int k = r == 14 ? 2 : r < 14 ? r & 1 : r - 15;  // first row, second, the row above
+                const float *base = r < 6 ? V + (r >> 1) * N : r < 12 ? U + ((r >> 1) - 3) * N : r < 14 ? D : r == 14 ? V + N : AL;
+                const unsigned o = n[k] ? so + oa + (k == 1 ? 4u * (unsigned)D2 : 0u) - (k == 2 && ina ? 4u * (unsigned)D2 : 0u)
+                                        : 0u;
+                const unsigned o2 = (k == 2 && n[2] && !ina) ? so + 4u * (unsigned)((y - 1) * D2 + x) : o;
+                cp_async_zfill<4>(d + r * 128, reinterpret_cast<const char *>(base) + o2, n[k]);
+            }
+        }
+        cp_async_commit();
+    };
+    // z = d + w0 (a0 - a0 of the slice before) + w1 (a1 - a1 of the row above) +
+    // w2 (a2 - a2 of the column to the left)
+    auto zrow = [&](F2 d, F2 a0, F2 p0, F2 a1, float above, F2 a2) {
+        const float la = __shfl_up_sync(0xffffffffu, lo(a2), 1), lb = __shfl_up_sync(0xffffffffu, hi(a2), 1);
+        const F2 left = pk(ledge ? 0.f : la, ledge ? 0.f : lb);
+        const F2 z = fma2(W0, sub2(a0, p0), d);
+        return fma2(W2, sub2(a2, left), fma2(W1, pk(lo(a1) - above, hi(a1) - lo(a1)), z));
+    };
+    // the forward differences of z (next: the slice after, below: the row after)
+    auto grad = [&](F2 z, F2 next, float below, bool fwd, F2 &g0, F2 &g1, F2 &g2) {
+        const float ra = __shfl_down_sync(0xffffffffu, lo(z), 1), rb = __shfl_down_sync(0xffffffffu, hi(z), 1);
+        g0 = mul2(O::dup(fwd ? wh0 : 0.f), sub2(next, z));
+        g1 = mul2(wf1, pk(hi(z) - lo(z), below - hi(z)));
+        g2 = mul2(O::dup(wf2), sub2(pk(ra, rb), z));
+    };
+    F2 cv[3] = {0, 0, 0}, cu[3] = {0, 0, 0}, cz = 0;        // slice s - 1: v, u and z(v)
+    F2 hv[3][3] = {}, hu[3][3] = {}, hd[3] = {}, hr[3] = {};  // v', u', d and the radii by slice mod 3
+    F2 z1c = 0, zuc = 0;                                    // slice s - 3: z'(v'), z of u'
+    double gap_acc = 0.0, dot_acc = 0.0;
+    const int sb = r0 - 2, nsteps = r1 - r0 + 5;
+    for (int k = 0; k < k3PAhead; ++k) issue(sb + k, k);
+    __syncthreads();
+    auto step = [&](auto ic, int t) {
+        constexpr int I = decltype(ic)::value, I1 = (I + 2) % 3, I2 = (I + 1) % 3;  // slices s, s - 3; s - 1; s - 2
+        const int s = sb + t, pr = t & 1, pw = pr ^ 1;  // exchange rows: written pr, read pw
+        cp_async_wait<k3PAhead - 1>();
+        __syncthreads();  // the rows that the last step wrote
+        issue(s + k3PAhead, (t + k3PAhead) & (k3PSlots - 1));
+        const char *rl = ring + (size_t)(t & (k3PSlots - 1)) * k3PSlot<ALPHA>;
+        auto row = [&](int r) { return *reinterpret_cast<const float *>(rl + r * 128 + 4 * lane); };
+        auto ld = [&](int a) { return pk(row(2 * a), row(2 * a + 1)); };
+        const F2 nv0 = ld(0), nv1 = ld(1), nv2 = ld(2), nd = ld(6);
+        // first iteration, z of slice s
+        const F2 nz = zrow(nd, nv0, cv[0], nv1, row(14), nv2);
+        xz0[pr][w][lane] = lo(nz);
+        hd[I] = nd;
+        // its update of slice s - 1
+        {
+            F2 g0, g1, g2;
+            grad(cz, nz, xz0[pw][w + 1][lane], s < D0, g0, g1, g2);
+            const F2 a0 = fma2(TAU, g0, cv[0]), a1 = fma2(TAU, g1, cv[1]), a2 = fma2(TAU, g2, cv[2]);
+            const F2 nn = fma2(a2, a2, fma2(a0, a0, mul2(a1, a1)));
+            const F2 rp = ALPHA ? hr[I1] : ((unsigned)(s - 1) < (unsigned)D0 ? radin : F2(0));
+            const F2 sc = O::scale(nn, rp);
+            const F2 B = qb[0];
+            hu[I1][0] = mul2(a0, sc);
+            hu[I1][1] = mul2(a1, sc);
+            hu[I1][2] = mul2(a2, sc);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) hv[I1][a] = fma2(B, sub2(hu[I1][a], cu[a]), hu[I1][a]);
+        }
+        // second iteration, z' of slice s - 2 (and z of u' there)
+        const F2 z1 = zrow(hd[I2], hv[I2][0], hv[I][0], hv[I2][1], xv1[pw][w][lane], hv[I2][2]);
+        F2 zu = 0;
+        if (GAP) zu = zrow(hd[I2], hu[I2][0], hu[I][0], hu[I2][1], xu1[GAP ? pw : 0][w][lane], hu[I2][2]);
+        xv1[pr][w + 1][lane] = hi(hv[I1][1]);
+        xz1[pr][w][lane] = lo(z1);
+        if (GAP) {
+            xu1[GAP ? pr : 0][w + 1][lane] = hi(hu[I1][1]);
+            xzu[GAP ? pr : 0][w][lane] = lo(zu);
+        }
+        // its update of slice s - 3
+        const int so = s - 3;
+        if (so >= r0) {
+            F2 g0, g1, g2;
+            grad(z1c, z1, xz1[pw][w + 1][lane], so + 1 < D0, g0, g1, g2);
+            const F2 a0 = fma2(TAU, g0, hv[I][0]), a1 = fma2(TAU, g1, hv[I][1]), a2 = fma2(TAU, g2, hv[I][2]);
+            const F2 nn = fma2(a2, a2, fma2(a0, a0, mul2(a1, a1)));
+            const F2 rp = ALPHA ? hr[I] : radin;
+            const F2 sc = O::scale(nn, rp);
+            const F2 B = qb[1];
+            const F2 un[3] = {mul2(a0, sc), mul2(a1, sc), mul2(a2, sc)};
+            const unsigned o = (unsigned)so * sbytes + oa, o2 = o + 4u * (unsigned)D2;
+            F2 vn[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) vn[a] = fma2(B, sub2(un[a], hu[I][a]), un[a]);
+            auto put = [&](float *base, int a, unsigned at, float v) {
+                *reinterpret_cast<float *>(reinterpret_cast<char *>(base + a * N) + at) = v;
+            };
+            if (outa)
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    put(UO, a, o, lo(un[a]));
+                    put(VO, a, o, lo(vn[a]));
+                }
+            if (outb)
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    put(UO, a, o2, hi(un[a]));
+                    put(VO, a, o2, hi(vn[a]));
+                }
+            if (GAP) {
+                F2 h0, h1, h2;
+                grad(zuc, zu, xzu[GAP ? pw : 0][w + 1][lane], so + 1 < D0, h0, h1, h2);
+                const F2 gg = fma2(h2, h2, fma2(h0, h0, mul2(h1, h1)));
+                const F2 in = fma2(h2, hu[I][2], fma2(h0, hu[I][0], mul2(h1, hu[I][1])));
+                gap_acc += O::sum(O::fms(rp, sqrt2(gg), in), outa, outb);
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+                    dot_acc += O::sum(mul2(sub2(hv[I][a], un[a]), sub2(un[a], hu[I][a])), outa, outb);
+            }
+        }
+        if (ALPHA) hr[I] = O::radius(pk(row(15), row(16)), rad, bnd);
+        z1c = z1;
+        zuc = zu;
+        cz = nz;
+        cv[0] = nv0;
+        cv[1] = nv1;
+        cv[2] = nv2;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) cu[a] = ld(3 + a);
+    };
+    for (int t = 0; t < nsteps; t += 3) {
+        step(std::integral_constant<int, 0>{}, t);
+        if (t + 1 < nsteps) step(std::integral_constant<int, 1>{}, t + 1);
+        if (t + 2 < nsteps) step(std::integral_constant<int, 2>{}, t + 2);
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    double *part = bf.part + (int64_t)b * bf.max_part * 2;
+    if (GAP) {
+        const double gsum = block_sum(gap_acc, sh);
+        const double dsum = block_sum(dot_acc, sh);
+        if (threadIdx.x == 0) {
+            part[tile * 2 + 0] = gsum;
+            part[tile * 2 + 1] = dsum;
+        }
+    }
+    if (!arrive_last(bf.ticket + b, gridDim.x, &flag)) return;
+    double gap = 0.0, dot = 0.0;
+    if (GAP) sum_pairs(part, (int)gridDim.x, sh, gap, dot);
+    if (threadIdx.x != 0) return;
+    bf.ticket[b] = 0;
+    IsoState s2 = st;
+    control(s2, im, A.max_iter, false, false, 0.0, 0.0, pin, bf.live);
+    control(s2, im, A.max_iter, GAP, GAP, gap, dot, pin, bf.live);
+    if (GAP && s2.status != kLive) {
+        // the check is at u': the final u is u', formed again from pin
+        s2.redo = 1;
+        s2.redo_vsel = st.vsel;
+    }
+    bf.st[b] = s2;
+}
+
+// The redo of a checked 3D pair: u' of its first iteration (iso2d_redo_kernel's
+// in three dimensions), in the pair's operations.
+template <bool ALPHA>
+__global__ void __launch_bounds__(256) iso3d_redo_kernel(Geometry g, IsoCall c, IsoBuffers bf) {
+    const int b = (int)blockIdx.y;
+    const IsoState st = bf.st[b];
+    if (st.redo != 1) return;
+    const IsoImage im = bf.img[b];
+    const int D0 = (int)g.L[0], D1 = (int)g.L[1], D2 = (int)g.L[2];
+    const int N = (int)g.N, S0 = D1 * D2;
+    const int pin = st.fin_par, pout = pin ^ 1;
+    const float *D = static_cast<const float *>(bf.d) + (int64_t)b * N;
+    const float *U = static_cast<const float *>(bf.U[pin]) + (int64_t)b * 3 * N;
+    const float *V0 = st.redo_vsel ? U : static_cast<const float *>(bf.V[pin]) + (int64_t)b * 3 * N;
+    const float *V1 = V0 + N, *V2 = V1 + N;
+    float *UO = static_cast<float *>(bf.U[pout]) + (int64_t)b * 3 * N;
+    const float *AL = ALPHA ? static_cast<const float *>(bf.alpha) + (int64_t)b * c.alpha_stride : nullptr;
+    const float wh0 = (float)c.wh[0], wh1 = (float)c.wh[1], wh2 = (float)c.wh[2], tau = (float)c.tau;
+    const float rad = (float)im.radius, bnd = (float)im.bound;
+    auto zat = [&](int o, int s, int y, int x) {
+        const float a = s > 0 ? V0[o - S0] : 0.f, e = y > 0 ? V1[o - D2] : 0.f, l = x > 0 ? V2[o - 1] : 0.f;
+        const float z = fmaf(wh0, __fsub_rn(V0[o], a), D[o]);
+        return fmaf(wh2, __fsub_rn(V2[o], l), fmaf(wh1, __fsub_rn(V1[o], e), z));
+    };
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += (int64_t)gridDim.x * blockDim.x) {
+        const int o = (int)p, s = o / S0, r = o - s * S0, y = r / D2, x = r - y * D2;
+        const float z = zat(o, s, y, x);
+        const float g0 = s + 1 < D0 ? __fmul_rn(wh0, __fsub_rn(zat(o + S0, s + 1, y, x), z)) : 0.f;
+        const float g1 = y + 1 < D1 ? __fmul_rn(wh1, __fsub_rn(zat(o + D2, s, y + 1, x), z)) : 0.f;
+        const float g2 = x + 1 < D2 ? __fmul_rn(wh2, __fsub_rn(zat(o + 1, s, y, x + 1), z)) : 0.f;
+        const float a0 = fmaf(tau, g0, V0[o]), a1 = fmaf(tau, g1, V1[o]), a2 = fmaf(tau, g2, V2[o]);
+        const float nn = fmaf(a2, a2, fmaf(a0, a0, __fmul_rn(a1, a1)));
+        const float rp = pixel_radius<float, ALPHA>(rad, bnd, AL, p);
+        const float sc = nn > __fmul_rn(rp, rp) ? __fmul_rn(rp, rsqrt_t(nn)) : 1.f;
+        UO[o] = __fmul_rn(a0, sc);
+        UO[o + (int64_t)N] = __fmul_rn(a1, sc);
+        UO[o + 2 * (int64_t)N] = __fmul_rn(a2, sc);
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Finalisation: z = d - G^T u (tv_iso.cpp:484-487, 539) back at the input's
 // scale (tv_iso.cpp:403-413), the dual q = u / wmax 2^e into bf.dual.
 // ---------------------------------------------------------------------------
@@ -3327,6 +3679,65 @@ void launch_quad(StepArgs A, const IsoCall &c, const IsoBuffers &bf, cudaStream_
     });
 }
 
+// Slices per block of a 3D pair: what costs least, waves times steps (5 more than
+// the slices written), at most 32: four iterations of 8, 5 and 2 volumes of 128^3
+// live of 8 take 598, 387 and 178 us at 16, 554, 365 and 182 at 32, 577, 397 and 227
+// at 64 (the sums are per block, so the split stays while volumes retire).
+int pair3d_rows(const Geometry &g) {
+    static const int64_t slots = [] {
+        int dev = 0, sms = 148;
+        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaGetLastError();
+        return (int64_t)sms * 2;
+    }();
+    const int64_t tiles = (int64_t)win_count((int)g.L[2], 32, k3PLeft, k3PRight) *
+                          win_count((int)g.L[1], k3PRows, k3PTop, k3PBot);
+    static const int rows_hint = [] {  // tuning hint FASTPROX_B200_PAIR_ROWS
+        const char *v = std::getenv("FASTPROX_B200_PAIR_ROWS");
+        const int r = v ? std::atoi(v) : 0;
+        return (r >= 4 && r <= 128) ? r : 0;
+    }();
+    int rows = rows_hint;
+    double best = 0.0;
+    for (int r = 4; r <= 32 && !rows_hint; r += 4) {
+        const int64_t blocks = g.B * tiles * ((g.L[0] + r - 1) / r);
+        const double cost = (double)((blocks + slots - 1) / slots) * (double)(std::min<int64_t>(r, g.L[0]) + 5);
+        if (!rows || cost < best) {
+            rows = r;
+            best = cost;
+        }
+    }
+    return rows;
+}
+int64_t pair3d_blocks(const Geometry &g) {  // per volume
+    const int rows = pair3d_rows(g);
+    return (int64_t)win_count((int)g.L[2], 32, k3PLeft, k3PRight) * win_count((int)g.L[1], k3PRows, k3PTop, k3PBot) *
+           ((g.L[0] + rows - 1) / rows);
+}
+template <bool ALPHA, bool GAP, bool V16>
+void launch_pair3d_v(StepArgs A, const IsoCall &c, const IsoBuffers &bf, cudaStream_t s) {
+    static std::atomic<unsigned long long> done{0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && !(done.load() & (1ull << dev))) {
+        cudaFuncSetAttribute(iso3d_pair_kernel<ALPHA, GAP, V16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)k3PSmem<ALPHA>);
+        done.fetch_or(1ull << dev);
+    }
+    A.rows = pair3d_rows(A.g);
+    const dim3 grid((unsigned)pair3d_blocks(A.g), 1, (unsigned)A.nimg);
+    launch_step(iso3d_pair_kernel<ALPHA, GAP, V16>, grid, 32 * k3PW, k3PSmem<ALPHA>, s, A, c, bf);
+}
+template <bool V16>
+void launch_pair3d(const StepArgs &A, const IsoCall &c, const IsoBuffers &bf, cudaStream_t s, bool gap) {
+    if (c.has_alpha) {
+        if (gap) launch_pair3d_v<true, true, V16>(A, c, bf, s);
+        else launch_pair3d_v<true, false, V16>(A, c, bf, s);
+    } else {
+        if (gap) launch_pair3d_v<false, true, V16>(A, c, bf, s);
+        else launch_pair3d_v<false, false, V16>(A, c, bf, s);
+    }
+}
+
 // The quad's redo: three iterations over whole images.
 template <class T>
 void quad_redo(const Geometry &g, const IsoCall &c, const IsoBuffers &bf, bool gaps, cudaStream_t s) {
@@ -3383,6 +3794,11 @@ cudaError_t step_t(const Geometry &g, const IsoCall &c, const IsoBuffers &bf, co
         return cudaGetLastError();
     }
     if (variant == kVariantPair || variant == kVariantPairGap) {
+        if (g.k == 3) {
+            if (g.L[2] % 4 == 0) launch_pair3d<true>(A, c, bf, s, variant == kVariantPairGap);
+            else launch_pair3d<false>(A, c, bf, s, variant == kVariantPairGap);
+            return cudaGetLastError();
+        }
         launch_pair<T>(sh, A, c, bf, s, variant == kVariantPairGap);
         return cudaGetLastError();
     }
@@ -3572,7 +3988,13 @@ bool pairs_enabled() {
     return on;
 }
 
-bool iso_pair_ok(const Geometry &g, const StepShape &sh, int max_part) {
+bool iso_pair_ok(int dtype, const Geometry &g, const StepShape &sh, int max_part) {
+    // 3D float32 volumes (iso3d_pair_kernel): windows at least three quarters full
+    // (below, single steps, whose tiles hold small planes without recomputation)
+    if (g.k == 3)
+        return pairs_enabled() && dtype == 1 && sh.kind == 5 && g.L[2] >= 24 && g.L[1] >= 12 &&
+               g.N < (int64_t(1) << 30) &&
+               pair3d_blocks(g) <= max_part;
     // one block per row up to 512 columns (the lean step's threads), else blocks of 512 columns
     return pairs_enabled() && g.k == 2 && sh.kind == 4 && sh.vec == 4 && (sh.gx == 1 ? g.L[1] <= kPairCols : sh.bx == 128) &&
            g.L[0] >= 2 && g.L[0] * sh.gx <= max_part;
@@ -3593,6 +4015,7 @@ bool iso_quad_ok(int dtype, const Geometry &g, int max_part) {
            g.L[0] * g.L[1] < (int64_t(1) << 31) && iso_quad_parts(dtype, g) <= max_part;
 }
 
+int64_t iso_pair3d_parts(int dtype, const Geometry &g) { return g.k == 3 && dtype == 1 ? pair3d_blocks(g) : 0; }
 int64_t iso_quad_parts(int dtype, const Geometry &g) {
     const int W = (int)std::min<int64_t>(g.L[1], 1 << 30);
     return g.k == 2 ? g.L[0] * (int64_t)quad_strips(W, dtype == 1 ? kQuadCols<float> : kQuadCols<double>) : 0;
@@ -3600,7 +4023,14 @@ int64_t iso_quad_parts(int dtype, const Geometry &g) {
 
 cudaError_t iso_redo(int dtype, const Geometry &g, const IsoCall &c, const IsoBuffers &bf, cudaStream_t s,
                      bool quads, bool gaps) {
-    if (g.k != 2 || g.B <= 0 || g.N <= 0) return cudaSuccess;
+    if (g.B <= 0 || g.N <= 0 || (g.k != 2 && !(g.k == 3 && dtype == 1))) return cudaSuccess;
+    if (g.k == 3) {
+        const dim3 grid3((unsigned)std::min<int64_t>((g.N + 255) / 256, 4096), (unsigned)g.B);
+        if (c.has_alpha) iso3d_redo_kernel<true><<<grid3, 256, 0, s>>>(g, c, bf);
+        else iso3d_redo_kernel<false><<<grid3, 256, 0, s>>>(g, c, bf);
+        iso2d_redo_state<<<(unsigned)((g.B + 127) / 128), 128, 0, s>>>(bf.st, g.B);
+        return cudaGetLastError();
+    }
     if (quads) {
         if (dtype == 1) quad_redo<float>(g, c, bf, gaps, s);
         else quad_redo<double>(g, c, bf, gaps, s);
