@@ -23,6 +23,7 @@
 #include <cmath>
 #include <cstdlib>
 
+#include "arith.cuh"
 #include "common.cuh"
 #include "launch.h"
 
@@ -394,21 +395,6 @@ int64_t tail_blocks() {
 // reciprocal square root, and lane 31 carries the three scalars of the next
 // warp's first column instead of re-reading them.
 // ---------------------------------------------------------------------------
-
-template <class T>
-__device__ __forceinline__ T rsqrt_t(T v);
-// float: the hardware reciprocal square root (rsqrtf's result on normal
-// numbers) with arguments below the smallest normal float taken as that
-// smallest normal (no rescaling of subnormal arguments; at a zero radius the
-// projection's scale stays rp times a finite number, 0)
-template <>
-__device__ __forceinline__ float rsqrt_t<float>(float v) {
-    float r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaxf(v, FLT_MIN)));
-    return r;
-}
-template <>
-__device__ __forceinline__ double rsqrt_t<double>(double v) { return rsqrt(v); }
 
 template <class T, int VEC, bool ALPHA, bool GAP, bool ZIN>
 __device__ __forceinline__ void lean_rows(const T *__restrict__ D, const T *__restrict__ U0, const T *__restrict__ U1,
@@ -1422,48 +1408,6 @@ __device__ __forceinline__ void quad_betas(double tn, double beta0, T (&beta)[4]
         beta[l] = (T)((tn - 1.0) / t2);
         tn = t2;
     }
-}
-
-// Packed float pairs (a lane's two columns) in 64-bit registers: sm_100's f32x2
-// arithmetic, each half one IEEE float32 operation rounded to nearest (the same
-// result as the scalar operation; nothing is fused that the scalar steps do not
-// fuse). Held as 64-bit values throughout: pairs packed from float2 around
-// every operation cost 84 register moves of 436 instructions per step.
-typedef unsigned long long F2;
-__device__ __forceinline__ F2 pk(float x, float y) {
-    F2 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
-    return d;
-}
-__device__ __forceinline__ float lo(F2 a) { return __uint_as_float((unsigned)a); }
-__device__ __forceinline__ float hi(F2 a) { return __uint_as_float((unsigned)(a >> 32)); }
-__device__ __forceinline__ F2 sub2(F2 a, F2 b) {  // a - b
-    F2 d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ F2 mul2(F2 a, F2 b) {  // a b
-    F2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {  // a b + c, one rounding
-    F2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-
-// sqrt of both halves (>= 0): s = x y from the hardware's reciprocal root y,
-// then one Newton step on s with its residual x - s^2 formed exactly by a fused
-// operation (Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000", 1990): the error before the last rounding is about 2^-44 of s,
-// below sqrtf's half unit in all but about one case in 10^6. Without the
-// library call's branches (two per row and lane).
-__device__ __forceinline__ F2 sqrt2(F2 x) {
-    const F2 y = pk(rsqrt_t(lo(x)), rsqrt_t(hi(x)));
-    const F2 s = mul2(x, y);
-    const F2 e = pk(fmaf(-lo(s), lo(s), lo(x)), fmaf(-hi(s), hi(s), hi(x)));
-    return fma2(mul2(e, pk(0.5f, 0.5f)), y, s);
 }
 
 // A lane's columns: the operations of a step on float pairs and on one double

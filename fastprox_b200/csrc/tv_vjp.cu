@@ -25,6 +25,7 @@
 #include <cfloat>
 #include <cmath>
 
+#include "arith.cuh"
 #include "common.cuh"
 #include "vjp.h"
 
@@ -636,16 +637,6 @@ __global__ void cg_pv(VjpGeom g, VjpBuffers bf) {
 // for the coordinates) they took 118 of the 250 us of an iteration on 48 x 256^2;
 // this takes 55 (its arrays' 180 MB about 27 at the copy rate, the rest FP64).
 constexpr int kTileW = 32, kTileH = 32, kTileT = 512;
-
-// x / nr from yr = 1 / nr rounded: the quotient of the reciprocal corrected twice
-// by its residual, formed exactly by a fused operation (Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000", 1990): the rounded quotient,
-// as the division gives it, while nothing underflows.
-__device__ __forceinline__ double div_by(double x, double nr, double yr) {
-    double q = __dmul_rn(x, yr);
-    q = __fma_rn(__fma_rn(-q, nr, x), yr, q);
-    return __fma_rn(__fma_rn(-q, nr, x), yr, q);
-}
 
 template <class T>
 __global__ void __launch_bounds__(kT) cg_prep2(VjpGeom g, VjpBuffers bf) {
