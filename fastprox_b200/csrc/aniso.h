@@ -94,6 +94,9 @@ __device__ __forceinline__ void check_done(AnState &s, double gp, double target)
 int an_pixel_blocks(const AnGeom &g);
 // Whether rounds run the piece passes (FASTPROX_B200_AN_FIB=0: the tiled ones).
 bool aniso_pieces_enabled();
+// Partial-sum slots per image that the piece passes need: one per block of the
+// second pass, whichever axes are active and however many images are live.
+int64_t aniso_piece_parts(int dtype, const AnGeom &g, bool has_beta);
 cudaError_t aniso_setup(int dtype, const AnGeom &g, const AnCall &c, const AnBuffers &bf, const void *x,
                         cudaStream_t s);
 // A warm start (tv_aniso.cpp:316-320, 436-486, 539-543, 630-684): the dual

@@ -500,6 +500,18 @@ fp_status check_image(const fp_op &op, const Arr &x) {
     return n < 2147483647.0 ? FP_OK : FP_ESHAPE;
 }
 
+AnGeom an_geom(const Geometry &g0) {
+    AnGeom g{};
+    g.k = g0.k;
+    for (int a = 0; a < 3; ++a) g.L[a] = g0.L[a];
+    g.S[g.k - 1] = 1;
+    for (int a = g.k - 2; a >= 0; --a) g.S[a] = g.S[a + 1] * g.L[a + 1];
+    for (int a = g.k; a < 3; ++a) g.S[a] = 1;
+    g.N = g0.N;
+    g.B = g0.B;
+    return g;
+}
+
 fp_status cuda_status(cudaError_t e) {
     if (e == cudaSuccess) return FP_OK;
     if (e == cudaErrorMemoryAllocation) return FP_ENOMEM;
@@ -567,6 +579,10 @@ fp_status fpb_workspace_build(const fp_op *op, const Arr &x, const fp_options &o
         int64_t nfmax = 0;
         for (int a = 0; a < g.k; ++a) nfmax = std::max<int64_t>(nfmax, g.N / std::max<int64_t>(g.L[a], 1));
         ws->max_part = (int)std::max<int64_t>(ws->max_part, 3 * ((nfmax + 127) / 128));
+        // a block of the piece passes per partial
+        if (g.N > 0 && g.B > 0)
+            ws->max_part = (int)std::max<int64_t>(ws->max_part,
+                                                  aniso_piece_parts(x.dtype, an_geom(g), !op->spatial.empty()));
     }
     // the first iterate of a pair launch whose second iteration carries the
     // check (the final u when it passes)
@@ -1143,14 +1159,7 @@ fp_status run_aniso(fp_workspace *ws, const fp_op *op, const void *xsrc, void *z
     const Geometry &g0 = ws->g;
     cudaStream_t s = ws->stream;
     const size_t T = ws->dtype == FP_F32 ? 4 : 8;
-    AnGeom g{};
-    g.k = g0.k;
-    for (int a = 0; a < 3; ++a) g.L[a] = g0.L[a];
-    g.S[g.k - 1] = 1;
-    for (int a = g.k - 2; a >= 0; --a) g.S[a] = g.S[a + 1] * g.L[a + 1];
-    for (int a = g.k; a < 3; ++a) g.S[a] = 1;
-    g.N = g0.N;
-    g.B = g0.B;
+    const AnGeom g = an_geom(g0);
     AnCall c{};
     int na = 0;
     for (int a = 0; a < 3; ++a) {
