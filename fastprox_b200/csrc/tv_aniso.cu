@@ -1471,8 +1471,13 @@ __global__ void __launch_bounds__(kMarkCols *kMarkParts) an_mark_cols(AnGeom g, 
         }
         part[ty][tx] = acc;
         __syncthreads();
+        const double own = acc;
         acc = 0.0;
         for (int j = 0; j < ty; ++j) acc += part[j][tx];
+        // the sum up to this part's last edge as the next part begins with it:
+        // both sides must take the edge alike, and entry by entry it may round
+        // to another double
+        const double end = acc + own;
         __syncthreads();
         if (act && i0 < i1) {
             double lsb = 0.0;
@@ -1481,7 +1486,7 @@ __global__ void __launch_bounds__(kMarkCols *kMarkParts) an_mark_cols(AnGeom g, 
             for (int i = i0; i < i1; ++i) {
                 const int64_t o = i * s;
                 const bool edge = i + 1 < n;
-                acc += (double)Q[o];
+                acc = i + 1 < i1 ? acc + (double)Q[o] : end;
                 double ls;
                 const bool flat = em.flat(o, -acc, ls);
                 if (edge && flat) F[o] |= bit;
