@@ -235,14 +235,58 @@ IsoCall call_for(fp_b200_batch *bt, const SlotHost &s, double tol, int max_iter)
     return c;
 }
 
+// The lists that a slot's tiles go to (single steps, quads) and how many.
+int single_list(const fp_b200_batch *bt, const SlotHost &s) { return s.vec == (bt->dtype == FP_F32 ? 4 : 2) ? 0 : 1; }
+int quad_list(const SlotHost &s) { return s.W % 4 == 0 ? 2 : 3; }
+
+// Room in the work lists for the tiles of every slot in use (with the rows that
+// h_slots gives). They are made for one tile per 1024 pixels and 64 more per image;
+// tall and narrow images, and quad tiles of few rows, have more.
+fp_status reserve_items(fp_b200_batch *bt) {
+    int64_t n[4] = {0, 0, 0, 0};
+    for (size_t i = 0; i < bt->sh.size(); ++i) {
+        if (!bt->sh[i].used) continue;
+        n[single_list(bt, bt->sh[i])] += bt->h_slots[i].nblk;
+        n[quad_list(bt->sh[i])] += bt->h_slots[i].nquad;
+    }
+    const int64_t need = *std::max_element(n, n + 4);
+    if (need <= bt->max_items) return FP_OK;
+    const int64_t cap = std::max(need, 2 * bt->max_items);
+    RagItem *dev[4] = {}, *host[4] = {};
+    fp_status s = FP_OK;
+    for (int l = 0; l < 4; ++l) {
+        if (s == FP_OK) s = balloc(bt, (void **)&dev[l], (size_t)cap * sizeof(RagItem));
+        if (s == FP_OK) s = halloc(bt, (void **)&host[l], (size_t)cap * sizeof(RagItem));
+    }
+    // the steps in flight read the old lists, and so do the captured graphs
+    if (s == FP_OK && cudaStreamSynchronize(bt->stream) != cudaSuccess) s = FP_EDEVICE;
+    if (s == FP_OK) {
+        for (auto &kv : bt->graphs) cudaGraphExecDestroy(kv.second);
+        bt->graphs.clear();
+        bt->max_items = cap;
+        bt->items_dirty = true;
+    }
+    for (int l = 0; l < 4; ++l) {
+        if (s == FP_OK) {
+            std::swap(bt->items[l], dev[l]);
+            std::swap(bt->h_items[l], host[l]);
+        }
+        // what is not in use: the old lists, or the new ones where one was missing
+        bt->allocs.erase(std::remove(bt->allocs.begin(), bt->allocs.end(), (void *)dev[l]), bt->allocs.end());
+        bt->pinned.erase(std::remove(bt->pinned.begin(), bt->pinned.end(), (void *)host[l]), bt->pinned.end());
+        if (dev[l]) cudaFree(dev[l]);
+        if (host[l]) cudaFreeHost(host[l]);
+    }
+    return s;
+}
+
 // the work lists from the slots in use
 void rebuild_items(fp_b200_batch *bt) {
-    int n[4] = {0, 0, 0, 0};
-    const int vfull = bt->dtype == FP_F32 ? 4 : 2;
+    int n[4] = {0, 0, 0, 0};  // at most max_items (reserve_items)
     for (size_t i = 0; i < bt->sh.size(); ++i) {
         SlotHost &s = bt->sh[i];
         if (!s.used) continue;
-        const int list = s.vec == vfull ? 0 : 1;
+        const int list = single_list(bt, s);
         const int span = 128 * s.vec;
         const RagSlot &rs = bt->h_slots[i];
         int blk = 0;
@@ -253,7 +297,7 @@ void rebuild_items(fp_b200_batch *bt) {
             }
         if (rs.nquad > 0) {  // quad tiles: qrows rows x iso_quad_warps() strips
             const int ns = iso_quad_strips(s.W), qw = iso_quad_warps();
-            const int list = s.W % 4 == 0 ? 2 : 3;
+            const int list = quad_list(s);
             int qb = 0;
             for (int r0 = 0; r0 < s.H; r0 += rs.qrows)
                 for (int st0 = 0; st0 < ns; st0 += qw) {
@@ -409,7 +453,7 @@ FP_API fp_status fp_b200_batch_create(const fp_op *op, int64_t max_images, int64
         bt->dtype = dtype;
         bt->max_slots = max_images;
         bt->max_pixels = (max_pixels + 3) / 4 * 4 + 4 * max_images;
-        // tiles: at least one per 128 x 4 x 4 pixels of the arena, plus one row of tiles per image
+        // tiles: one per 128 x 4 x 2 pixels of the arena and 64 more per image (reserve_items makes more)
         bt->max_items = bt->max_pixels / 1024 + 64 * max_images + 1024;
         const size_t T = dtype == FP_F32 ? 4 : 8, P = (size_t)bt->max_pixels, S = (size_t)max_images;
         fp_status s = FP_OK;
@@ -564,6 +608,11 @@ FP_API fp_status fp_b200_batch_admit(fp_b200_batch *bt, const void *x, int64_t h
         rs.wh1 = c.wh[1];
         rs.tau = c.tau;
         bt->h_slots[slot] = rs;
+        if (fp_status r = reserve_items(bt)) {
+            s.used = false;
+            arena_give(bt, off, N);
+            return r;
+        }
         cudaStream_t st = bt->stream;
         const size_t T = bt->dtype == FP_F32 ? 4 : 8;
         cudaError_t e = cudaMemcpyAsync(bt->slots + slot, bt->h_slots + slot, sizeof(RagSlot), cudaMemcpyHostToDevice, st);
