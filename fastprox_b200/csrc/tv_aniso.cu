@@ -1486,7 +1486,8 @@ __global__ void __launch_bounds__(kMarkCols *kMarkParts) an_mark_cols(AnGeom g, 
             for (int i = i0; i < i1; ++i) {
                 const int64_t o = i * s;
                 const bool edge = i + 1 < n;
-                acc = i + 1 < i1 ? acc + (double)Q[o] : end;
+                acc += (double)Q[o];
+                if (i + 1 == i1) acc = end;
                 double ls;
                 const bool flat = em.flat(o, -acc, ls);
                 if (edge && flat) F[o] |= bit;
