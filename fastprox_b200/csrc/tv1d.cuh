@@ -45,24 +45,12 @@ struct Num;
 template <>
 struct Num<double> {
     static __device__ __forceinline__ double inf() { return CUDART_INF; }
-    static __host__ __device__ __forceinline__ double mul(double a, double b) {
-#ifdef __CUDA_ARCH__
-        return __dmul_rn(a, b);
-#else
-        return a * b;
-#endif
-    }
+    static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
 };
 template <>
 struct Num<float> {
     static __device__ __forceinline__ float inf() { return CUDART_INF_F; }
-    static __host__ __device__ __forceinline__ float mul(float a, float b) {
-#ifdef __CUDA_ARCH__
-        return __fmul_rn(a, b);
-#else
-        return a * b;
-#endif
-    }
+    static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
 };
 
 // 1/m by division.
@@ -284,9 +272,8 @@ struct NoWeight {
 constexpr int kScanUnroll = 4;  // scan steps per trip of tv1d_warp's loop
 
 // tv1d_fiber_sink on the fibres of one warp at once: lane t scans fibre t when
-// `act`, every lane of the warp calls it, and n is the same for all. COPY: a
-// fibre that is its own prox is written through the sink too (every entry a
-// segment of its own; without COPY the sink's storage is the input's). Run one
+// `act`, every lane of the warp calls it, and n is the same for all. A fibre that
+// is its own prox is not written (the sink's storage is the input's). Run one
 // lane per thread, the scans drift apart and a warp runs each lane's branches
 // in turn; here the warp takes one CondatScan step of every live scan per trip
 // of a loop that all its lanes share, and every step is the same arithmetic,
@@ -295,7 +282,7 @@ constexpr int kScanUnroll = 4;  // scan steps per trip of tv1d_warp's loop
 // with zero-weight edges (pieces) run tv1d_fiber_sink after the loop. A scan
 // takes at most 2 (n + 1)^2 steps (every jump moves the segment's start
 // forward, and between jumps k only grows): the loop stops there.
-template <class C, bool COPY = false, class In, class Sink, class Wt, class Rcp>
+template <class C, class In, class Sink, class Wt, class Rcp>
 __device__ __forceinline__ void tv1d_warp(const In &in, const Sink &out, int n, double lam_d, bool has_w, const Wt &w,
                                           const Rcp &rcp, bool act) {
     const C lam = (C)lam_d;
@@ -366,10 +353,6 @@ __device__ __forceinline__ void tv1d_warp(const In &in, const Sink &out, int n, 
     else run(0ll);
     if (fill) out.finish(n);
     if (serial) tv1d_fiber_sink<C>(in, out, n, lam_d, true, w, rcp);
-    if (COPY && act && !fill && !serial) {
-        for (int i = 0; i < n; ++i) out.segment(i, i, (double)in(i));
-        out.finish(n);
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -423,10 +406,10 @@ struct PieceScan {
     int dir;  // a jump that waits: 1 down, 2 up
     C vmin, vmax, ref, s;
 
-    __host__ __device__ __forceinline__ C y(int i) const { return yr[W ? 2 * i : i]; }
-    __host__ __device__ __forceinline__ C r(int i) const { return W ? yr[2 * i + 1] : l; }
+    __device__ __forceinline__ C y(int i) const { return yr[W ? 2 * i : i]; }
+    __device__ __forceinline__ C r(int i) const { return W ? yr[2 * i + 1] : l; }
     // A segment from entry `at`, its first sample taken: s0 = sigma r_e.
-    __host__ __device__ __forceinline__ void open(int at, C s0) {
+    __device__ __forceinline__ void open(int at, C s0) {
         k = k0 = km = kp = at;
         ref = y(at);
         const C ra = r(at);
@@ -440,7 +423,7 @@ struct PieceScan {
     // take no branch: past a jump or the end they compute on and change
     // nothing (k runs on past n - 1; it is not read then). Entries up to
     // n + kPieceUnroll - 1 of yr, and 1/m up to that m, are read and unused.
-    __host__ __device__ __forceinline__ void trip() {
+    __device__ __forceinline__ void trip() {
         C yv[kPieceUnroll], rv[kPieceUnroll], q[kPieceUnroll];
         const int left = n - 1 - k;
 #pragma unroll
@@ -477,7 +460,7 @@ struct PieceScan {
     }
     // The segment that a waiting jump (or the fibre's end) closes: its last
     // entry and value, and which it was (1 down, 2 up, 3 the end). 0: none.
-    __host__ __device__ __forceinline__ int event(int &e, C &v) const {
+    __device__ __forceinline__ int event(int &e, C &v) const {
         if (dir == 0 && k < n - 1) return 0;
         int d = dir;
         C ve = C(0);
@@ -490,7 +473,7 @@ struct PieceScan {
         return d;
     }
     // The next segment after a jump of direction d at edge e.
-    __host__ __device__ __forceinline__ void jump(int e, int d) { open(e + 1, d == 1 ? r(e) : -r(e)); }
+    __device__ __forceinline__ void jump(int e, int d) { open(e + 1, d == 1 ? r(e) : -r(e)); }
 };
 
 // Trips of the scan until `ev` (given each segment as it closes: end, value
