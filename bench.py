@@ -49,10 +49,10 @@ B, H, W = 64, 512, 512
 # DRAM bytes (read + write) of one launch of the dominant kernel, the quad
 # launch (four iterations over the 64 images, the fourth with the gap check),
 # from one ncu capture of this batch (profiles/iso2d_quad_64x512_fp32.md:
-# 378.6 MB read + 232.7 MB written): below the 4 x 40 B per pixel of its four
+# 377.8 MB read + 230.5 MB written): below the 4 x 40 B per pixel of its four
 # iterations, since d, u, v and alpha are read once for all four and only the
 # fourth's u, v are written.
-QUAD_TRAFFIC = 611245056
+QUAD_TRAFFIC = 608262656
 QUAD_KIND, QUAD_ITERS = 3, 4  # fp_b200_workspace_step_times kind of the quad launch, its iterations
 GAMMAS = (0.05, 0.1, 0.2)
 TOL, MAX_ITER = 1e-6, 20000

@@ -3,16 +3,16 @@
 // (continuous batching). A B200 extension of the C ABI; no counterpart in the
 // reference, whose driver takes one array shape per call.
 //
-// Device memory (all allocated at creation): an arena of pixels holding d and
+// Device memory (allocated at creation, but for longer work lists: reserve_items): an arena of pixels holding d and
 // the ping-pong dual pairs u, v of every admitted image (a first-fit free list
 // of pixel ranges on the host places them), per-slot constants and state,
 // partial sums and tickets, and two work lists of (image, tile) items, one
 // for rows of a multiple of 4 pixels (16-byte vectors) and one for the rest.
 // A step launches the single-step kernel over each list (each block in the
 // variant its image's state asks for), on the 4-wide float list the two pair
-// variants (two iterations per launch), and over a third list of quad tiles
-// (float rows of a multiple of 4 pixels) the quad (four iterations per
-// launch); chunks of steps are replayed as CUDA graphs, captured again only
+// variants (two iterations per launch), and over two lists of quad tiles (float
+// rows of a multiple of 4 pixels, and other rows of 32 pixels or more) the quad
+// (four iterations per launch); chunks of steps are replayed as CUDA graphs, captured again only
 // when the work lists outgrow their current size class.
 #include <cuda_runtime_api.h>
 

@@ -1321,13 +1321,17 @@ __global__ void iso2d_redo_state(IsoState *st, int64_t B) {
 // Traffic per pixel and four iterations: d, u, v, alpha read once (rows of a
 // block's halo again, from L2 mostly), u, v written once: about 40 B against
 // 4 x 40 B for four single steps.
-// What bounds it: with 16 warps per SM (128 registers) a step of a warp is 300
-// instructions over four dependent levels; 58 % of the issue slots, 27 % of the
-// DRAM sectors. 436 instructions a step (84 of them register moves, 78 integer
+// What bounds it: with 16 warps per SM (128 registers) a step of a warp is 311
+// instructions over four dependent levels: 60 % of the issue slots, while the 608
+// MB that a launch on 64 x 512^2 moves (604 MB of inputs and outputs) leave HBM at
+// 3.6 TB/s, 0.54 of the measured copy rate. The float kernels spill at four blocks
+// per SM (bytes stored and loaded a thread: 48 to 80 and 68 to 104 with 16-byte
+// copies, 60 to 72 and 72 to 84 with 8, 160 to 172 and 236 to 416 with 4); local
+// loads are 0.3 % of the 16-byte kernel's instructions. 436 instructions a step (84 of them register moves, 78 integer
 // address work, 27 shuffles) took 227 us a launch on 64 x 512^2; pairs held in
 // 64-bit registers, four steps unrolled with fixed ring slots, the sums of four
 // rows at a time, momenta in shared memory and a square root without branches
-// made it 170 us (64 x 512^2 with pixel weights 48.8 -> 35.1 ms a solve).
+// made it 171 us (64 x 512^2 with pixel weights 48.8 -> 35.3 ms a solve).
 // Float64: one column per lane (windows of 32, 24 written), the same ring in bytes;
 // bound by the four dependent levels of a step (FP64 latency, 0.25 us each at three
 // blocks per SM) more than by FP64 rate. Four 384 x 320 images at 1e-8: 26.4 ms in
@@ -2913,7 +2917,7 @@ __global__ void __launch_bounds__(k3VX / 2 * k3VY, 4) iso3d_v2_kernel(StepArgs A
 // instructions per warp and step, two dependent iterations, a barrier), with 54 B of
 // DRAM traffic a voxel per two iterations at 3.6 TB/s. Four iterations of 8 x 128^3:
 // 730 us in single steps (three of 166, one of 230), 554 in two pairs; 5 volumes
-// live: 473 and 365; 2: 223 and 182. A solve of 8 to 1e-5: 110.9 -> 86.4 ms.
+// live: 473 and 365; 2: 223 and 182. A solve of 8 to 1e-5: 102.7 -> 78.3 ms.
 // ---------------------------------------------------------------------------
 constexpr int k3PW = 8;               // warps per block
 constexpr int k3PRows = 2 * k3PW;     // window rows
@@ -3570,8 +3574,8 @@ void quad_kernels(int W, const F &f) {
 // The quad launch: blocks of kQuadWarps tiles (a strip by `rows` rows). A
 // tile's march takes rows + 8 steps and the SMs hold a fixed number of
 // blocks at once, so the rows are chosen (4 to 64, in steps of 4) for the
-// fewest waves of resident blocks times steps per tile: 48 on 64 images of
-// 512^2 (three waves of 56 steps, against five of 40 at 32 rows), 8 for one
+// fewest waves of resident blocks times steps per tile: 64 on 64 images of
+// 512^2 (two waves of 72 steps, against three of 56 at 48 rows), 8 for one
 // image (a single wave of short tiles). Small launches take 4 rows (64^2: 0.58 ms
 // a solve against 0.64 at 8).
 template <class T>

@@ -277,15 +277,16 @@ FP_API void fp_b200_release_cached(void);
  * Results are the same bits whatever else is in the batch.
  *
  * create: capacity for max_images images and max_pixels pixels in all, every
- * byte of device memory allocated here, on the current device; dtype FP_F32
+ * byte of device memory allocated here, on the current device (but for longer
+ * work lists, made by admit where images have more tiles than their pixels
+ * suggest: tall ones a few pixels wide, quad tiles of a few rows); dtype FP_F32
  * or FP_F64 (the images' dtype). admit: x and z are device pointers to
  * contiguous (height, width) arrays (z may be x), copied in now, solved by
  * later runs; tol and max_iter as in fp_prox, per image; FP_ENOMEM when no
  * slot or not enough contiguous pixels are free (admit again after a run has
  * finished others). run: repeats `steps` steps of every live image (as a
  * captured CUDA graph; a step advances an image by one iteration, or by four
- * on float images whose width is a multiple of 4, in two launches of two
- * iterations each) until at least one image has finished or none is live;
+ * on float images whose width is a multiple of 4 or at least 32) until at least one image has finished or none is live;
  * writes the finished images' z, and their slots, gaps and iterations (a
  * negative count: stopped at max_iter) into arrays of max_images entries;
  * *nlive, the images still iterating. max_chunks > 0 bounds the chunks of
@@ -306,8 +307,9 @@ FP_API fp_status fp_b200_batch_set_graphs(fp_b200_batch *bt, int on);
  * height); the tuner sets it. */
 FP_API fp_status fp_b200_batch_set_rows(fp_b200_batch *bt, int rows);
 /* Quad launches (four iterations per launch) for the float images of rows of a
- * multiple of 4 pixels admitted from now on: on (default) or off, and the rows
- * of a quad tile (0 keeps the current, 32 by default). For the tuner. */
+ * multiple of 4 pixels, or of 32 pixels or more, admitted from now on: on
+ * (default) or off, and the rows of a quad tile (0 keeps the current, 32 by
+ * default). For the tuner. */
 FP_API fp_status fp_b200_batch_set_quads(fp_b200_batch *bt, int on, int rows);
 FP_API fp_status fp_b200_batch_admit(fp_b200_batch *bt, const void *x, int64_t height, int64_t width, double gamma,
                                      double tol, int max_iter, void *z, int *slot);
