@@ -96,11 +96,12 @@ __device__ __forceinline__ bool arrive_last(unsigned *ticket, unsigned nblk, int
 
 // Sum of part[i * stride + off] for i < n in a fixed order (a strided pass
 // per thread, then the block tree), read past L1. Valid in thread 0. The loads
-// go eight at a time: one after another, the 57 of each thread for the quad's
+// go U at a time: one after another, the 57 of each thread for the quad's
 // sums of a 1531 x 1021 image held the launch's last block for 30 us.
+template <int U = 8>
 __device__ __forceinline__ double sum_partials(const double *part, int n, int stride, int off, double *sh) {
     double s = 0.0;
-#pragma unroll 8
+#pragma unroll U
     for (int i = threadIdx.x; i < n; i += blockDim.x) s += __ldcg(part + (int64_t)i * stride + off);
     return block_sum(s, sh);
 }

@@ -2629,9 +2629,16 @@ __global__ void __launch_bounds__(k3TX * k3TY) iso3d_kernel(StepArgs A, IsoCall 
     }
     if (!arrive_last(bf.ticket + b, nblk, &flag)) return;
     double gap = 0.0, dot = 0.0;
-    if (GAP || test) sum_pairs(part, nblk, sh, gap, dot);
-    if (!GAP) gap = 0.0;
-    if (!test) dot = 0.0;
+    if (sizeof(T) == 8) {
+        // one sum at a time and load by load: with the pairs' loads in flight the
+        // plain step gets 64 registers and spills (64^3 5.9 ms a solve, then 6.3)
+        if (GAP) gap = sum_partials<1>(part, nblk, 2, 0, sh);
+        if (test) dot = sum_partials<1>(part, nblk, 2, 1, sh);
+    } else {
+        if (GAP || test) sum_pairs(part, nblk, sh, gap, dot);
+        if (!GAP) gap = 0.0;
+        if (!test) dot = 0.0;
+    }
     if (threadIdx.x != 0) return;
     bf.ticket[b] = 0;
     IsoState s2 = st;
