@@ -378,6 +378,10 @@ __device__ __forceinline__ void tv1d_warp(const In &in, const Sink &out, int n, 
 // The segments are those of CondatScan over the whole fibre, for any input: a
 // lane whose guess never meets the true scan is passed over. The work is the
 // scan's, plus about a segment per piece.
+// An edge of zero weight cuts a fibre in two that share nothing: the segment
+// before it ends there as at a fibre's end, and the next one opens as at a
+// fibre's beginning, which again depends on nothing before, so a cut is handed
+// over like a jump (its mark, 3, is a direction of its own).
 // The step itself is CondatScan's arithmetic without its opening case: a
 // segment opens at the jump (or start) with its first sample taken, and jumps
 // found within a trip of kPieceUnroll steps are handled together at its end
@@ -479,10 +483,10 @@ struct PieceScan {
 // Trips of the scan until `ev` (given each segment as it closes: end, value
 // and direction; it says whether to go on) has stopped every lane. A scan
 // takes at most 2 (n + 1)^2 steps, and every trip takes at least one step or
-// one segment per live lane.
+// one segment per live lane. n: the fibre's entries.
 template <class S, class C, class Ev>
-__device__ __forceinline__ void piece_trips(S &p, bool live, const Ev &ev, C, int *err) {
-    const unsigned most = 2u * (unsigned)(p.n + 1) * (unsigned)(p.n + 1);  // n < 46340
+__device__ __forceinline__ void piece_trips(S &p, bool live, int n, const Ev &ev, C, int *err) {
+    const unsigned most = 2u * (unsigned)(n + 1) * (unsigned)(n + 1);  // n < 46340
     for (unsigned it = 0; __any_sync(0xffffffffu, live); ++it) {
         if (it > most) {
             if (live) atomicExch(err, 4);
@@ -506,10 +510,13 @@ __device__ __forceinline__ void piece_trips(S &p, bool live, const Ev &ev, C, in
 // sub len; every lane of the warp calls it, with live false for groups that
 // have nothing to scan (their marks stay). mark: n bytes, zero before; val: n
 // values (the segments' at their ends); le, lv: this lane's list of `cap`
-// segments. Afterwards every mark is a segment's end.
-template <class C, bool W>
+// segments. Afterwards every mark is a segment's end. CUT: cut(e) says whether
+// edge e is one of zero weight (its radius in yr is 0, and the radii are those of
+// the whole fibre's edges: none is clamped).
+template <class C, bool W, bool CUT, class Cut>
 __device__ __forceinline__ void tv1d_pieces(const C *yr, const C *rc, C l, int n, int P, int len, int sub, bool live,
-                                            unsigned char *mark, C *val, int *le, C *lv, int cap, int *err) {
+                                            unsigned char *mark, C *val, int *le, C *lv, int cap, const Cut &cut,
+                                            int *err) {
     PieceScan<C, W> p;
     p.yr = yr;
     p.rc = rc;
@@ -517,19 +524,36 @@ __device__ __forceinline__ void tv1d_pieces(const C *yr, const C *rc, C l, int n
     p.n = n;
     const int c0 = sub * len, c1 = c0 + len < n ? c0 + len : n;
     const bool mine = live && c0 < n;
+    // the scan's end: the fibre's, or the first cut at or after entry i
+    auto seek = [&](int i) {
+        if constexpr (CUT) {
+            while (i < n - 1 && !cut(i)) ++i;
+            p.n = i + 1;
+        }
+    };
+    auto last = [&](int e, int dir) { return dir == 3 && (!CUT || e == n - 1); };  // the fibre's last segment
+    auto past = [&](int e, int dir) {  // beyond a cut
+        if (CUT && dir == 3) seek(e + 1);
+    };
     bool own = sub == 0;
     int xe = 0, xs = 0;  // the segment that ended this lane's piece
     C xv = C(0);
-    if (mine) p.open(c0, C(0));
+    if (mine) {
+        seek(c0);
+        p.open(c0, C(0));
+    }
     piece_trips(
-        p, mine,
+        p, mine, n,
         [&](int e, C v, int dir) {
             if (e < c1) {
                 val[e] = v;
                 mark[e] = (unsigned char)dir;
                 own = true;
             }
-            if (dir != 3 && e + 1 < c1) return true;
+            if (!last(e, dir) && e + 1 < c1) {
+                past(e, dir);
+                return true;
+            }
             xe = e;
             xs = dir;
             xv = v;
@@ -546,26 +570,30 @@ __device__ __forceinline__ void tv1d_pieces(const C *yr, const C *rc, C l, int n
         }
         ++cnt;
     };
-    bool go = mine && own && xs != 3;
+    bool go = mine && own && !last(xe, xs);
     if (mine && own && xe >= c1) {
         put(xe, xv);
-        if (xs != 3 && mark[xe] == xs) {
+        if (!last(xe, xs) && mark[xe] == xs) {
             nxt = xe / len;
             at = xe;
             go = false;
         }
     }
-    if (go) p.jump(xe, xs);
+    if (go) {
+        past(xe, xs);
+        p.jump(xe, xs);
+    }
     piece_trips(
-        p, go,
+        p, go, n,
         [&](int e, C v, int dir) {
             put(e, v);
-            if (dir == 3) return false;
+            if (last(e, dir)) return false;
             if (mark[e] == dir) {
                 nxt = e / len;
                 at = e;
                 return false;
             }
+            past(e, dir);
             return true;
         },
         C(0), err);
@@ -607,14 +635,17 @@ __device__ __forceinline__ void tv1d_pieces(const C *yr, const C *rc, C l, int n
                 val[xe] = xv;
                 mark[xe] = kMarkFinal;
             }
+            seek(xe + 1);
             p.jump(xe, xs);
         }
         piece_trips(
-            p, again,
+            p, again, n,
             [&](int e, C v, int dir) {
                 val[e] = v;
                 mark[e] = kMarkFinal;
-                return dir != 3 && e != at;
+                if (last(e, dir) || e == at) return false;
+                past(e, dir);
+                return true;
             },
             C(0), err);
     }
