@@ -1331,7 +1331,7 @@ __global__ void iso2d_redo_state(IsoState *st, int64_t B) {
 // address work, 27 shuffles) took 227 us a launch on 64 x 512^2; pairs held in
 // 64-bit registers, four steps unrolled with fixed ring slots, the sums of four
 // rows at a time, momenta in shared memory and a square root without branches
-// made it 171 us (64 x 512^2 with pixel weights 48.8 -> 35.3 ms a solve).
+// made it 171 us (64 x 512^2 with pixel weights 47.6 -> 34.7 ms a solve).
 // Float64: one column per lane (windows of 32, 24 written), the same ring in bytes;
 // bound by the four dependent levels of a step (FP64 latency, 0.25 us each at three
 // blocks per SM) more than by FP64 rate. Four 384 x 320 images at 1e-8: 26.4 ms in
@@ -2924,7 +2924,7 @@ __global__ void __launch_bounds__(k3VX / 2 * k3VY, 4) iso3d_v2_kernel(StepArgs A
 // instructions per warp and step, two dependent iterations, a barrier), with 54 B of
 // DRAM traffic a voxel per two iterations at 3.6 TB/s. Four iterations of 8 x 128^3:
 // 730 us in single steps (three of 166, one of 230), 554 in two pairs; 5 volumes
-// live: 473 and 365; 2: 223 and 182. A solve of 8 to 1e-5: 102.7 -> 78.3 ms.
+// live: 473 and 365; 2: 223 and 182. A solve of 8 to 1e-5: 110.3 -> 86.2 ms.
 // ---------------------------------------------------------------------------
 constexpr int k3PW = 8;               // warps per block
 constexpr int k3PRows = 2 * k3PW;     // window rows
